@@ -409,7 +409,8 @@ static int capture_step(sem_batch* b, const BatchArgs& base)
             ba.queue = gr.d_queue;
             cudaMemsetAsync(gr.d_queue, 0, sizeof(int), gr.fork);
             dispatch_batch_n(gr.N, [&](auto nv) {
-                return batch_launch_step<decltype(nv)::value>(ba, gr.grid, gr.smem, gr.fork);
+                return batch_launch_step<decltype(nv)::value>(ba, ctx_mesh(b->ctx[gr.members[0]]), gr.grid, gr.smem,
+                                                               gr.fork);
             });
             cudaEventRecord(gr.done, gr.fork);
             cudaStreamWaitEvent(cs, gr.done, 0);

@@ -66,7 +66,7 @@ size_t batch_smem_n(int kmax);
 template <int N>
 cudaError_t batch_prepare(size_t smem, int* per_sm);
 template <int N>
-cudaError_t batch_launch_step(const BatchArgs& ba, int grid, size_t smem, cudaStream_t st);
+cudaError_t batch_launch_step(const BatchArgs& ba, const DevMesh& m0, int grid, size_t smem, cudaStream_t st);
 template <int N>
 cudaError_t batch_launch_probe(const BatchInst* inst, const int* list, int nlist, int kmax, int reps, float* sink,
                                int grid, cudaStream_t st);
@@ -82,7 +82,8 @@ namespace semgb {
 
 template <int N>
 __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned char* smraw, double* red,
-                              MinresScal<float>& sc, double* sweep_state, float* fdmS, float* fdmL)
+                              MinresScal<float>& sc, double* sweep_state, float* fdmS, float* fdmL,
+                              const CgTab<N>& tab)
 {
     constexpr int NN = N * N;
     const DevMesh& m = I.m;
@@ -148,7 +149,7 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
     mx.fused = 0;
     mx.outer_scale = ba.outer_scale;
     mx.adaptive = 1;
-    mixed_solve<N, OP_RES, true>(m, a, I.w, mx, 0, m.E, true, smraw, red, sc, sweep_state, fdmS, fdmL);
+    mixed_solve<N, OP_RES, MIXED_BATCH>(m, a, I.w, mx, 0, m.E, true, smraw, red, sc, sweep_state, fdmS, fdmL, &tab);
     // unmask(p) (schrodinger.hpp:105-106): owner copies are never written here
     for (long long idx = threadIdx.x; idx < n; idx += blockDim.x) {
         const int e = (int)(idx / NN);
@@ -169,7 +170,7 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
 
 // one time step of every instance in ba.order (all of degree N)
 template <int N>
-__global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_bdf2(BatchArgs ba)
+__global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_bdf2(BatchArgs ba, const __grid_constant__ CgTab<N> tab)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[34];
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_bdf2(BatchArgs ba)
         if (q >= ba.n) break;
         if (threadIdx.x == 0) I = ba.inst[ba.order[q]];
         __syncthreads();
-        bdf2_instance<N>(I, ba, smraw, red, sc, sweep_state, fdmS, fdmL);
+        bdf2_instance<N>(I, ba, smraw, red, sc, sweep_state, fdmS, fdmL, tab);
         __syncthreads();
     }
 }
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_probe(const BatchInst* i
 template <int N>
 size_t batch_smem_n(int kmax)
 {
-    return std::max(range_smem_bytes<N, double, OP_RES>(kmax), range_smem_bytes<N, float, OP_RES>(kmax));
+    return std::max(range_smem_bytes<N, double, OP_RES>(kmax), cg_smem_bytes<N>(kmax));
 }
 
 // shared-memory opt-in and resident blocks per SM of the step kernel
@@ -243,9 +244,9 @@ cudaError_t batch_prepare(size_t smem, int* per_sm)
 }
 
 template <int N>
-cudaError_t batch_launch_step(const BatchArgs& ba, int grid, size_t smem, cudaStream_t st)
+cudaError_t batch_launch_step(const BatchArgs& ba, const DevMesh& m0, int grid, size_t smem, cudaStream_t st)
 {
-    k_batch_bdf2<N><<<grid, BATCH_TPB, smem, st>>>(ba);
+    k_batch_bdf2<N><<<grid, BATCH_TPB, smem, st>>>(ba, cg_table<N>(m0));
     return cudaGetLastError();
 }
 
@@ -268,7 +269,8 @@ cudaError_t batch_launch_probe(const BatchInst* inst, const int* list, int nlist
     namespace semgb {                                                                                    \
     template size_t batch_smem_n<NV>(int);                                                               \
     template cudaError_t batch_prepare<NV>(size_t, int*);                                                \
-    template cudaError_t batch_launch_step<NV>(const BatchArgs&, int, size_t, cudaStream_t);             \
+    template cudaError_t batch_launch_step<NV>(const BatchArgs&, const DevMesh&, int, size_t,            \
+                                                 cudaStream_t);                                          \
     template cudaError_t batch_launch_probe<NV>(const BatchInst*, const int*, int, int, int, float*, int, \
                                                 cudaStream_t);                                           \
     }

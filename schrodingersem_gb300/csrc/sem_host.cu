@@ -211,6 +211,7 @@ static int grid_1d(long long n) { return (int)std::min<long long>((n + 255) / 25
 
 // dynamic shared memory a persistent solver block may use for staging
 static const size_t kSolverSmemBudget = 160 * 1024;
+static const size_t kCgSmemBudget = 2 * 108 * 1024;
 // the resident inner solve may use all of an SM's shared memory (227 KB per
 // block, less the kernel's static arrays)
 static const size_t kResidentSmemBudget = 227 * 1024 - 512;
@@ -338,7 +339,8 @@ struct sem_ctx {
     unsigned flags = 0;
     std::vector<double> x, w, D;           // D column-major
     std::vector<double> Drow_host;         // D row-major (DevMesh::Dh)
-    std::vector<float> D32_host, S32_host; // FP32 D and preconditioner basis S, row-major
+    std::vector<double> S_host;            // preconditioner basis row-major (DevMesh::Sh)
+    unsigned res_epoch = 0;                // last epoch on the resident solver's exchange words (0: clear them)
     std::vector<double> coords;            // [n_nodes][2]
     std::vector<int> elements;             // [E][4]
     std::vector<int> fl_host;              // DevMesh::flags, host copy
@@ -509,11 +511,27 @@ static void fdm_basis(int N, const std::vector<double>& w, const std::vector<dou
             B[(size_t)i * N + j] = k / std::sqrt(w[i] * w[j]);
         }
     sym_eig_jacobi(N, B, Q);
+    // even modes first, each parity by ascending eigenvalue, and every mode
+    // made exactly even or odd (the nodes and weights are symmetric, so the
+    // computed vectors are to rounding): the line passes contract the two
+    // parities separately (sem_lines.cuh)
+    std::vector<int> order;
+    for (int par = 0; par < 2; ++par) {
+        const size_t first = order.size();
+        for (int k = 0; k < N; ++k)
+            if ((Q[k] * Q[(size_t)(N - 1) * N + k] < 0) == (par == 1)) order.push_back(k);
+        std::sort(order.begin() + first, order.end(),
+                  [&](int a, int b) { return B[(size_t)a * N + a] < B[(size_t)b * N + b]; });
+    }
     S.assign((size_t)N * N, 0.0);
     lam.assign(N, 0.0);
     for (int k = 0; k < N; ++k) {
-        lam[k] = B[(size_t)k * N + k];
-        for (int i = 0; i < N; ++i) S[(size_t)i * N + k] = Q[(size_t)i * N + k] / std::sqrt(w[i]);
+        const int q = order[k];
+        const double sg = k < (N + 1) / 2 ? 1.0 : -1.0;
+        lam[k] = B[(size_t)q * N + q];
+        for (int i = 0; i < N; ++i)
+            S[(size_t)i * N + k] = 0.5 * (Q[(size_t)i * N + q] / std::sqrt(w[i]) +
+                                          sg * Q[(size_t)(N - 1 - i) * N + q] / std::sqrt(w[N - 1 - i]));
     }
 }
 
@@ -859,8 +877,8 @@ static int build_ctx(sem_ctx* c, int p, int n_nodes, const double* coords, int n
         for (size_t i = 0; i < v.size(); ++i) f[i] = (float)v[i];
         return f;
     };
-    c->D32_host = Drowf;
-    c->S32_host = tof(fS);
+    c->S_host = fS;
+    d.Sh = c->S_host.data();
     int s = 0;
     if ((s = upload(c, fl, &d.flags)) || (s = upload(c, sbase, &d.side_base)) ||
         (s = upload(c, sstep, &d.side_step)) || (s = upload(c, csrc, &d.corner_src)) ||
@@ -1474,24 +1492,7 @@ static int run_mixed(sem_ctx* c, int op, const double* pot, double alpha, double
             resident = resident_plan<decltype(nv)::value>(c->E, c->sms, kResidentSmemBudget, &grid, &rst, &kmax,
                                                           &smem);
         });
-    if (!resident)
-        dispatch_n(c->N, [&](auto nv) {
-            grid = solver_plan<decltype(nv)::value>(op, true, c->E, c->sms, kSolverSmemBudget, &kmax, &smem);
-            return cudaSuccess;
-        });
-    if (grid <= 0) return fail(SEM_ERR_CUDA, "could not size the cooperative grid");
-    unsigned long long *slots = nullptr, *xa = nullptr, *xb = nullptr;
-    if (resident) {
-        const size_t words = 2 * (size_t)grid * RESIDENT_SLOT_STRIDE;
-        if ((s = wsget(c, "res_slots", words, &slots)) || (s = wsget(c, "res_xa", 2 * (size_t)c->n, &xa)) ||
-            (s = wsget(c, "res_xb", 2 * (size_t)c->n, &xb)))
-            return s;
-        SEM_CUDA(cudaMemsetAsync(slots, 0, words * sizeof(unsigned long long), c->stream));
-        SEM_CUDA(cudaMemsetAsync(xa, 0, 2 * (size_t)c->n * sizeof(unsigned long long), c->stream));
-        SEM_CUDA(cudaMemsetAsync(xb, 0, 2 * (size_t)c->n * sizeof(unsigned long long), c->stream));
-    }
     SolveArgs a{};
-    a.kmax = kmax;
     a.op = op;
     a.nc = nc;
     a.pot = pot;
@@ -1507,30 +1508,72 @@ static int run_mixed(sem_ctx* c, int op, const double* pot, double alpha, double
     a.timeout_ns = (long long)(c->timeout_ms * 1e6);
     a.sync = sync;
     a.out = out;
-    SEM_CUDA(cudaMemsetAsync(sync, 0, sizeof(GridSync), c->stream));
-    SEM_CUDA(cudaMemsetAsync(out, 0, sizeof(SolveOut), c->stream));
-    if (c->profile) SEM_CUDA(cudaEventRecord(c->ev[0], c->stream));
-    cudaError_t e = cudaSuccess;
-    if (resident)
-        dispatch_resident(c->N, [&](auto nv) {
-            e = launch_resident<decltype(nv)::value>(c->dm, a, w, mx, c->D32_host.data(), c->S32_host.data(), rst,
-                                                     slots, xa, xb, grid, smem, c->stream);
-        });
-    else
-        e = dispatch_n(c->N, [&](auto nv) {
-            return launch_solver<decltype(nv)::value>(c->dm, a, &w, &mx, grid, smem, c->stream);
-        });
-    if (e != cudaSuccess) return fail(SEM_ERR_CUDA, std::string("cooperative launch: ") + cudaGetErrorString(e));
-    if (c->profile) SEM_CUDA(cudaEventRecord(c->ev[1], c->stream));
-    c->stats.kernel_launches++;
-    c->stats.solver_launches++;
-    if (resident) c->stats.resident_launches++;
-    if ((s = finish_solve(c, out, sync, res))) return s;
-    *sweeps = c->h_out->sweeps;
-    c->stats.solver_iterations_fp32 += res->n_iter;
-    c->stats.fp32_applies += res->n_iter + *sweeps;
-    c->stats.fp64_applies += *sweeps + 1;
-    return SEM_OK;
+    int done_it = 0, done_sweeps = 0;  // a resident solve that gave up
+    for (;;) {
+        unsigned long long *slots = nullptr, *xa = nullptr, *xb = nullptr;
+        unsigned epoch0 = 0;
+        if (resident) {
+            const size_t words = 2 * (size_t)grid * RESIDENT_SLOT_STRIDE;
+            if ((s = wsget(c, "res_slots", words, &slots)) || (s = wsget(c, "res_xa", 2 * (size_t)c->n, &xa)) ||
+                (s = wsget(c, "res_xb", 2 * (size_t)c->n, &xb)))
+                return s;
+            // the words' epochs run on from solve to solve (at most four per
+            // iteration); cleared for the first, after a failed one and long
+            // before the counter wraps
+            epoch0 = c->res_epoch;
+            c->res_epoch = 0;
+            if (epoch0 == 0 || epoch0 > 0x40000000u || maxit > 0x10000000) {
+                epoch0 = 0;
+                SEM_CUDA(cudaMemsetAsync(slots, 0, words * sizeof(unsigned long long), c->stream));
+                SEM_CUDA(cudaMemsetAsync(xa, 0, 2 * (size_t)c->n * sizeof(unsigned long long), c->stream));
+                SEM_CUDA(cudaMemsetAsync(xb, 0, 2 * (size_t)c->n * sizeof(unsigned long long), c->stream));
+            }
+        } else {
+            dispatch_n(c->N, [&](auto nv) {
+                grid = solver_plan<decltype(nv)::value>(op, mx.fdm ? SOLVE_MIXED_FDM : SOLVE_MIXED, c->E, c->sms,
+                                                        mx.fdm ? kCgSmemBudget : kSolverSmemBudget, &kmax, &smem);
+                return cudaSuccess;
+            });
+            if (grid <= 0) return fail(SEM_ERR_CUDA, "could not size the cooperative grid");
+        }
+        a.kmax = kmax;
+        SEM_CUDA(cudaMemsetAsync(sync, 0, sizeof(GridSync), c->stream));
+        SEM_CUDA(cudaMemsetAsync(out, 0, sizeof(SolveOut), c->stream));
+        if (c->profile) SEM_CUDA(cudaEventRecord(c->ev[0], c->stream));
+        cudaError_t e = cudaSuccess;
+        if (resident)
+            dispatch_resident(c->N, [&](auto nv) {
+                e = launch_resident<decltype(nv)::value>(c->dm, a, w, mx, rst, slots, xa, xb, epoch0, grid, smem,
+                                                         c->stream);
+            });
+        else
+            e = dispatch_n(c->N, [&](auto nv) {
+                return launch_solver<decltype(nv)::value>(c->dm, a, &w, &mx, grid, smem, c->stream);
+            });
+        if (e != cudaSuccess) return fail(SEM_ERR_CUDA, std::string("cooperative launch: ") + cudaGetErrorString(e));
+        if (c->profile) SEM_CUDA(cudaEventRecord(c->ev[1], c->stream));
+        c->stats.kernel_launches++;
+        c->stats.solver_launches++;
+        if (resident) c->stats.resident_launches++;
+        if ((s = finish_solve(c, out, sync, res))) return s;
+        c->stats.solver_iterations_fp32 += res->n_iter;
+        c->stats.fp32_applies += res->n_iter + c->h_out->sweeps;
+        c->stats.fp64_applies += c->h_out->sweeps + 1;
+        res->n_iter += done_it;
+        *sweeps = c->h_out->sweeps + done_sweeps;
+        if (!resident) return SEM_OK;
+        c->res_epoch = c->h_out->epoch;
+        if (!c->h_out->fallback) return SEM_OK;
+        // the resident iteration broke down, stalled or did not help: go on
+        // from its solution on the staged kernel, MINRES only
+        done_it = res->n_iter;
+        done_sweeps = *sweeps;
+        resident = false;
+        mx.minres = 1;
+        a.x_is_zero = 0;
+        a.r0_given = c->h_out->r0;
+        a.maxit = maxit - done_it;
+    }
 }
 
 static int run_krylov(sem_ctx* c, int op, const double* pot, double alpha, double* const x[2],
@@ -1553,7 +1596,7 @@ static int run_krylov(sem_ctx* c, int op, const double* pot, double alpha, doubl
     int grid = 0, kmax = 1;
     size_t smem = 0;
     dispatch_n(c->N, [&](auto nv) {
-        grid = solver_plan<decltype(nv)::value>(op, false, c->E, c->sms, kSolverSmemBudget, &kmax, &smem);
+        grid = solver_plan<decltype(nv)::value>(op, SOLVE_FP64, c->E, c->sms, kSolverSmemBudget, &kmax, &smem);
         return cudaSuccess;
     });
     if (grid <= 0) return fail(SEM_ERR_CUDA, "could not size the cooperative grid");

@@ -58,7 +58,8 @@ struct DevMesh {
     const double *g11 = nullptr, *g12 = nullptr, *g22 = nullptr, *mass = nullptr;
     const float *g11f = nullptr, *g12f = nullptr, *g22f = nullptr, *massf = nullptr;
     // element fast-diagonalisation preconditioner: 1-D GLL generalised
-    // eigenvectors S(i,k) at [i*N+k] (K s = lambda W s, S^T W S = I), their
+    // eigenvectors S(i,k) at [i*N+k] (K s = lambda W s, S^T W S = I; the
+    // (N+1)/2 even modes first, then the odd ones), their
     // eigenvalues, and per element {ax ay, ay/ax, ax/ay, 0} of the element's
     // rectangle approximation (half widths ax, ay)
     const double* fdmS64 = nullptr;
@@ -95,7 +96,8 @@ struct DevMesh {
     const int* bulk_pair_ptr = nullptr;
     const int* bulk_pairs = nullptr;
     int* dev_err = nullptr;  // set by a kernel whose bounded wait expired (pipelined apply)
-    const double* Dh = nullptr;  // host copy of D, row-major (launchers that pass D by value)
+    const double* Dh = nullptr;  // host copies of D and of the preconditioner basis S, row-major
+    const double* Sh = nullptr;  // (launchers that pass them by value)
     // on-the-fly geometry of the FP32 Res apply: per element {x1-x0, x2-x3,
     // x3-x0, x2-x1, y1-y0, y2-y3, y3-y0, y2-y1} (FP32), the host LGL nodes and
     // weights, and the metric convention (1: SEM_FLAG_METRIC_CORRECTED)
@@ -121,7 +123,9 @@ struct SolveOut {
     int status;      // 0 or SEM_ERR_DEVICE_WAIT
     int inner_iters; // mixed mode: total FP32 iterations
     int sweeps;      // mixed mode: refinement sweeps
-    int pad;
+    int fallback;    // resident kernel: the inner solver gave up, continue with MINRES
+    unsigned epoch;  // resident kernel: last epoch used on the exchange words
+    double r0;       // mixed mode: the norm the stopping test is relative to
 };
 
 template <typename T>
@@ -149,6 +153,7 @@ struct SolveArgs {
     int rel_to_b;     // mixed solver: stop on |r| < tol |b| + tol instead of tol |r_0| + tol
                       // (the same test when x_0 = 0; used with warm starts)
     long long timeout_ns;
+    double r0_given;  // mixed solver: > 0 replaces the norm the stopping test is relative to
     GridSync* sync;
     SolveOut* out;
 };
@@ -165,6 +170,7 @@ struct MixedArgs {
     const float* pot32;  // FP32 copy of the potential (V or c)
     const float* pinv32; // diagonal preconditioner P^-1 (continuous format), or null
     int fdm;             // element fast-diagonalisation preconditioner (Res only; uses KrylovWork::Z)
+    int minres;          // with fdm: MINRES from the first sweep on
     int fused;           // inner solve with the single-barrier MINRES iteration (Res only)
     double outer_scale;  // refinement stops at |r| < outer_scale * (tol |r0| + tol)
     int adaptive;        // inner tolerance of a sweep no tighter than the outer test needs
@@ -250,8 +256,9 @@ cudaError_t launch_learn(const DevMesh& m, const LearnArgs& a, cudaStream_t st);
 // launch_solver runs MINRES (op OP_RES/OP_HELM), PCG (OP_LAPLACE) or, when
 // mx is given, the mixed-precision refinement.  work points to a
 // KrylovWork<double> (FP64 solvers) or KrylovWork<float> (mixed).
+enum SolveKind : int { SOLVE_FP64 = 0, SOLVE_MIXED = 1, SOLVE_MIXED_FDM = 2 };
 template <int N>
-int solver_plan(int op, bool mixed, int E, int sms, size_t smem_budget, int* kmax, size_t* smem);
+int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax, size_t* smem);
 template <int N>
 cudaError_t launch_solver(const DevMesh& m, const SolveArgs& a, const void* work, const MixedArgs* mx,
                           int grid, size_t smem, cudaStream_t st);
@@ -259,17 +266,16 @@ cudaError_t launch_solver(const DevMesh& m, const SolveArgs& a, const void* work
 // (Res operator, element preconditioner; sem_resident.cuh), instantiated for
 // N = 5, 7, 9, 11.  resident_plan returns false when a block's share of the
 // mesh does not fit on chip; then the staged kernel (launch_solver) is used.
-// D32h / S32h: host FP32 copies of D and of the preconditioner basis S, both
-// row-major.  slots: 2 * grid * RESIDENT_SLOT_STRIDE words; xa, xb: 2 n words
-// each (the tagged ring exchange); all cleared before the launch.
-constexpr int RESIDENT_SLOT_STRIDE = 16;  // one 128-byte line per block's all-reduce word
+// slots: 2 * grid * RESIDENT_SLOT_STRIDE words; xa, xb: n pairs of words each
+// (the tagged ring exchange); epoch0: the last epoch used on them (0 for
+// cleared words), SolveOut::epoch the one this launch ended with.
+constexpr int RESIDENT_SLOT_STRIDE = 16;  // one 128-byte line per block's all-reduce words
 template <int N>
 bool resident_plan(int E, int sms, size_t smem_budget, int* grid, int* st, int* kmax64, size_t* smem);
 template <int N>
 cudaError_t launch_resident(const DevMesh& m, const SolveArgs& a, const KrylovWork<float>& w, const MixedArgs& mx,
-                            const float* D32h, const float* S32h, int st, unsigned long long* slots,
-                            unsigned long long* xa, unsigned long long* xb, int grid, size_t smem,
-                            cudaStream_t stream);
+                            int st, unsigned long long* slots, void* xa, void* xb, unsigned epoch0, int grid,
+                            size_t smem, cudaStream_t stream);
 
 }  // namespace semgb
 

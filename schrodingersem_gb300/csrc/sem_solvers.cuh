@@ -14,6 +14,7 @@
 #include <cfloat>
 #include <limits>
 
+#include "sem_cg.cuh"
 #include "sem_device.cuh"
 
 namespace semgb {
@@ -786,15 +787,26 @@ __global__ void __launch_bounds__(SOLVER_TPB, 1)
 // [eb, ee): the cooperative kernel gives every block a slice of one mesh
 // (grid barriers and grid reductions); the batched kernel gives one block a
 // whole instance (a.sync == nullptr: block barriers and block reductions).
-// Returns false when a wait timed out.  `leader` writes a.out.  LEAN
-// compiles only the unpreconditioned and element-preconditioned inner
-// iterations (the batched kernels).
-template <int N, int OP, bool LEAN = false>
+// Returns false when a wait timed out.  `leader` writes a.out.
+//
+// With the element preconditioner (FDM kinds) the inner solver is the
+// complex-symmetric conjugate gradient iteration of cg_core, whose
+// correction is taken when it is finite; when it breaks down, stalls or fails
+// to halve the true residual, the remaining sweeps use the preconditioned
+// MINRES, which cannot break down.
+enum MixedKind : int {
+    MIXED_PLAIN = 0,  // no or diagonal preconditioner
+    MIXED_BATCH = 1,  // batched instances: no preconditioner or the element one
+    MIXED_FDM = 2     // element preconditioner
+};
+template <int N, int OP, int KIND>
 __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a, const KrylovWork<float>& w,
                                             const MixedArgs& mx, int eb, int ee, bool leader,
                                             unsigned char* smraw, double* red, MinresScal<float>& sc,
-                                            double* sweep_state, float* fdmS, float* fdmL)
+                                            double* sweep_state, float* fdmS, float* fdmL,
+                                            const CgTab<N>* tab = nullptr)
 {
+    static_assert(KIND == MIXED_PLAIN || OP == OP_RES, "the element preconditioner is the stage operator's");
     constexpr int NN = N * N;
     constexpr int NC = op_nc<OP>();
     double* sm64 = (double*)smraw;
@@ -809,6 +821,8 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
     bool ok = true;
     int sweep = 0, inner_total = 0;
     bool conv = false;
+    bool cg = KIND != MIXED_PLAIN && mx.fdm && !mx.minres;  // the same on every thread
+    double last_rn = 0.0;
     for (;;) {
         // ---- FP64 residual r = unmask(b) - DSS(A_local(unmask(x)))
         const bool applied = (sweep > 0) || !a.x_is_zero;
@@ -857,7 +871,7 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
         if (!ok) return false;
         if (threadIdx.x == 0) {
             const double rn = sqrt(rr);
-            if (sweep == 0) sweep_state[0] = want_b ? sqrt(bbv) : rn;
+            if (sweep == 0) sweep_state[0] = a.r0_given > 0.0 ? a.r0_given : want_b ? sqrt(bbv) : rn;
             sweep_state[1] = rn;
             const double r0 = sweep_state[0];
             const bool c = rn < mx.outer_scale * (a.tol * r0 + a.tol);
@@ -869,12 +883,7 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
             break;
         }
         // ---- FP32 inner solve A d = r (relative tolerance inner_tol)
-        load_dmat_raw<N, float>(sm32, m);
-        if (OP == OP_RES && mx.fdm) load_fdm_basis<N, float>(fdmS, fdmL, m);
-        __syncthreads();
         const double* r64c[2] = {mx.r64[0], mx.r64[1]};
-        auto rhs = [&](const NodeInfo&, int, long long flat, int c) -> float { return (float)r64c[c][flat]; };
-        MinresOut ir{};
         const int budget = min(mx.inner_maxit, a.maxit - inner_total);
         // the inner solve reduces by inner_tol, or (last sweep) by no more
         // than the outer test still needs, with a margin for the FP32
@@ -884,9 +893,45 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
             const double need = mx.outer_scale * (a.tol * sweep_state[0] + a.tol) / sweep_state[1];
             itol = fmax(itol, fmin(0.3 * need, 0.5));
         }
+        if constexpr (KIND != MIXED_PLAIN) {
+            const double rn = sweep_state[1];
+            if (cg && sweep > 0 && !(rn < 0.5 * last_rn)) cg = false;
+            last_rn = rn;
+            if (mx.fdm) {
+                load_fdm_basis<N, float>(fdmS, fdmL, m);
+                __syncthreads();
+            }
+            if (cg) {
+                const double inv = 1.0 / rn;
+                CgOut cr{};
+                if (!cg_core<N>(smraw, kmax, m, *tab, mx.pot32, (float)a.alpha, eb, ee, w, a.sync, a.timeout_ns, slot,
+                                [&](long long flat, int c) -> float { return (float)(r64c[c][flat] * inv); }, mx.x32,
+                                budget, (float)itol, fdmL, cr))
+                    return false;
+                inner_total += cr.it;
+                ++sweep;
+                if (cr.usable) {  // x += d (FP64, owner copies)
+#pragma unroll 4
+                    for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
+                        const int e = (int)(idx / NN);
+                        const int node = (int)(idx - (long long)e * NN);
+                        if (!ni_owner(node_info<N>(m, e, node % N, node / N))) continue;
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) xp[c][idx] += (double)mx.x32[c][idx] * rn;
+                    }
+                }
+                cg = cr.usable && cr.conv;
+                if (!grid_barrier(a.sync, a.timeout_ns)) return false;
+                continue;
+            }
+        }
+        load_dmat_raw<N, float>(sm32, m);
+        __syncthreads();
+        auto rhs = [&](const NodeInfo&, int, long long flat, int c) -> float { return (float)r64c[c][flat]; };
+        MinresOut ir{};
         bool okc = false;
         bool done_fdm = false;
-        if constexpr (OP == OP_RES) {
+        if constexpr (KIND != MIXED_PLAIN) {
             if (mx.fdm) {
                 okc = minres_core<N, float, OP, 2>(sm32, kmax, red, sc, m, mx.pot32, (float)a.alpha, eb, ee, w,
                                                    a.sync, a.timeout_ns, slot, rhs, mx.x32, budget, itol,
@@ -894,8 +939,8 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
                 done_fdm = true;
             }
         }
-        if (done_fdm) {
-        } else if constexpr (LEAN) {  // batched instances: no preconditioner or the element one
+        if (done_fdm || KIND == MIXED_FDM) {
+        } else if constexpr (KIND != MIXED_PLAIN) {
             okc = minres_core<N, float, OP, 0>(sm32, kmax, red, sc, m, mx.pot32, (float)a.alpha, eb, ee, w, a.sync,
                                                a.timeout_ns, slot, rhs, mx.x32, budget, itol, 0.0, ir,
                                                (const float*)nullptr);
@@ -945,10 +990,27 @@ __global__ void __launch_bounds__(SOLVER_TPB, 1)
     __shared__ double red[34];
     __shared__ MinresScal<float> sc;
     __shared__ double sweep_state[3];  // r0, |r|, done
+    int eb, ee;
+    block_range(m.E, eb, ee);
+    mixed_solve<N, OP, MIXED_PLAIN>(m, a, w, mx, eb, ee, blockIdx.x == 0, smraw, red, sc, sweep_state, nullptr,
+                                    nullptr);
+}
+
+// the same with the element preconditioner
+constexpr int CG_TPB = 256;
+template <int N>
+__global__ void __launch_bounds__(CG_TPB, 2)
+    k_cg_mixed(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ CgTab<N> tab)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ double red[34];
+    __shared__ MinresScal<float> sc;
+    __shared__ double sweep_state[3];  // r0, |r|, done
     __shared__ float fdmS[N * N], fdmL[N];  // element preconditioner basis
     int eb, ee;
     block_range(m.E, eb, ee);
-    mixed_solve<N, OP>(m, a, w, mx, eb, ee, blockIdx.x == 0, smraw, red, sc, sweep_state, fdmS, fdmL);
+    mixed_solve<N, OP_RES, MIXED_FDM>(m, a, w, mx, eb, ee, blockIdx.x == 0, smraw, red, sc, sweep_state, fdmS, fdmL,
+                                      &tab);
 }
 
 // --------------------------------------------------------- persistent PCG
@@ -1089,18 +1151,20 @@ __global__ void __launch_bounds__(SOLVER_TPB, 1)
 
 // dynamic shared memory of a solver kernel for a given staging capacity
 template <int N>
-size_t solver_smem(int op, bool mixed, int kmax)
+size_t solver_smem(int op, int kind, int kmax)
 {
     const bool two = (op == OP_RES);
     const size_t d = two ? range_smem_bytes<N, double, OP_RES>(kmax) : range_smem_bytes<N, double, OP_HELM>(kmax);
-    const size_t f = two ? range_smem_bytes<N, float, OP_RES>(kmax) : range_smem_bytes<N, float, OP_HELM>(kmax);
-    return mixed ? (d > f ? d : f) : d;
+    const size_t c = kind == SOLVE_MIXED_FDM ? cg_smem_bytes<N>(kmax) : 0;
+    return d > c ? d : c;
 }
 
 template <int N>
-static const void* solver_fn(int op, bool mixed)
+static const void* solver_fn(int op, int kind)
 {
-    if (mixed) return op == OP_RES ? (const void*)k_minres_mixed<N, OP_RES> : (const void*)k_minres_mixed<N, OP_HELM>;
+    if (kind == SOLVE_MIXED_FDM) return (const void*)k_cg_mixed<N>;
+    if (kind == SOLVE_MIXED)
+        return op == OP_RES ? (const void*)k_minres_mixed<N, OP_RES> : (const void*)k_minres_mixed<N, OP_HELM>;
     switch (op) {
         case OP_RES: return (const void*)k_minres<N, double, OP_RES>;
         case OP_HELM: return (const void*)k_minres<N, double, OP_HELM>;
@@ -1108,22 +1172,32 @@ static const void* solver_fn(int op, bool mixed)
     }
 }
 
-// Plan a cooperative launch: one block per SM (fewer for small meshes) and
-// the largest staging capacity kmax <= the block's element count that fits
-// in smem_budget bytes.  Returns the grid, or 0 on failure.
+// Plan a cooperative launch: one block per SM (fewer for small meshes), two
+// smaller ones for the element-preconditioned kernel on meshes that give each
+// SM several passes, so that one block's loads overlap the other's passes,
+// and the largest staging capacity kmax <= the block's element count that
+// fits in smem_budget bytes per SM.  Returns the grid, or 0 on failure.
 template <int N>
-int solver_plan(int op, bool mixed, int E, int sms, size_t smem_budget, int* kmax_out, size_t* smem_out)
+int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_out, size_t* smem_out)
 {
-    int grid = E < sms ? E : sms;
+    const bool fdm = kind == SOLVE_MIXED_FDM;
+    int per = 1;
+    if (fdm && (long long)E * N * N >= 4096ll * sms) per = 2;
+    int grid = E < per * sms ? E : per * sms;
     if (grid < 1) grid = 1;
     int kmax = (E + grid - 1) / grid;
-    while (kmax > 1 && solver_smem<N>(op, mixed, kmax) > smem_budget) kmax = (kmax + 1) / 2;
-    const size_t smem = solver_smem<N>(op, mixed, kmax);
-    const void* fn = solver_fn<N>(op, mixed);
+    const int share = kmax;
+    while (kmax > 1 && solver_smem<N>(op, kind, kmax) > smem_budget / per)
+        kmax = fdm ? kmax - 1 : (kmax + 1) / 2;
+    if (fdm) kmax = (share + (share + kmax - 1) / kmax - 1) / ((share + kmax - 1) / kmax);  // even passes
+    const size_t smem = solver_smem<N>(op, kind, kmax);
+    const void* fn = solver_fn<N>(op, kind);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SOLVER_TPB, smem) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : SOLVER_TPB, smem) != cudaSuccess ||
+        per_sm < 1)
         return 0;
+    if (grid > per_sm * sms) grid = per_sm * sms;
     *kmax_out = kmax;
     *smem_out = smem;
     return grid;
@@ -1135,11 +1209,17 @@ cudaError_t launch_solver(const DevMesh& m, const SolveArgs& a, const void* work
 {
     DevMesh mm = m;
     SolveArgs aa = a;
-    const bool mixed = mx != nullptr;
-    const void* fn = solver_fn<N>(a.op, mixed);
-    if (mixed) {
+    const int kind = !mx ? SOLVE_FP64 : mx->fdm ? SOLVE_MIXED_FDM : SOLVE_MIXED;
+    const void* fn = solver_fn<N>(a.op, kind);
+    if (kind != SOLVE_FP64) {
         KrylovWork<float> ww = *(const KrylovWork<float>*)work;
         MixedArgs xx = *mx;
+        if (kind == SOLVE_MIXED_FDM) {
+            if (!m.Dh || !m.Sh) return cudaErrorInvalidValue;
+            CgTab<N> tab = cg_table<N>(m);
+            void* args[] = {&mm, &aa, &ww, &xx, &tab};
+            return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(CG_TPB), args, smem, st);
+        }
         void* args[] = {&mm, &aa, &ww, &xx};
         return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(SOLVER_TPB), args, smem, st);
     }
