@@ -223,23 +223,6 @@ template <int N>
 struct DMat2 {
     unsigned long long d[N * N];
 };
-__device__ __forceinline__ unsigned long long f2pack(float a, float b)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2unpack(unsigned long long v, float& a, float& b)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long f2fma(unsigned long long a, unsigned long long b, unsigned long long c)
-{
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
 // Line contraction of both Res components: oa[o] = ca[o] + sum_k M(o,k) a[k]
 // (and b) with M = D (TR false) or D^T (TR true), k ascending; paired FP32
 // FMAs when F2 (measured faster for N <= 11, slower above), else scalar.

@@ -83,7 +83,7 @@ namespace semgb {
 template <int N>
 __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned char* smraw, double* red,
                               MinresScal<float>& sc, double* sweep_state, float* fdmS, float* fdmL,
-                              const CgTab<N>& tab)
+                              const EoD<N, double>& et, const CgTab<N>& tab)
 {
     constexpr int NN = N * N;
     const DevMesh& m = I.m;
@@ -149,7 +149,8 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
     mx.fused = 0;
     mx.outer_scale = ba.outer_scale;
     mx.adaptive = 1;
-    mixed_solve<N, OP_RES, MIXED_BATCH>(m, a, I.w, mx, 0, m.E, true, smraw, red, sc, sweep_state, fdmS, fdmL, &tab);
+    mixed_solve<N, OP_RES, MIXED_BATCH>(m, a, I.w, mx, 0, m.E, true, smraw, red, sc, sweep_state, fdmS, fdmL, et,
+                                     &tab);
     // unmask(p) (schrodinger.hpp:105-106): owner copies are never written here
     for (long long idx = threadIdx.x; idx < n; idx += blockDim.x) {
         const int e = (int)(idx / NN);
@@ -170,7 +171,7 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
 
 // one time step of every instance in ba.order (all of degree N)
 template <int N>
-__global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_bdf2(BatchArgs ba, const __grid_constant__ CgTab<N> tab)
+__global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_bdf2(BatchArgs ba, const __grid_constant__ EoD<N, double> et, const __grid_constant__ CgTab<N> tab)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[34];
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_bdf2(BatchArgs ba, const
         if (q >= ba.n) break;
         if (threadIdx.x == 0) I = ba.inst[ba.order[q]];
         __syncthreads();
-        bdf2_instance<N>(I, ba, smraw, red, sc, sweep_state, fdmS, fdmL, tab);
+        bdf2_instance<N>(I, ba, smraw, red, sc, sweep_state, fdmS, fdmL, et, tab);
         __syncthreads();
     }
 }
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_probe(const BatchInst* i
         for (int r = 0; r < reps; ++r)
             for (int e0 = 0; e0 < m.E; e0 += kmax)
                 apply_range<N, float, OP_RES>(
-                    sm, kmax, fac, I.pot32, 0.01f, e0, min(kmax, m.E - e0),
+                    sm, kmax, nullptr, fac, I.pot32, 0.01f, e0, min(kmax, m.E - e0),
                     [&](int, int, int, long long flat, float* u) {
                         u[0] = I.w.L[0][flat];
                         u[1] = I.w.L[0][n + flat];
@@ -246,7 +247,7 @@ cudaError_t batch_prepare(size_t smem, int* per_sm)
 template <int N>
 cudaError_t batch_launch_step(const BatchArgs& ba, const DevMesh& m0, int grid, size_t smem, cudaStream_t st)
 {
-    k_batch_bdf2<N><<<grid, BATCH_TPB, smem, st>>>(ba, cg_table<N>(m0));
+    k_batch_bdf2<N><<<grid, BATCH_TPB, smem, st>>>(ba, eo_d_table<N, double>(m0.Dh), cg_table<N>(m0));
     return cudaGetLastError();
 }
 

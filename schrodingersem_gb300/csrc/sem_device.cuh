@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "sem_internal.h"
+#include "sem_lines.cuh"
 
 namespace semgb {
 
@@ -147,25 +148,34 @@ __device__ __forceinline__ T dss_value(const DevMesh& m, const T* Y, const NodeI
         if (ni_lone(ni)) return own;
         return own + ldcg(Y + ((long long)sb + (long long)ni.k * ss));  // owner + other in either copy: same bits
     }
-    const int* cl = m.corner_nb + (size_t)(4 * e + ni.sc) * CORNER_NB_MAX;
-    int q[CORNER_NB_MAX];
-#pragma unroll
-    for (int k = 0; k < CORNER_NB_MAX; ++k) q[k] = __ldg(cl + k);
+    // the copy list as two 16-byte loads; more than four copies are rare, so a
+    // warp seldom takes the second half (an FP64 addition costs a whole warp's
+    // issue for one corner lane)
+    const int4* cl = reinterpret_cast<const int4*>(m.corner_nb + (size_t)(4 * e + ni.sc) * CORNER_NB_MAX);
+    const int4 qa = __ldg(cl), qb = __ldg(cl + 1);
     if (ni_boundary(ni)) return MODE == DSS_SUM ? own : T(0);
     if (MODE == DSS_MASK && !ni_owner(ni)) return T(0);
     T s = T(0);  // csum = 0, then += in connected_elements order (global_sum.hpp:56-59)
-    if (q[0] == -2) {  // more copies than the table holds
+    if (qa.x == -2) {  // more copies than the table holds
         const int node = __ldg(m.corner_node + 4 * e + ni.sc);
         const int q0 = __ldg(m.node_ptr + node), q1 = __ldg(m.node_ptr + node + 1);
         for (int k = q0; k < q1; ++k) s += ldcg(Y + __ldg(m.node_flat + k));
         return s;
     }
+    const int q[CORNER_NB_MAX] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
     T v[CORNER_NB_MAX];
 #pragma unroll
-    for (int k = 0; k < CORNER_NB_MAX; ++k) v[k] = q[k] >= 0 ? ldcg(Y + q[k]) : T(0);
+    for (int k = 0; k < 4; ++k) v[k] = q[k] >= 0 ? ldcg(Y + q[k]) : T(0);
 #pragma unroll
-    for (int k = 0; k < CORNER_NB_MAX; ++k)
+    for (int k = 0; k < 4; ++k)
         if (q[k] >= 0) s += v[k];
+    if (q[4] >= 0) {
+#pragma unroll
+        for (int k = 4; k < CORNER_NB_MAX; ++k) v[k] = q[k] >= 0 ? ldcg(Y + q[k]) : T(0);
+#pragma unroll
+        for (int k = 4; k < CORNER_NB_MAX; ++k)
+            if (q[k] >= 0) s += v[k];
+    }
     return s;
 }
 
@@ -294,10 +304,16 @@ __device__ __forceinline__ void apply_chunk(ApplySmem<N, T, OP>& s, const Fac<T>
 // staged range are issued before the first barrier, so one pass costs one
 // memory latency instead of one per small chunk.
 // Shared layout (type T): D[NN] | u[NC][kmax*NN] | f1[NC][kmax*NN] | f2[NC][kmax*NN]
+// (FP64: element stride line_es(N) instead of NN)
+template <int N, typename T>
+__host__ __device__ constexpr int range_es()
+{
+    return sizeof(T) == 8 ? line_es(N) : N * N;
+}
 template <int N, typename T, int OP>
 __host__ __device__ constexpr size_t range_smem_bytes(int kmax)
 {
-    return sizeof(T) * ((size_t)N * N + 3ull * op_nc<OP>() * (size_t)kmax * N * N);
+    return sizeof(T) * ((size_t)N * N + 3ull * op_nc<OP>() * (size_t)kmax * range_es<N, T>());
 }
 
 template <int N, typename T>
@@ -308,21 +324,192 @@ __device__ __forceinline__ void load_dmat_raw(T* sm, const DevMesh& m)
 }
 
 template <int N, typename T, int OP, bool POST, class Load, class Post, class Store>
-__device__ __forceinline__ void apply_range_post(T* sm, int kmax, const Fac<T>& fac,
+__device__ __forceinline__ void apply_range_post(T* sm, int kmax, const EoD<N, double>* et, const Fac<T>& fac,
                                                  const T* __restrict__ pot, T alpha, int e0, int ne,
                                                  Load&& load, Post&& post, Store&& store);
 
 // One block-wide pass over elements [e0, e0+ne), ne <= kmax.  Every thread
 // of the block must call it.  Same operator and callbacks as apply_chunk.
+// FP64 contracts lines by parity with the table et (FP32 ignores it).
 template <int N, typename T, int OP, class Load, class Store>
-__device__ __forceinline__ void apply_range(T* sm, int kmax, const Fac<T>& fac,
+__device__ __forceinline__ void apply_range(T* sm, int kmax, const EoD<N, double>* et, const Fac<T>& fac,
                                             const T* __restrict__ pot, T alpha, int e0, int ne,
                                             Load&& load, Store&& store)
 {
     apply_range_post<N, T, OP, false>(
-        sm, kmax, fac, pot, alpha, e0, ne,
+        sm, kmax, et, fac, pot, alpha, e0, ne,
         [&](int e, int i, int j, long long flat, T* u, T*) { load(e, i, j, flat, u); },
         [&](int, int, int, long long, const T*, const T*) {}, store);
+}
+
+// factors of node `node` of staged element le: from global memory (elements
+// from e0 on), or from shared planes laid out like the inputs
+template <int N>
+struct Gg64 {
+    const double *a, *b, *c;
+    __device__ __forceinline__ Gg64(const Fac<double>& f, int e0)
+        : a(f.g11 + (long long)e0 * N * N), b(f.g12 + (long long)e0 * N * N), c(f.g22 + (long long)e0 * N * N)
+    {
+    }
+    __device__ __forceinline__ void at(int le, int node, double& g11, double& g12, double& g22) const
+    {
+        const int q = le * (N * N) + node;
+        g11 = __ldg(a + q);
+        g12 = __ldg(b + q);
+        g22 = __ldg(c + q);
+    }
+};
+template <int N>
+struct Gs64 {
+    const double* g;  // g11, g12, g22 planes, st apart
+    int st;
+    __device__ __forceinline__ void at(int le, int node, double& g11, double& g12, double& g22) const
+    {
+        const int q = le * line_es(N) + node;
+        g11 = g[q];
+        g12 = g[st + q];
+        g22 = g[2 * st + q];
+    }
+};
+
+// The FP64 element operator on lines (GB300's FP64 pipe issues one warp
+// instruction per 16 cycles and SM, so an FP64 pass costs what it issues:
+// the parity split takes 56 instead of 81 operations per line at N = 9).
+// su holds the inputs of ne elements (NC planes of st values, line_es apart);
+// on return s1 holds D^T f1 and s2 D^T f2, whose sum is the weak Laplacian.
+// Row passes take the element fastest (no bank conflicts), the column pass the
+// position fastest (neighbouring lanes read neighbouring factors).
+template <int N, int NC, class G>
+__device__ __forceinline__ void laplace64(const EoD<N, double>& t, const double* su, double* s1, double* s2, int st,
+                                          const G& fac, int ne)
+{
+    constexpr int ES = line_es(N);
+    const int per = ne * N;
+    const LineNe nb = line_ne(ne);
+    for (int L = threadIdx.x; L < NC * per; L += blockDim.x) {  // u_xi
+        const int c = NC == 2 && L >= per ? 1 : 0;
+        int pos, le;
+        line_of(L - c * per, nb, pos, le);
+        const int o = c * st + le * ES + pos * N;
+        double u[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) u[k] = su[o + k];
+        eo_d<N, false>(t, u, u);
+#pragma unroll
+        for (int k = 0; k < N; ++k) s1[o + k] = u[k];
+    }
+    __syncthreads();
+    for (int L = threadIdx.x; L < NC * per; L += blockDim.x) {  // u_eta, fluxes, D^T f2
+        const int c = NC == 2 && L >= per ? 1 : 0;
+        const int le = (L - c * per) / N, pos = (L - c * per) - le * N;
+        const int o = c * st + le * ES + pos;
+        double us[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) us[k] = su[o + k * N];
+        eo_d<N, false>(t, us, us);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const double ur = s1[o + k * N];
+            double g11, g12, g22;
+            fac.at(le, pos + k * N, g11, g12, g22);
+            s1[o + k * N] = g11 * ur - g12 * us[k];
+            us[k] = g22 * us[k] - g12 * ur;
+        }
+        eo_d<N, true>(t, us, us);
+#pragma unroll
+        for (int k = 0; k < N; ++k) s2[o + k * N] = us[k];
+    }
+    __syncthreads();
+    for (int L = threadIdx.x; L < NC * per; L += blockDim.x) {  // D^T f1
+        const int c = NC == 2 && L >= per ? 1 : 0;
+        int pos, le;
+        line_of(L - c * per, nb, pos, le);
+        const int o = c * st + le * ES + pos * N;
+        double f[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) f[k] = s1[o + k];
+        eo_d<N, true>(t, f, f);
+#pragma unroll
+        for (int k = 0; k < N; ++k) s1[o + k] = f[k];
+    }
+    __syncthreads();
+}
+
+// The same for a few elements (at most four values per thread): one thread per
+// node and component.  A warp instruction costs the FP64 pipe the same for one
+// lane as for 32, so with little work the length of a thread's chain sets the
+// time, and 4N products of a node are shorter than a line's (N = 5, 9: 20 and
+// 36 products against 80 and 224 operations).  D row-major in shared memory;
+// s2 is zero on return.
+//
+// laplace64_nodes: the form whose instruction count per FP64 pipe (four per
+// SM, warps spread over them in turn) is smaller
+__host__ __device__ constexpr int laplace64_cost(int N, int nc, int ne, bool nodes)
+{
+    const int H = N / 2, C = (N + 1) / 2, values = (nc * ne * N * N + 127) / 128;
+    return nodes ? values * (4 * N + 9) : (nc * ne * N + 127) / 128 * (8 * H * C + 16 * H + 4 * N) + 4 * values;
+}
+__host__ __device__ constexpr bool laplace64_nodes(int N, int nc, int ne, int threads)
+{
+    return nc * ne * N * N <= 4 * threads && laplace64_cost(N, nc, ne, true) < laplace64_cost(N, nc, ne, false);
+}
+template <int N, int NC, class G>
+__device__ __forceinline__ void laplace64_small(const double* D, const double* su, double* s1, double* s2, int st,
+                                                const G& fac, int ne)
+{
+    constexpr int NN = N * N, ES = line_es(N);
+    const int total = ne * NN;
+    double lap[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int t = threadIdx.x + h * blockDim.x;
+        if (t < NC * total) {
+            const int c = NC == 2 && t >= total ? 1 : 0;
+            const int le = (t - c * total) / NN, node = (t - c * total) - le * NN;
+            const int i = node % N, j = node / N;
+            double g11, g12, g22;
+            fac.at(le, node, g11, g12, g22);
+            const double* u = su + c * st + le * ES;
+            double ur = 0.0, us = 0.0;
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                ur = fma(D[i * N + k], u[k + j * N], ur);
+                us = fma(D[j * N + k], u[i + k * N], us);
+            }
+            s1[c * st + le * ES + node] = g11 * ur - g12 * us;
+            s2[c * st + le * ES + node] = g22 * us - g12 * ur;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int t = threadIdx.x + h * blockDim.x;
+        if (t < NC * total) {
+            const int c = NC == 2 && t >= total ? 1 : 0;
+            const int le = (t - c * total) / NN, node = (t - c * total) - le * NN;
+            const int i = node % N, j = node / N;
+            const double* f1 = s1 + c * st + le * ES + j * N;
+            const double* f2 = s2 + c * st + le * ES + i;
+            double a = 0.0;
+#pragma unroll
+            for (int k = 0; k < N; ++k) a = fma(D[k * N + i], f1[k], a);
+#pragma unroll
+            for (int k = 0; k < N; ++k) a = fma(D[k * N + j], f2[k * N], a);
+            lap[h] = a;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int t = threadIdx.x + h * blockDim.x;
+        if (t < NC * total) {
+            const int c = NC == 2 && t >= total ? 1 : 0;
+            const int le = (t - c * total) / NN, node = (t - c * total) - le * NN;
+            s1[c * st + le * ES + node] = lap[h];
+            s2[c * st + le * ES + node] = 0.0;
+        }
+    }
+    __syncthreads();
 }
 
 // apply_range with the input split in two: load(e,i,j,flat,u,aux) computes
@@ -331,14 +518,16 @@ __device__ __forceinline__ void apply_range(T* sm, int kmax, const Fac<T>& fac,
 // caller's global stores for the node (aux is parked in the flux area, free
 // until the flux phase).
 template <int N, typename T, int OP, bool POST, class Load, class Post, class Store>
-__device__ __forceinline__ void apply_range_post(T* sm, int kmax, const Fac<T>& fac,
+__device__ __forceinline__ void apply_range_post(T* sm, int kmax, const EoD<N, double>* et, const Fac<T>& fac,
                                                  const T* __restrict__ pot, T alpha, int e0, int ne,
                                                  Load&& load, Post&& post, Store&& store)
 {
     constexpr int NN = N * N;
     constexpr int NC = op_nc<OP>();
+    constexpr bool LINES = sizeof(T) == 8 && OP != OP_MASS;
+    constexpr int ES = range_es<N, T>();
     const int total = ne * NN;
-    const int st = kmax * NN;
+    const int st = kmax * ES;
     const T* D = sm;
     T* su = sm + NN;
     T* sf1 = su + NC * st;
@@ -353,8 +542,8 @@ __device__ __forceinline__ void apply_range_post(T* sm, int kmax, const Fac<T>& 
         load(e, node % N, node / N, (long long)e * NN + node, u, aux);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            su[c * st + t] = u[c];
-            if (POST) sf1[c * st + t] = aux[c];
+            su[c * st + le * ES + node] = u[c];
+            if (POST) sf1[c * st + le * ES + node] = aux[c];
         }
     }
     if (POST) {
@@ -365,8 +554,8 @@ __device__ __forceinline__ void apply_range_post(T* sm, int kmax, const Fac<T>& 
             T u[NC], aux[NC];
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                u[c] = su[c * st + t];
-                aux[c] = sf1[c * st + t];
+                u[c] = su[c * st + le * ES + node];
+                aux[c] = sf1[c * st + le * ES + node];
             }
             post(e, node % N, node / N, (long long)e * NN + node, u, aux);
         }
@@ -379,15 +568,21 @@ __device__ __forceinline__ void apply_range_post(T* sm, int kmax, const Fac<T>& 
             const int e = e0 + le;
             const long long flat = (long long)e * NN + node;
             T o[NC];
-            o[0] = __ldg(fac.mass + flat) * su[t];
+            o[0] = __ldg(fac.mass + flat) * su[le * ES + node];
             store(e, node % N, node / N, flat, o);
         }
         __syncthreads();
         return;
     }
     // 2. contravariant fluxes
+    if constexpr (LINES) {
+        if (laplace64_nodes(N, NC, ne, blockDim.x))
+            laplace64_small<N, NC>(D, su, sf1, sf2, st, Gg64<N>(fac, e0), ne);
+        else
+            laplace64<N, NC>(*et, su, sf1, sf2, st, Gg64<N>(fac, e0), ne);
+    }
 #pragma unroll 4
-    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    for (int t = threadIdx.x; !LINES && t < total; t += blockDim.x) {
         const int le = t / NN;
         const int node = t - le * NN;
         const int i = node % N, j = node / N;
@@ -406,7 +601,7 @@ __device__ __forceinline__ void apply_range_post(T* sm, int kmax, const Fac<T>& 
             sf2[c * st + t] = g22 * us - g12 * ur;
         }
     }
-    __syncthreads();
+    if (!LINES) __syncthreads();
     // 3. weak divergence + mass/potential terms
 #pragma unroll 4
     for (int t = threadIdx.x; t < total; t += blockDim.x) {
@@ -421,15 +616,20 @@ __device__ __forceinline__ void apply_range_post(T* sm, int kmax, const Fac<T>& 
         T lap[NC], u[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            const T* f1 = sf1 + c * st + le * NN;
-            const T* f2 = sf2 + c * st + le * NN;
-            T a = T(0);
+            const int q = c * st + le * ES + node;
+            if constexpr (LINES) {
+                lap[c] = sf1[q] + sf2[q];
+            } else {
+                const T* f1 = sf1 + c * st + le * NN;
+                const T* f2 = sf2 + c * st + le * NN;
+                T a = T(0);
 #pragma unroll
-            for (int k = 0; k < N; ++k) a = fma(D[k * N + i], f1[k + j * N], a);
+                for (int k = 0; k < N; ++k) a = fma(D[k * N + i], f1[k + j * N], a);
 #pragma unroll
-            for (int k = 0; k < N; ++k) a = fma(D[k * N + j], f2[i + k * N], a);
-            lap[c] = a;
-            u[c] = su[c * st + t];
+                for (int k = 0; k < N; ++k) a = fma(D[k * N + j], f2[i + k * N], a);
+                lap[c] = a;
+            }
+            u[c] = su[q];
         }
         T o[NC];
         if (OP == OP_LAPLACE) {
@@ -751,6 +951,13 @@ __device__ __forceinline__ void grid_sum2(double v0, double v1, double* partials
     r0 = red[33];
     r1 = red[32];
     __syncthreads();
+}
+
+__device__ __forceinline__ void block_range(int E, int& eb, int& ee)
+{
+    const int G = gridDim.x;
+    eb = (int)((long long)blockIdx.x * E / G);
+    ee = (int)((long long)(blockIdx.x + 1) * E / G);
 }
 
 }  // namespace semgb

@@ -212,6 +212,9 @@ static int grid_1d(long long n) { return (int)std::min<long long>((n + 255) / 25
 // dynamic shared memory a persistent solver block may use for staging
 static const size_t kSolverSmemBudget = 160 * 1024;
 static const size_t kCgSmemBudget = 2 * 108 * 1024;
+static const size_t kK64SmemBudget = 224 * 1024;
+// all-reduce words of the FP64 solvers: two sets of at most 160 lines
+static const size_t kSlotWords = 2 * 160 * RESIDENT_SLOT_STRIDE;
 // the resident inner solve may use all of an SM's shared memory (227 KB per
 // block, less the kernel's static arrays)
 static const size_t kResidentSmemBudget = 227 * 1024 - 512;
@@ -341,6 +344,7 @@ struct sem_ctx {
     std::vector<double> Drow_host;         // D row-major (DevMesh::Dh)
     std::vector<double> S_host;            // preconditioner basis row-major (DevMesh::Sh)
     unsigned res_epoch = 0;                // last epoch on the resident solver's exchange words (0: clear them)
+    unsigned kr_epoch = 0;                 // the same for the FP64 solvers' reduction words
     std::vector<double> coords;            // [n_nodes][2]
     std::vector<int> elements;             // [E][4]
     std::vector<int> fl_host;              // DevMesh::flags, host copy
@@ -1400,6 +1404,7 @@ static int krylov_work(sem_ctx* c, int nc, KrylovWork<double>* w, GridSync** syn
     for (int k = 0; k < 2; ++k)
         if ((s = wsget(c, yn[k], v, &w->Y[k]))) return s;
     if ((s = wsget(c, "kr_part", 2 * 152 * 64, &w->partials))) return s;
+    if ((s = wsget(c, "kr_slots", kSlotWords, &w->slots))) return s;
     if ((s = wsget(c, "kr_sync", 1, sync))) return s;
     if ((s = wsget(c, "kr_out", 1, out))) return s;
     return SEM_OK;
@@ -1595,12 +1600,19 @@ static int run_krylov(sem_ctx* c, int op, const double* pot, double alpha, doubl
     if (s) return s;
     int grid = 0, kmax = 1;
     size_t smem = 0;
+    int resident = 1;
     dispatch_n(c->N, [&](auto nv) {
-        grid = solver_plan<decltype(nv)::value>(op, SOLVE_FP64, c->E, c->sms, kSolverSmemBudget, &kmax, &smem);
+        constexpr int NV = decltype(nv)::value;
+        grid = solver_plan<NV>(op, SOLVE_FP64_RES, c->E, c->sms, kK64SmemBudget, &kmax, &smem);
+        if (grid <= 0) {
+            resident = 0;
+            grid = solver_plan<NV>(op, SOLVE_FP64, c->E, c->sms, kK64SmemBudget, &kmax, &smem);
+        }
         return cudaSuccess;
     });
     if (grid <= 0) return fail(SEM_ERR_CUDA, "could not size the cooperative grid");
     SolveArgs a{};
+    a.resident = resident;
     a.kmax = kmax;
     a.op = op;
     a.nc = nc;
@@ -1618,6 +1630,15 @@ static int run_krylov(sem_ctx* c, int op, const double* pot, double alpha, doubl
     a.out = out;
     SEM_CUDA(cudaMemsetAsync(sync, 0, sizeof(GridSync), c->stream));
     SEM_CUDA(cudaMemsetAsync(out, 0, sizeof(SolveOut), c->stream));
+    // the reduction words' epochs run on from solve to solve (three per
+    // iteration at most); cleared for the first, after a failed one and long
+    // before the counter wraps
+    w.epoch0 = c->kr_epoch;
+    c->kr_epoch = 0;
+    if (w.epoch0 == 0 || w.epoch0 > 0x40000000u || maxit > 0x10000000) {
+        w.epoch0 = 0;
+        SEM_CUDA(cudaMemsetAsync(w.slots, 0, kSlotWords * sizeof(unsigned long long), c->stream));
+    }
     if (c->profile) SEM_CUDA(cudaEventRecord(c->ev[0], c->stream));
     cudaError_t e = dispatch_n(c->N, [&](auto nv) {
         return launch_solver<decltype(nv)::value>(c->dm, a, &w, nullptr, grid, smem, c->stream);
@@ -1627,6 +1648,7 @@ static int run_krylov(sem_ctx* c, int op, const double* pot, double alpha, doubl
     c->stats.kernel_launches++;
     c->stats.solver_launches++;
     if ((s = finish_solve(c, out, sync, res))) return s;
+    c->kr_epoch = c->h_out->epoch;
     c->stats.solver_iterations_fp64 += res->n_iter;
     c->stats.fp64_applies += res->n_iter + 1 + (x_is_zero ? 0 : 1);
     return SEM_OK;

@@ -107,6 +107,8 @@ struct DevMesh {
     int corrected = 0;
 };
 
+constexpr int RESIDENT_SLOT_STRIDE = 16;  // words: one 128-byte line per block's all-reduce words
+
 // Grid barrier and error state of a persistent (cooperative) kernel.
 struct GridSync {
     unsigned int count;
@@ -124,7 +126,7 @@ struct SolveOut {
     int inner_iters; // mixed mode: total FP32 iterations
     int sweeps;      // mixed mode: refinement sweeps
     int fallback;    // resident kernel: the inner solver gave up, continue with MINRES
-    unsigned epoch;  // resident kernel: last epoch used on the exchange words
+    unsigned epoch;  // resident and FP64 kernels: last epoch used on the exchange words
     double r0;       // mixed mode: the norm the stopping test is relative to
 };
 
@@ -137,6 +139,8 @@ struct KrylovWork {
     T* AZ;          // single-barrier MINRES: assembled A z_i (continuous format)
     T* Y3;          // single-barrier MINRES: y_i before the r2 correction
     T* Z[2];        // element preconditioner: z = P^-1 r of the last two iterations
+    unsigned long long* slots;  // FP64 solvers: [2][grid][RESIDENT_SLOT_STRIDE] tagged words of the reductions
+    unsigned epoch0;            // last epoch used on them
 };
 
 struct SolveArgs {
@@ -150,6 +154,7 @@ struct SolveArgs {
     double tol;
     int x_is_zero;
     int kmax;         // elements staged per pass (solver_plan)
+    int resident;     // FP64 solvers: the vectors stay in shared memory (SOLVE_FP64_RES)
     int rel_to_b;     // mixed solver: stop on |r| < tol |b| + tol instead of tol |r_0| + tol
                       // (the same test when x_0 = 0; used with warm starts)
     long long timeout_ns;
@@ -256,7 +261,7 @@ cudaError_t launch_learn(const DevMesh& m, const LearnArgs& a, cudaStream_t st);
 // launch_solver runs MINRES (op OP_RES/OP_HELM), PCG (OP_LAPLACE) or, when
 // mx is given, the mixed-precision refinement.  work points to a
 // KrylovWork<double> (FP64 solvers) or KrylovWork<float> (mixed).
-enum SolveKind : int { SOLVE_FP64 = 0, SOLVE_MIXED = 1, SOLVE_MIXED_FDM = 2 };
+enum SolveKind : int { SOLVE_FP64 = 0, SOLVE_MIXED = 1, SOLVE_MIXED_FDM = 2, SOLVE_FP64_RES = 3 };
 template <int N>
 int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax, size_t* smem);
 template <int N>
@@ -269,7 +274,6 @@ cudaError_t launch_solver(const DevMesh& m, const SolveArgs& a, const void* work
 // slots: 2 * grid * RESIDENT_SLOT_STRIDE words; xa, xb: n pairs of words each
 // (the tagged ring exchange); epoch0: the last epoch used on them (0 for
 // cleared words), SolveOut::epoch the one this launch ended with.
-constexpr int RESIDENT_SLOT_STRIDE = 16;  // one 128-byte line per block's all-reduce words
 template <int N>
 bool resident_plan(int E, int sms, size_t smem_budget, int* grid, int* st, int* kmax64, size_t* smem);
 template <int N>

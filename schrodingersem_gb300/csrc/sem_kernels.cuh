@@ -6,12 +6,31 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <mutex>
+#include <set>
+#include <utility>
 
 #include "sem_apply_bulk.cuh"
 #include "sem_device.cuh"
 #include "sem_solvers.cuh"
 
 namespace semgb {
+
+// shared-memory opt-in of a kernel, a per-device attribute: set once per device
+// (the current one, which owns the launch's stream) and kernel, under a lock
+inline cudaError_t smem_opt_in(const void* kern, size_t bytes)
+{
+    static std::mutex mu;
+    static std::set<std::pair<int, const void*>> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count({dev, kern})) return cudaSuccess;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) done.insert({dev, kern});
+    return e;
+}
 
 // element-local operator, input gathered with unmask semantics when GATHER
 template <int N, typename T, int OP, bool GATHER>
@@ -36,6 +55,112 @@ __global__ void __launch_bounds__(geo_tpb(N))
             y0[flat] = o[0];
             if (op_nc<OP>() == 2) y1[flat] = o[op_nc<OP>() - 1];
         });
+}
+
+// The FP64 element operator on lines (laplace64), K elements per block.  Warps
+// of a block are spread over the SM's four FP64 pipes in turn, and a warp
+// instruction costs a pipe the same however many lanes are active, so a block
+// costs laplace64_cost instructions per pipe, and the grid that of the SM with
+// the most blocks.  K minimises it (host integer work, a microsecond at most on
+// large meshes): small meshes spread over every SM, large ones fill their
+// warps.  Measured with K fixed by warp filling alone: 201 us instead of the
+// node kernel's 150 at p = 12, 64 x 64 (5 warps per block, 4.5 blocks per SM).
+// Where the line kernels run.  Measured on a GB300 against the kernels with one
+// thread per node (k_apply, k_combo_f), which reach 0.9 of the FP64 pipe: at 3 M
+// nodes the lines take 0.77-0.91 of their time for two components at p >= 6 and
+// 0.86-0.97 for one, and 1.0-1.1 at p <= 5, where the parity split saves little;
+// below about 1e5 nodes (one component: 1e6) their longer chains and coarser
+// blocks lose it again (p = 3, 1.5e5 nodes: 26.8 against 24.8 us)
+template <int N>
+inline bool lines64(int nc, int E)
+{
+    const long long nodes = (long long)E * N * N;
+    if (nc == 2) return N >= 9 ? nodes >= 100000 : N >= 7 && nodes >= 400000;
+    return N >= 7 && nodes >= 1000000;
+}
+
+// blocks of 256 threads per SM the FP64 one-pass kernels are compiled for: left
+// alone the compiler gathers a whole line's loads in up to 255 registers, and
+// one block per SM has nothing to run while it waits for them
+__host__ __device__ constexpr int geo64_minb(int N) { return N <= 10 ? 3 : 2; }
+
+template <int N, int NC>
+struct Geo64 {
+    static constexpr size_t bytes(int k) { return sizeof(double) * ((size_t)N * N + 3ull * NC * k * line_es(N)); }
+    static constexpr int kmax()
+    {
+        int k = 1;
+        while (NC * (k + 1) * N <= 256 && bytes(k + 1) <= 100 * 1024) ++k;
+        return k;
+    }
+    static int pick(int E)
+    {
+        constexpr int sms = 152;
+        int best = 1;
+        long long cost = -1;
+        const int top = std::min(kmax(), (E + sms - 1) / sms);
+        for (int k = 1; k <= top; ++k) {
+            const int blocks = (E + k - 1) / k, lines = NC * k * N;
+            const int one = laplace64_nodes(N, NC, k, threads(k)) ? laplace64_cost(N, NC, k, true)
+                                                                  : laplace64_cost(N, NC, k, false);
+            const long long c = (long long)((blocks + sms - 1) / sms) * one;
+            if (cost < 0 || c < cost || (c == cost && lines <= 128)) {
+                best = k;
+                cost = c;
+            }
+        }
+        return best;
+    }
+    static int threads(int k)
+    {
+        const int lines = NC * k * N, values = NC * k * N * N;
+        const int t = std::max(lines, std::min(values, 256));
+        return (t + 31) / 32 * 32;
+    }
+    template <class F>
+    static cudaError_t opt_in(F kern)  // per device, once
+    {
+        if (bytes(kmax()) <= 48 * 1024) return cudaSuccess;
+        return smem_opt_in((const void*)kern, bytes(kmax()));
+    }
+};
+
+template <int N, int OP, bool GATHER>
+__global__ void __launch_bounds__(256, geo64_minb(N))
+    k_apply64(DevMesh m, const __grid_constant__ EoD<N, double> et, int K, const double* __restrict__ pot, double alpha,
+              const double* __restrict__ in0, const double* __restrict__ in1, double* __restrict__ y0,
+              double* __restrict__ y1)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double* sm = (double*)smraw;
+    load_dmat_raw<N, double>(sm, m);
+    const int e0 = blockIdx.x * K;
+    apply_range<N, double, OP>(
+        sm, K, &et, fac_of<double>(m), pot, alpha, e0, min(K, m.E - e0),
+        [&](int e, int i, int j, long long flat, double* u) {
+            long long src = flat;
+            if (GATHER) src = ni_gather_src(m, node_info<N>(m, e, i, j), e, flat);
+            u[0] = in0[src];
+            if (op_nc<OP>() == 2) u[op_nc<OP>() - 1] = in1[src];
+        },
+        [&](int, int, int, long long flat, const double* o) {
+            y0[flat] = o[0];
+            if (op_nc<OP>() == 2) y1[flat] = o[op_nc<OP>() - 1];
+        });
+}
+
+template <int N, int OP, bool GATHER>
+inline cudaError_t launch_apply64(const DevMesh& m, const double* pot, double alpha, const double* in0,
+                                  const double* in1, double* y0, double* y1, cudaStream_t st)
+{
+    constexpr int NC = op_nc<OP>();
+    using G = Geo64<N, NC>;
+    const cudaError_t e = G::opt_in(k_apply64<N, OP, GATHER>);
+    if (e != cudaSuccess) return e;
+    const int K = G::pick(m.E);
+    k_apply64<N, OP, GATHER><<<(m.E + K - 1) / K, G::threads(K), G::bytes(K), st>>>(
+        m, eo_d_table<N, double>(m.Dh), K, pot, alpha, in0, in1, y0, y1);
+    return cudaGetLastError();
 }
 
 template <int N, typename T, int MODE>
@@ -237,6 +362,35 @@ __global__ void __launch_bounds__(geo_tpb(N))
         });
 }
 
+// the same on lines
+template <int N>
+__global__ void __launch_bounds__(256, geo64_minb(N))
+    k_combo_f64(DevMesh m, const __grid_constant__ EoD<N, double> et, int K, const double* __restrict__ V,
+              const double* __restrict__ p, ZList zl, double* y)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double* sm = (double*)smraw;
+    load_dmat_raw<N, double>(sm, m);
+    const int nz = zl.nz;
+    const long long n = m.n;
+    const int e0 = blockIdx.x * K;
+    apply_range<N, double, OP_F>(
+        sm, K, &et, fac_of<double>(m), V, 0.0, e0, min(K, m.E - e0),
+        [&](int e, int i, int j, long long flat, double* u) {
+            const long long src = ni_gather_src(m, node_info<N>(m, e, i, j), e, flat);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                double v = p[q * n + src];
+                for (int l = 0; l < nz; ++l) v = v + zl.c[l] * zl.z[l][q * n + src];
+                u[q] = v;
+            }
+        },
+        [&](int, int, int, long long flat, const double* o) {
+            y[flat] = o[0];
+            y[n + flat] = o[1];
+        });
+}
+
 // p_out = unmask(p_in + (c0 z0 + c1 z1 + ...)), both planes
 template <int N>
 __global__ void k_update(DevMesh m, const double* __restrict__ p_in, ZList zl,
@@ -393,13 +547,23 @@ cudaError_t launch_apply(const DevMesh& m, int op, bool fp32, const void* pot, d
         k_apply<N, T, OPK, false><<<grid, tpb, 0, st>>>(m, (const T*)pot, (T)alpha,               \
                                                         (const T*)in0, (const T*)in1, (T*)y0,     \
                                                         (T*)y1);
+#define SEM_APPLY64_CASE(OPK)                                                                      \
+    if (!lines64<N>(op_nc<OPK>(), m.E)) {                                                          \
+        SEM_APPLY_CASE(double, OPK)                                                                \
+        break;                                                                                     \
+    }                                                                                              \
+    return gather ? launch_apply64<N, OPK, true>(m, (const double*)pot, alpha, (const double*)in0, \
+                                                 (const double*)in1, (double*)y0, (double*)y1, st) \
+                  : launch_apply64<N, OPK, false>(m, (const double*)pot, alpha, (const double*)in0, \
+                                                  (const double*)in1, (double*)y0, (double*)y1, st);
     if (!fp32) {
+        if (op != OP_MASS && !m.Dh) return cudaErrorInvalidValue;
         switch (op) {
-            case OP_LAPLACE: SEM_APPLY_CASE(double, OP_LAPLACE) break;
-            case OP_HELM: SEM_APPLY_CASE(double, OP_HELM) break;
+            case OP_LAPLACE: SEM_APPLY64_CASE(OP_LAPLACE)
+            case OP_HELM: SEM_APPLY64_CASE(OP_HELM)
             case OP_MASS: SEM_APPLY_CASE(double, OP_MASS) break;
-            case OP_RES: SEM_APPLY_CASE(double, OP_RES) break;
-            case OP_F: SEM_APPLY_CASE(double, OP_F) break;
+            case OP_RES: SEM_APPLY64_CASE(OP_RES)
+            case OP_F: SEM_APPLY64_CASE(OP_F)
             default: return cudaErrorInvalidValue;
         }
     } else {
@@ -410,6 +574,7 @@ cudaError_t launch_apply(const DevMesh& m, int op, bool fp32, const void* pot, d
         }
     }
 #undef SEM_APPLY_CASE
+#undef SEM_APPLY64_CASE
     return cudaGetLastError();
 }
 
@@ -539,8 +704,17 @@ template <int N>
 cudaError_t launch_combo_f(const DevMesh& m, const double* V, const double* p, const ZList& zl,
                            double* y, cudaStream_t st)
 {
-    const int grid = (m.E + geo_k(N) - 1) / geo_k(N);
-    k_combo_f<N><<<grid, geo_tpb(N), 0, st>>>(m, V, p, zl, y);
+    if (!lines64<N>(2, m.E)) {
+        k_combo_f<N><<<(m.E + geo_k(N) - 1) / geo_k(N), geo_tpb(N), 0, st>>>(m, V, p, zl, y);
+        return cudaGetLastError();
+    }
+    if (!m.Dh) return cudaErrorInvalidValue;
+    using G = Geo64<N, 2>;
+    const cudaError_t e = G::opt_in(k_combo_f64<N>);
+    if (e != cudaSuccess) return e;
+    const int K = G::pick(m.E);
+    k_combo_f64<N><<<(m.E + K - 1) / K, G::threads(K), G::bytes(K), st>>>(
+        m, eo_d_table<N, double>(m.Dh), K, V, p, zl, y);
     return cudaGetLastError();
 }
 

@@ -16,13 +16,28 @@
 #include <cstdint>
 #include <cstring>
 
-#include "sem_apply_bulk.cuh"  // packed FP32 pair helpers
 
 namespace semgb {
 
 // ------------------------------------------------ packed FP32 pair arithmetic
 // (each lane an IEEE FP32 operation)
 typedef unsigned long long f2_t;
+__device__ __forceinline__ unsigned long long f2pack(float a, float b)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2unpack(unsigned long long v, float& a, float& b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long f2fma(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
 __device__ __forceinline__ f2_t f2add(f2_t a, f2_t b)
 {
     f2_t d;

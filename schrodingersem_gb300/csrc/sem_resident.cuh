@@ -618,8 +618,8 @@ __host__ __device__ constexpr size_t res_stage_bytes(int st, int k64)
 }
 template <int N>
 __global__ void __launch_bounds__(RES_TPB, 1)
-    k_resident(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ CgTab<N> tab,
-               ResArgs ra)
+    k_resident(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ EoD<N, double> et,
+               const __grid_constant__ CgTab<N> tab, ResArgs ra)
 {
     constexpr int NN = N * N;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(RES_TPB, 1)
             __syncthreads();
             for (int e0 = eb; e0 < ee; e0 += kmax)
                 apply_range<N, double, OP_RES>(
-                    sm64, kmax, fac64, pot64, a.alpha, e0, min(kmax, ee - e0),
+                    sm64, kmax, &et, fac64, pot64, a.alpha, e0, min(kmax, ee - e0),
                     [&](int e, int i, int j, long long flat, double* u) {
                         const long long src = ni_gather_src(m, node_info<N>(m, e, i, j), e, flat);
                         u[0] = xp[0][src];
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(RES_TPB, 1)
         double itol = mx.inner_tol;
         if (mx.adaptive) {
             const double need = mx.outer_scale * (a.tol * sweep_state[0] + a.tol) / sweep_state[1];
-            itol = fmax(itol, fmin(0.3 * need, 0.5));
+            itol = fmax(itol, fmin(CG_MARGIN * need, 0.5));
         }
         const double rn = sweep_state[1];
         if (sweep > 0 && !(rn < 0.5 * last_rn)) {
@@ -788,9 +788,10 @@ cudaError_t launch_resident(const DevMesh& m, const SolveArgs& a, const KrylovWo
     SolveArgs aa = a;
     KrylovWork<float> ww = w;
     MixedArgs xx = mx;
+    EoD<N, double> et = eo_d_table<N, double>(m.Dh);
     CgTab<N> tab = cg_table<N>(m);
     ResArgs ra{st, (ulonglong2*)xa, (ulonglong2*)xb, slots, epoch0};
-    void* args[] = {&mm, &aa, &ww, &xx, &tab, &ra};
+    void* args[] = {&mm, &aa, &ww, &xx, &et, &tab, &ra};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(RES_TPB), args, smem, stream);
 }
 

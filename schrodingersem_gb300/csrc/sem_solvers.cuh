@@ -16,6 +16,7 @@
 
 #include "sem_cg.cuh"
 #include "sem_device.cuh"
+#include "sem_krylov64.cuh"
 
 namespace semgb {
 
@@ -330,7 +331,7 @@ __device__ __forceinline__ bool minres_core(T* sm, int kmax, double* red, Minres
         if (!grid_barrier(gs, tmo)) return false;
         for (int e0 = eb; e0 < ee; e0 += kmax)
             apply_range<N, T, OP>(
-                sm, kmax, fac, pot, alpha, e0, min(kmax, ee - e0),
+                sm, kmax, nullptr, fac, pot, alpha, e0, min(kmax, ee - e0),
                 [&](int e, int i, int j, long long flat, T* u) {
                     const NodeInfo ni = node_info<N>(m, e, i, j);
                     const bool own = ni_owner(ni);
@@ -346,7 +347,7 @@ __device__ __forceinline__ bool minres_core(T* sm, int kmax, double* red, Minres
     } else {
         for (int e0 = eb; e0 < ee; e0 += kmax)
             apply_range<N, T, OP>(
-                sm, kmax, fac, pot, alpha, e0, min(kmax, ee - e0),
+                sm, kmax, nullptr, fac, pot, alpha, e0, min(kmax, ee - e0),
                 [&](int e, int i, int j, long long flat, T* u) {
                     const NodeInfo ni = node_info<N>(m, e, i, j);
                     const bool own = ni_owner(ni);
@@ -441,7 +442,7 @@ __device__ __forceinline__ bool minres_core(T* sm, int kmax, double* red, Minres
                 T* Zn = w.Z[it & 1];
                 for (int e0 = eb; e0 < ee; e0 += kmax)
                     apply_range_post<N, T, OP, true>(
-                        sm, kmax, fac, pot, alpha, e0, min(kmax, ee - e0),
+                        sm, kmax, nullptr, fac, pot, alpha, e0, min(kmax, ee - e0),
                         [&](int e, int i, int j, long long flat, T* u, T* aux) {
                             const NodeInfo ni = node_info<N>(m, e, i, j);
 #pragma unroll
@@ -464,7 +465,7 @@ __device__ __forceinline__ bool minres_core(T* sm, int kmax, double* red, Minres
             } else {
                 for (int e0 = eb; e0 < ee; e0 += kmax)
                     apply_range_post<N, T, OP, true>(
-                        sm, kmax, fac, pot, alpha, e0, min(kmax, ee - e0),
+                        sm, kmax, nullptr, fac, pot, alpha, e0, min(kmax, ee - e0),
                         [&](int, int, int, long long flat, T* u, T* aux) {
                             const T pv = PRE == 1 ? pinv[flat] : T(1);
 #pragma unroll
@@ -496,14 +497,8 @@ __device__ __forceinline__ bool minres_core(T* sm, int kmax, double* red, Minres
                 iy = tmp;
             }
             if (threadIdx.x == 0) {
-                if constexpr (sizeof(T) == 4) {
-                    scal_step_rsqrt(sc, sc.alpha_i, bnew2, eps_mach, tol_rel, tol_abs);
-                    sc.stop = sc.conv || it == maxit;
-                } else {
-                    scal_givens(sc, sc.alpha_i, sqrt(bnew2), eps_mach, tol_rel, tol_abs);
-                    sc.stop = sc.conv || it == maxit;
-                    scal_publish(sc, it + 1, 0.0);
-                }
+                scal_step_rsqrt(sc, sc.alpha_i, bnew2, eps_mach, tol_rel, tol_abs);
+                sc.stop = sc.conv || it == maxit;
             }
             __syncthreads();
             if (sc.stop) break;
@@ -577,7 +572,7 @@ __device__ __forceinline__ bool minres_core_fused(T* sm, int kmax, double* red, 
     T part = T(0), partz = T(0);
     for (int e0 = eb; e0 < ee; e0 += kmax)
         apply_range<N, T, OP>(
-            sm, kmax, fac, pot, alpha, e0, min(kmax, ee - e0),
+            sm, kmax, nullptr, fac, pot, alpha, e0, min(kmax, ee - e0),
             [&](int e, int i, int j, long long flat, T* u) {
                 const NodeInfo ni = node_info<N>(m, e, i, j);
                 const bool own = ni_owner(ni);
@@ -618,7 +613,7 @@ __device__ __forceinline__ bool minres_core_fused(T* sm, int kmax, double* red, 
             T s1 = T(0), s2 = T(0);
             for (int e0 = eb; e0 < ee; e0 += kmax)
                 apply_range<N, T, OP>(
-                    sm, kmax, fac, pot, alpha, e0, min(kmax, ee - e0),
+                    sm, kmax, nullptr, fac, pot, alpha, e0, min(kmax, ee - e0),
                     [&](int e, int i, int j, long long flat, T* u) {
                         const NodeInfo ni = node_info<N>(m, e, i, j);
                         const bool own = ni_owner(ni);
@@ -709,72 +704,6 @@ __device__ __forceinline__ bool minres_core_fused(T* sm, int kmax, double* red, 
     return true;
 }
 
-__device__ __forceinline__ void block_range(int E, int& eb, int& ee)
-{
-    const int G = gridDim.x;
-    eb = (int)((long long)blockIdx.x * E / G);
-    ee = (int)((long long)(blockIdx.x + 1) * E / G);
-}
-
-// ---------------------------------------------------------- plain MINRES
-template <int N, typename T, int OP>
-__global__ void __launch_bounds__(SOLVER_TPB, 1)
-    k_minres(DevMesh m, SolveArgs a, KrylovWork<T> w)
-{
-    constexpr int NC = op_nc<OP>();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ double red[34];
-    __shared__ MinresScal<T> sc;
-    T* sm = (T*)smraw;
-    load_dmat_raw<N, T>(sm, m);
-    __syncthreads();
-    const Fac<T> fac = fac_of<T>(m);
-    const long long n = m.n;
-    const T* pot = (const T*)a.pot;
-    const T alpha = (T)a.alpha;
-    const T* bp[2] = {(const T*)a.b[0], (const T*)a.b[1]};
-    T* xp[2] = {(T*)a.x[0], (T*)a.x[1]};
-    int eb, ee;
-    block_range(m.E, eb, ee);
-    const int kmax = a.kmax;
-    int slot = 0;
-    // P0: Y[1] = A_local(unmask(x0))
-    if (!a.x_is_zero) {
-        T* Y1 = w.Y[1];
-        for (int e0 = eb; e0 < ee; e0 += kmax)
-            apply_range<N, T, OP>(
-                sm, kmax, fac, pot, alpha, e0, min(kmax, ee - e0),
-                [&](int e, int i, int j, long long flat, T* u) {
-                    const long long src = ni_gather_src(m, node_info<N>(m, e, i, j), e, flat);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) u[c] = xp[c][src];
-                },
-                [&](int, int, int, long long flat, const T* o) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) Y1[c * n + flat] = o[c];
-                });
-        if (!grid_barrier(a.sync, a.timeout_ns)) return;
-    }
-    // r0 = unmask(b) - DSS(A_local(unmask(x0)))
-    const bool xz = a.x_is_zero != 0;
-    const T* Y1 = w.Y[1];
-    auto rhs = [&](const NodeInfo& ni, int e, long long flat, int c) -> T {
-        T r = bp[c][ni_gather_src(m, ni, e, flat)];
-        if (!xz) r = r - dss_value<N, T, DSS_CONT>(m, Y1 + c * n, ni, e, flat);
-        return r;
-    };
-    MinresOut r{};
-    if (!minres_core<N, T, OP, 0>(sm, kmax, red, sc, m, pot, alpha, eb, ee, w, a.sync, a.timeout_ns, slot,
-                                      rhs, xp, a.maxit, a.tol, a.tol, r, (const T*)nullptr))
-        return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.out->success = r.conv ? 1 : 0;
-        a.out->n_iter = r.conv ? r.it : (a.maxit >= 1 ? a.maxit + 1 : 1);
-        a.out->residual = r.phibar;
-        a.out->status = 0;
-    }
-}
-
 // ------------------------------------------- mixed-precision refinement
 // FP64 iterative refinement around an FP32 inner MINRES.  Each sweep:
 // r = b - A x in FP64 (true residual, continuous format); stop when
@@ -804,7 +733,7 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
                                             const MixedArgs& mx, int eb, int ee, bool leader,
                                             unsigned char* smraw, double* red, MinresScal<float>& sc,
                                             double* sweep_state, float* fdmS, float* fdmL,
-                                            const CgTab<N>* tab = nullptr)
+                                            const EoD<N, double>& et, const CgTab<N>* tab = nullptr)
 {
     static_assert(KIND == MIXED_PLAIN || OP == OP_RES, "the element preconditioner is the stage operator's");
     constexpr int NN = N * N;
@@ -827,11 +756,12 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
         // ---- FP64 residual r = unmask(b) - DSS(A_local(unmask(x)))
         const bool applied = (sweep > 0) || !a.x_is_zero;
         if (applied) {
+            __syncthreads();  // the staging area overlays the inner solve's
             load_dmat_raw<N, double>(sm64, m);
             __syncthreads();
             for (int e0 = eb; e0 < ee; e0 += kmax)
                 apply_range<N, double, OP>(
-                    sm64, kmax, fac64, pot64, a.alpha, e0, min(kmax, ee - e0),
+                    sm64, kmax, &et, fac64, pot64, a.alpha, e0, min(kmax, ee - e0),
                     [&](int e, int i, int j, long long flat, double* u) {
                         const long long src = ni_gather_src(m, node_info<N>(m, e, i, j), e, flat);
 #pragma unroll
@@ -891,7 +821,7 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
         double itol = mx.inner_tol;
         if (mx.adaptive) {
             const double need = mx.outer_scale * (a.tol * sweep_state[0] + a.tol) / sweep_state[1];
-            itol = fmax(itol, fmin(0.3 * need, 0.5));
+            itol = fmax(itol, fmin((cg ? CG_MARGIN : 0.3) * need, 0.5));
         }
         if constexpr (KIND != MIXED_PLAIN) {
             const double rn = sweep_state[1];
@@ -984,7 +914,8 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
 
 template <int N, int OP>
 __global__ void __launch_bounds__(SOLVER_TPB, 1)
-    k_minres_mixed(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx)
+    k_minres_mixed(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx,
+                   const __grid_constant__ EoD<N, double> et)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[34];
@@ -993,14 +924,15 @@ __global__ void __launch_bounds__(SOLVER_TPB, 1)
     int eb, ee;
     block_range(m.E, eb, ee);
     mixed_solve<N, OP, MIXED_PLAIN>(m, a, w, mx, eb, ee, blockIdx.x == 0, smraw, red, sc, sweep_state, nullptr,
-                                    nullptr);
+                                    nullptr, et);
 }
 
 // the same with the element preconditioner
 constexpr int CG_TPB = 256;
 template <int N>
 __global__ void __launch_bounds__(CG_TPB, 2)
-    k_cg_mixed(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ CgTab<N> tab)
+    k_cg_mixed(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ EoD<N, double> et,
+               const __grid_constant__ CgTab<N> tab)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[34];
@@ -1010,141 +942,7 @@ __global__ void __launch_bounds__(CG_TPB, 2)
     int eb, ee;
     block_range(m.E, eb, ee);
     mixed_solve<N, OP_RES, MIXED_FDM>(m, a, w, mx, eb, ee, blockIdx.x == 0, smraw, red, sc, sweep_state, fdmS, fdmL,
-                                      &tab);
-}
-
-// --------------------------------------------------------- persistent PCG
-// include/pcg.hpp:59-97 with the identity preconditioner.  Vectors r, p in
-// the continuous format; three grid barriers per iteration.
-template <int N, typename T>
-__global__ void __launch_bounds__(SOLVER_TPB, 1)
-    k_pcg(DevMesh m, SolveArgs a, KrylovWork<T> w)
-{
-    constexpr int NN = N * N;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ double red[34];
-    __shared__ double ps[4];  // rho, rho_prev, bnorm, stop flag
-    __shared__ T pc[2];       // beta, alpha of the current iteration
-    T* sm = (T*)smraw;
-    load_dmat_raw<N, T>(sm, m);
-    __syncthreads();
-    const Fac<T> fac = fac_of<T>(m);
-    const T* b = (const T*)a.b[0];
-    T* x = (T*)a.x[0];
-    T* R = w.L[0];
-    T* Pv = w.L[1];
-    int eb, ee;
-    block_range(m.E, eb, ee);
-    const long long nb = (long long)eb * NN, ne = (long long)ee * NN;
-    const int kmax = a.kmax;
-    int slot = 0;
-    bool ok = true;
-    auto store_y = [&](T* Yb) {
-        return [=](int, int, int, long long flat, const T* o) { Yb[flat] = o[0]; };
-    };
-    if (!a.x_is_zero) {
-        for (int e0 = eb; e0 < ee; e0 += kmax)
-            apply_range<N, T, OP_LAPLACE>(
-                sm, kmax, fac, (const T*)nullptr, T(0), e0, min(kmax, ee - e0),
-                [&](int e, int i, int j, long long flat, T* u) {
-                    u[0] = x[ni_gather_src(m, node_info<N>(m, e, i, j), e, flat)];
-                },
-                store_y(w.Y[1]));
-        if (!grid_barrier(a.sync, a.timeout_ns)) return;
-    }
-    T pb = T(0), pr = T(0);
-    for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
-        const int e = (int)(idx / NN);
-        const int node = (int)(idx - (long long)e * NN);
-        const NodeInfo ni = node_info<N>(m, e, node % N, node / N);
-        const T bv = b[ni_gather_src(m, ni, e, idx)];
-        T r = bv;
-        if (!a.x_is_zero) r = bv - dss_value<N, T, DSS_CONT>(m, w.Y[1], ni, e, idx);
-        R[idx] = r;
-        if (ni_owner(ni)) {
-            pb = fma(bv, bv, pb);
-            pr = fma(r, r, pr);
-        }
-    }
-    double bb = 0.0, rho0 = 0.0;
-    grid_sum2_t<T>(pb, pr, w.partials, slot, a.sync, a.timeout_ns, red, ok, bb, rho0);
-    slot ^= 1;
-    if (!ok) return;
-    if (threadIdx.x == 0) {
-        ps[0] = rho0;
-        ps[1] = 0.0;
-        ps[2] = sqrt(bb);
-        ps[3] = 0.0;
-        pc[0] = T(0);
-    }
-    __syncthreads();
-    bool conv = false;
-    int it = 0;
-    double dummy = 0.0;
-    for (it = 0; it < a.maxit; ++it) {
-        const T beta = pc[0];
-        for (int e0 = eb; e0 < ee; e0 += kmax)
-            apply_range<N, T, OP_LAPLACE>(
-                sm, kmax, fac, (const T*)nullptr, T(0), e0, min(kmax, ee - e0),
-                [&](int, int, int, long long flat, T* u) {
-                    const T pv = (it == 0) ? R[flat] : R[flat] + beta * Pv[flat];
-                    Pv[flat] = pv;
-                    u[0] = pv;
-                },
-                store_y(w.Y[0]));
-        // the assembly below reads other blocks' element outputs
-        if (!grid_barrier(a.sync, a.timeout_ns)) return;
-        T pap = T(0);
-#pragma unroll 4
-        for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
-            const int e = (int)(idx / NN);
-            const int node = (int)(idx - (long long)e * NN);
-            const NodeInfo ni = node_info<N>(m, e, node % N, node / N);
-            if (ni_owner(ni)) pap = fma(Pv[idx], dss_value<N, T, DSS_CONT>(m, w.Y[0], ni, e, idx), pap);
-        }
-        double pAp = 0.0;
-        grid_sum2_t<T>(pap, T(0), w.partials, slot, a.sync, a.timeout_ns, red, ok, pAp, dummy);
-        slot ^= 1;
-        if (!ok) return;
-        if (threadIdx.x == 0) pc[1] = (T)(ps[0] / pAp);
-        __syncthreads();
-        const T al = pc[1];
-        T prr = T(0);
-#pragma unroll 4
-        for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
-            const int e = (int)(idx / NN);
-            const int node = (int)(idx - (long long)e * NN);
-            const NodeInfo ni = node_info<N>(m, e, node % N, node / N);
-            const bool own = ni_owner(ni);
-            const T ap = dss_value<N, T, DSS_CONT>(m, w.Y[0], ni, e, idx);
-            if (own) x[idx] += al * Pv[idx];
-            const T r = R[idx] - al * ap;
-            R[idx] = r;
-            if (own) prr = fma(r, r, prr);
-        }
-        if (threadIdx.x == 0) {
-            ps[1] = ps[0];  // rho_prev = rho
-            ps[3] = sqrt(ps[0]) < a.tol * ps[2] ? 1.0 : 0.0;  // pcg.hpp:84, rho of this iteration's start
-        }
-        __syncthreads();
-        conv = ps[3] != 0.0;
-        if (conv) break;
-        double rho = 0.0;
-        grid_sum2_t<T>(prr, T(0), w.partials, slot, a.sync, a.timeout_ns, red, ok, rho, dummy);
-        slot ^= 1;
-        if (!ok) return;
-        if (threadIdx.x == 0) {
-            pc[0] = (T)(rho / ps[1]);
-            ps[0] = rho;
-        }
-        __syncthreads();
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.out->success = conv ? 1 : 0;
-        a.out->n_iter = it;
-        a.out->residual = sqrt(ps[1]);  // rho of the last iteration's start (pcg.hpp:93)
-        a.out->status = 0;
-    }
+                                      et, &tab);
 }
 
 // ------------------------------------------------------------- launchers
@@ -1153,6 +951,12 @@ __global__ void __launch_bounds__(SOLVER_TPB, 1)
 template <int N>
 size_t solver_smem(int op, int kind, int kmax)
 {
+    if (kind == SOLVE_FP64 || kind == SOLVE_FP64_RES) {
+        const bool r = kind == SOLVE_FP64_RES;
+        return op == OP_RES    ? k64_smem_bytes<N, OP_RES>(kmax, r)
+               : op == OP_HELM ? k64_smem_bytes<N, OP_HELM>(kmax, r)
+                               : k64_smem_bytes<N, OP_LAPLACE>(kmax, r);
+    }
     const bool two = (op == OP_RES);
     const size_t d = two ? range_smem_bytes<N, double, OP_RES>(kmax) : range_smem_bytes<N, double, OP_HELM>(kmax);
     const size_t c = kind == SOLVE_MIXED_FDM ? cg_smem_bytes<N>(kmax) : 0;
@@ -1165,36 +969,54 @@ static const void* solver_fn(int op, int kind)
     if (kind == SOLVE_MIXED_FDM) return (const void*)k_cg_mixed<N>;
     if (kind == SOLVE_MIXED)
         return op == OP_RES ? (const void*)k_minres_mixed<N, OP_RES> : (const void*)k_minres_mixed<N, OP_HELM>;
+    if (kind == SOLVE_FP64_RES)
+        return op == OP_RES    ? (const void*)k_minres64r<N, OP_RES>
+               : op == OP_HELM ? (const void*)k_minres64r<N, OP_HELM>
+                               : (const void*)k_pcg64r<N>;
     switch (op) {
-        case OP_RES: return (const void*)k_minres<N, double, OP_RES>;
-        case OP_HELM: return (const void*)k_minres<N, double, OP_HELM>;
-        default: return (const void*)k_pcg<N, double>;
+        case OP_RES: return (const void*)k_minres64<N, OP_RES>;
+        case OP_HELM: return (const void*)k_minres64<N, OP_HELM>;
+        default: return (const void*)k_pcg64<N>;
     }
+}
+
+// threads of the FP64 solvers: one per value of a small share (the smaller the
+// block, the cheaper its barriers), at most K64_TPB
+inline int k64_threads(int N, int nc, int share)
+{
+    const int v = nc * share * N * N, top = k64_tpb(N);
+    return v >= top ? top : v < 128 ? 128 : (v + 31) / 32 * 32;
 }
 
 // Plan a cooperative launch: one block per SM (fewer for small meshes), two
 // smaller ones for the element-preconditioned kernel on meshes that give each
 // SM several passes, so that one block's loads overlap the other's passes,
 // and the largest staging capacity kmax <= the block's element count that
-// fits in smem_budget bytes per SM.  Returns the grid, or 0 on failure.
+// fits in smem_budget bytes per SM.  Returns the grid, or 0 on failure (for
+// SOLVE_FP64_RES also when the block's elements do not fit in one pass).
 template <int N>
 int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_out, size_t* smem_out)
 {
     const bool fdm = kind == SOLVE_MIXED_FDM;
     int per = 1;
     if (fdm && (long long)E * N * N >= 4096ll * sms) per = 2;
+    const bool f64 = kind == SOLVE_FP64 || kind == SOLVE_FP64_RES;
+    if (f64 && sms > 32 * K64_MAXQ) sms = 32 * K64_MAXQ;
     int grid = E < per * sms ? E : per * sms;
     if (grid < 1) grid = 1;
     int kmax = (E + grid - 1) / grid;
     const int share = kmax;
+    if (kind == SOLVE_FP64_RES && solver_smem<N>(op, kind, kmax) > smem_budget) return 0;  // does not fit
     while (kmax > 1 && solver_smem<N>(op, kind, kmax) > smem_budget / per)
-        kmax = fdm ? kmax - 1 : (kmax + 1) / 2;
-    if (fdm) kmax = (share + (share + kmax - 1) / kmax - 1) / ((share + kmax - 1) / kmax);  // even passes
+        kmax = kind != SOLVE_MIXED ? kmax - 1 : (kmax + 1) / 2;
+    if (kind != SOLVE_MIXED)  // even passes
+        kmax = (share + (share + kmax - 1) / kmax - 1) / ((share + kmax - 1) / kmax);
     const size_t smem = solver_smem<N>(op, kind, kmax);
     const void* fn = solver_fn<N>(op, kind);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : SOLVER_TPB, smem) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : f64 ? k64_tpb(N) : SOLVER_TPB,
+                                                      smem) != cudaSuccess ||
         per_sm < 1)
         return 0;
     if (grid > per_sm * sms) grid = per_sm * sms;
@@ -1209,23 +1031,25 @@ cudaError_t launch_solver(const DevMesh& m, const SolveArgs& a, const void* work
 {
     DevMesh mm = m;
     SolveArgs aa = a;
-    const int kind = !mx ? SOLVE_FP64 : mx->fdm ? SOLVE_MIXED_FDM : SOLVE_MIXED;
+    const int kind = !mx ? (a.resident ? SOLVE_FP64_RES : SOLVE_FP64) : mx->fdm ? SOLVE_MIXED_FDM : SOLVE_MIXED;
     const void* fn = solver_fn<N>(a.op, kind);
-    if (kind != SOLVE_FP64) {
+    if (!m.Dh || !m.Sh) return cudaErrorInvalidValue;
+    EoD<N, double> et = eo_d_table<N, double>(m.Dh);
+    if (mx) {
         KrylovWork<float> ww = *(const KrylovWork<float>*)work;
         MixedArgs xx = *mx;
         if (kind == SOLVE_MIXED_FDM) {
-            if (!m.Dh || !m.Sh) return cudaErrorInvalidValue;
             CgTab<N> tab = cg_table<N>(m);
-            void* args[] = {&mm, &aa, &ww, &xx, &tab};
+            void* args[] = {&mm, &aa, &ww, &xx, &et, &tab};
             return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(CG_TPB), args, smem, st);
         }
-        void* args[] = {&mm, &aa, &ww, &xx};
+        void* args[] = {&mm, &aa, &ww, &xx, &et};
         return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(SOLVER_TPB), args, smem, st);
     }
     KrylovWork<double> ww = *(const KrylovWork<double>*)work;
-    void* args[] = {&mm, &aa, &ww};
-    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(SOLVER_TPB), args, smem, st);
+    void* args[] = {&mm, &aa, &ww, &et, &ww.slots, &ww.epoch0};
+    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(k64_threads(N, a.nc, (m.E + grid - 1) / grid)), args,
+                                       smem, st);
 }
 
 }  // namespace semgb
