@@ -411,11 +411,11 @@ int sem_ctx_dataset(sem_ctx* ctx, void** X, float** T, long long* rows, int* d_i
  * state -- advanced together by schro_omp::schrodinger_bdf2
  * (include/openmp_impl/schrodinger.hpp:22-128) with the mixed-precision
  * stage solve (FP32 inner MINRES, FP64 refinement on the true residual;
- * SEM_PRECOND_FDM by default).  One persistent launch per time step serves
- * all instances (a block per instance, largest first, block-local barriers
- * and reductions); the step is captured once as a CUDA graph and replayed.
- * The elements each block stages per pass are chosen per degree by a timing
- * sweep at creation (sem_batch_stats.kmax_of_p). */
+ * SEM_PRECOND_FDM by default).  One persistent launch per time step and size class serves
+ * all instances (a cluster of 1 to 8 blocks per instance by its size, largest
+ * first, cluster barriers and reductions); the step is captured once as a CUDA
+ * graph and replayed.  A block stages as many elements per pass as give each of
+ * its threads a line (sem_batch_stats.kmax_of_p: the largest of the degree). */
 typedef struct sem_batch sem_batch;
 typedef struct {
     long long steps;              /* time steps run (all instances together) */

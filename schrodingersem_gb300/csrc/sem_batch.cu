@@ -6,18 +6,7 @@
 // MINRES (FP32 inner iterations, FP64 refinement judged on the true
 // residual).
 //
-// Execution: one persistent launch per time step for all instances.  Blocks
-// take instances from a device work queue (largest first); a block advances
-// its instance by one step on its own -- projection, right-hand side, the
-// complete refined MINRES solve with block barriers and block reductions,
-// unmask -- so instances never wait for one another and each records its
-// own convergence flag and iteration count.  The step (queue reset + kernel)
-// is captured once as a CUDA graph and replayed; every per-step quantity
-// (history slot, BDF coefficient) is derived on the device from the
-// instance's own step counter, so the same graph serves every step.  The
-// staging capacity (elements per pass of the element kernels, which sets
-// the threads working on one element) is chosen per degree by a timing
-// sweep at setup.
+// Execution: see sem_batch.cuh.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -52,13 +41,15 @@ cudaError_t dispatch_batch_n(int N, F&& f)
 }
 }  // namespace
 
-// instances of one degree: their order (largest first), queue and launch shape
+// instances of one degree and cluster size: their order (largest first), queue
+// and launch shape
 struct BatchGroup {
     int N = 0;
+    int cluster = 1;  // blocks per instance with the element preconditioner
     std::vector<int> members;
     int* d_order = nullptr;
     int* d_queue = nullptr;
-    int grid = 0;
+    int grid = 0, grid_plain = 0;  // clusters (blocks without the preconditioner)
     size_t smem = 0;
     cudaStream_t fork = nullptr;
     cudaEvent_t done = nullptr;
@@ -117,59 +108,6 @@ extern "C" int sem_batch_destroy(sem_batch* b)
     return SEM_OK;
 }
 
-// Staging capacity per degree: time block-local FP32 Res applies over the
-// group's largest instances for kmax = 1, 2, 4, ... (as far as the element
-// count and the shared-memory budget allow) and keep the fastest.
-static int tune_group(sem_batch* b, BatchGroup& g, int* kmax_out)
-{
-    const int N = g.N;
-    std::vector<int> list(g.members.begin(), g.members.begin() + std::min<size_t>(g.members.size(), 64));
-    long long emax = 0;
-    for (int i : list) emax = std::max<long long>(emax, b->nloc[i] / (N * N));
-    int* dl = nullptr;
-    float* sink = nullptr;
-    int s = 0;
-    if ((s = balloc(b, (void**)&dl, sizeof(int) * list.size())) || (s = balloc(b, (void**)&sink, sizeof(float))))
-        return s;
-    BCUDA(cudaMemcpy(dl, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice));
-    cudaEvent_t e0, e1;
-    BCUDA(cudaEventCreate(&e0));
-    BCUDA(cudaEventCreate(&e1));
-    float best = 1e30f;
-    int best_k = 1;
-    const int grid = std::min<int>((int)list.size(), b->sms);
-    for (int kmax = 1; kmax <= 256; kmax *= 2) {
-        if (kmax > 1 && kmax / 2 >= emax) break;
-        size_t sm = 0;
-        dispatch_batch_n(N, [&](auto nv) {
-            sm = batch_smem_n<decltype(nv)::value>(kmax);
-            return cudaSuccess;
-        });
-        if (sm > BATCH_SMEM_BUDGET) break;
-        auto launch = [&]() {
-            return dispatch_batch_n(N, [&](auto nv) {
-                return batch_launch_probe<decltype(nv)::value>(b->d_inst, dl, (int)list.size(), kmax, 8, sink, grid,
-                                                               b->stream);
-            });
-        };
-        BCUDA(launch());  // warm-up
-        BCUDA(cudaEventRecord(e0, b->stream));
-        BCUDA(launch());
-        BCUDA(cudaEventRecord(e1, b->stream));
-        BCUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        BCUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best) {
-            best = ms;
-            best_k = kmax;
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    *kmax_out = best_k;
-    return SEM_OK;
-}
-
 extern "C" int sem_batch_create(sem_batch** out, int n_inst, const int* p, const int* n_nodes,
                                 const double* const* coords, const int* n_elements, const int* const* elements,
                                 unsigned flags)
@@ -203,9 +141,15 @@ extern "C" int sem_batch_create(sem_batch** out, int n_inst, const int* p, const
     float* pool32 = nullptr;
     double* vpool = nullptr;
     SolveOut* outs = nullptr;
-    const long long per64 = 12, per32 = 25;  // values per local node
+    // values per local node; FP32 vectors are read as pairs: an even count each
+    const long long per64 = 12, per32 = 24;
+    long long pot_tot = 0;
+    for (long long v : b->nloc) pot_tot += v + (v & 1);
+    float4* fpool = nullptr;
+    float* wpool = nullptr;
     if ((s = balloc(b, (void**)&pool64, sizeof(double) * per64 * tot)) ||
-        (s = balloc(b, (void**)&pool32, sizeof(float) * per32 * tot)) ||
+        (s = balloc(b, (void**)&pool32, sizeof(float) * (per32 * tot + pot_tot))) ||
+        (s = balloc(b, (void**)&fpool, sizeof(float4) * tot)) || (s = balloc(b, (void**)&wpool, sizeof(float) * tot)) ||
         (s = balloc(b, (void**)&vpool, sizeof(double) * tot)) ||
         (s = balloc(b, (void**)&b->d_step, sizeof(int) * n)) ||
         (s = balloc(b, (void**)&b->d_status, sizeof(int) * n)) ||
@@ -215,7 +159,7 @@ extern "C" int sem_batch_create(sem_batch** out, int n_inst, const int* p, const
         sem_batch_destroy(b);
         return s;
     }
-    if (cudaMemset(pool32, 0, sizeof(float) * per32 * tot) != cudaSuccess ||
+    if (cudaMemset(pool32, 0, sizeof(float) * (per32 * tot + pot_tot)) != cudaSuccess ||
         cudaMemset(pool64, 0, sizeof(double) * per64 * tot) != cudaSuccess) {
         sem_batch_destroy(b);
         return bfail(SEM_ERR_CUDA, "cudaMemset of the batch pools");
@@ -249,49 +193,65 @@ extern "C" int sem_batch_create(sem_batch** out, int n_inst, const int* p, const
         for (int q = 0; q < 2; ++q) I.w.Z[q] = t32(2 * v);
         I.w.Y3 = t32(2 * v);
         I.x32 = t32(2 * v);
-        I.pot32 = t32(v);
+        I.pot32 = t32(v + (v & 1));
         I.V = vpool + ov;
+        I.fac4 = fpool + ov;
+        I.nnw = wpool + ov;
+        const cudaError_t pe = dispatch_batch_n(b->N[i], [&](auto nv) {
+            return batch_prep_instance<decltype(nv)::value>(I.m, fpool + ov, wpool + ov, nullptr);
+        });
+        if (pe != cudaSuccess) {
+            sem_batch_destroy(b);
+            return bfail(SEM_ERR_CUDA, cudaGetErrorString(pe));
+        }
         ov += v;
         I.out = outs + i;
         I.step = b->d_step + i;
         I.status = b->d_status + i;
         I.iters = b->d_iters + i;
-        I.kmax = 1;
+        I.kmax = I.kmax64 = 1;
     }
-    cudaError_t e = cudaMemcpy(b->d_inst, b->h_inst.data(), sizeof(BatchInst) * n, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        sem_batch_destroy(b);
-        return bfail(SEM_ERR_CUDA, cudaGetErrorString(e));
-    }
-    // degree groups, largest instances first
-    for (int N = BATCH_MIN_N; N <= BATCH_MAX_N; ++N) {
-        BatchGroup g;
-        g.N = N;
-        for (int i = 0; i < n; ++i)
-            if (b->N[i] == N) g.members.push_back(i);
-        if (g.members.empty()) continue;
-        std::stable_sort(g.members.begin(), g.members.end(), [&](int x, int y) { return b->nloc[x] > b->nloc[y]; });
-        b->groups.push_back(std::move(g));
-    }
-    for (BatchGroup& g : b->groups) {
-        int kmax = 1;
-        if ((s = tune_group(b, g, &kmax))) {
-            sem_batch_destroy(b);
-            return s;
+    cudaError_t e = cudaSuccess;
+    // groups by degree and cluster size, largest instances first
+    for (int N = BATCH_MAX_N; N >= BATCH_MIN_N; --N)
+        for (int C = 8; C >= 1; C /= 2) {
+            BatchGroup g;
+            g.N = N;
+            g.cluster = C;
+            for (int i = 0; i < n; ++i)
+                if (b->N[i] == N && batch_cluster(b->nloc[i]) == C) g.members.push_back(i);
+            if (g.members.empty()) continue;
+            std::stable_sort(g.members.begin(), g.members.end(),
+                             [&](int x, int y) { return b->nloc[x] > b->nloc[y]; });
+            b->groups.push_back(std::move(g));
         }
-        b->stats.kmax_of_p[g.N - 1] = kmax;
-        for (int i : g.members) b->h_inst[i].kmax = kmax;
-        int per_sm = 0;
-        dispatch_batch_n(g.N, [&](auto nv) {
-            g.smem = batch_smem_n<decltype(nv)::value>(kmax);
+    for (BatchGroup& g : b->groups) {
+        int per_sm = 0, per_sm_plain = 0;
+        e = dispatch_batch_n(g.N, [&](auto nv) {
+            constexpr int NV = decltype(nv)::value;
+            for (int i : g.members) {
+                BatchInst& I = b->h_inst[i];
+                batch_pass<NV>(I.m.E, g.cluster, &I.kmax, &I.kmax64);
+                g.smem = std::max(g.smem, batch_smem_n<NV>(I.kmax, I.kmax64));
+                b->stats.kmax_of_p[NV - 1] = std::max(b->stats.kmax_of_p[NV - 1], I.kmax);
+            }
             return cudaSuccess;
         });
-        e = dispatch_batch_n(g.N, [&](auto nv) { return batch_prepare<decltype(nv)::value>(g.smem, &per_sm); });
-        if (e != cudaSuccess || per_sm < 1) {
+        // one opt-in per kernel: the largest of its groups
+        size_t opt = 0;
+        for (const BatchGroup& h : b->groups)
+            if (h.N == g.N) opt = std::max(opt, h.smem);
+        if (e == cudaSuccess)
+            e = dispatch_batch_n(g.N, [&](auto nv) { return batch_prepare<decltype(nv)::value>(opt, true, &per_sm); });
+        if (e == cudaSuccess)
+            e = dispatch_batch_n(
+                g.N, [&](auto nv) { return batch_prepare<decltype(nv)::value>(opt, false, &per_sm_plain); });
+        if (e != cudaSuccess || per_sm < 1 || per_sm_plain < 1) {
             sem_batch_destroy(b);
             return bfail(SEM_ERR_CUDA, "batched step kernel does not fit");
         }
-        g.grid = std::min<int>((int)g.members.size(), b->sms * per_sm);
+        g.grid = std::max(1, std::min<int>((int)g.members.size(), b->sms * per_sm / g.cluster));
+        g.grid_plain = std::min<int>((int)g.members.size(), b->sms * per_sm_plain);
         if ((s = balloc(b, (void**)&g.d_order, sizeof(int) * g.members.size())) ||
             (s = balloc(b, (void**)&g.d_queue, sizeof(int)))) {
             sem_batch_destroy(b);
@@ -409,8 +369,9 @@ static int capture_step(sem_batch* b, const BatchArgs& base)
             ba.queue = gr.d_queue;
             cudaMemsetAsync(gr.d_queue, 0, sizeof(int), gr.fork);
             dispatch_batch_n(gr.N, [&](auto nv) {
-                return batch_launch_step<decltype(nv)::value>(ba, ctx_mesh(b->ctx[gr.members[0]]), gr.grid, gr.smem,
-                                                               gr.fork);
+                return batch_launch_step<decltype(nv)::value>(ba, ctx_mesh(b->ctx[gr.members[0]]),
+                                                               ba.fdm ? gr.grid : gr.grid_plain,
+                                                               ba.fdm ? gr.cluster : 1, gr.smem, gr.fork);
             });
             cudaEventRecord(gr.done, gr.fork);
             cudaStreamWaitEvent(cs, gr.done, 0);

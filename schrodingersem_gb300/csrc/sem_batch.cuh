@@ -6,18 +6,18 @@
 // MINRES (FP32 inner iterations, FP64 refinement judged on the true
 // residual).
 //
-// Execution: one persistent launch per time step for all instances.  Blocks
-// take instances from a device work queue (largest first); a block advances
-// its instance by one step on its own -- projection, right-hand side, the
-// complete refined MINRES solve with block barriers and block reductions,
-// unmask -- so instances never wait for one another and each records its
-// own convergence flag and iteration count.  The step (queue reset + kernel)
+// Execution: one persistent launch per time step and group of instances (same
+// degree and cluster size) on forked streams.  A cluster of 1, 2, 4 or 8 blocks
+// takes an instance from its group's device work queue (largest first) and
+// advances it by one step on its own -- projection, right-hand side, the
+// complete refined stage solve with cluster barriers and reductions through
+// distributed shared memory, unmask -- so instances never wait for one another
+// and each records its own convergence flag and iteration count.  The cluster
+// size grows with the instance (batch_cluster), so that the largest ones do not
+// set the length of a step from a single SM.  The step (queue resets + kernels)
 // is captured once as a CUDA graph and replayed; every per-step quantity
-// (history slot, BDF coefficient) is derived on the device from the
-// instance's own step counter, so the same graph serves every step.  The
-// staging capacity (elements per pass of the element kernels, which sets
-// the threads working on one element) is chosen per degree by a timing
-// sweep at setup.
+// (history slot, BDF coefficient) is derived on the device from the instance's
+// own step counter, so the same graph serves every step.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -27,10 +27,16 @@
 
 namespace semgb {
 
-constexpr int BATCH_TPB = 512;
+// threads per block: with the element preconditioner two blocks per SM, without
+// (one block per instance, MINRES) one
+constexpr int BATCH_TPB = 256, BATCH_TPB_PLAIN = 512;
 constexpr int BATCH_MIN_N = 3;  // p = 2
 constexpr int BATCH_MAX_N = 9;  // p = 8
-constexpr size_t BATCH_SMEM_BUDGET = 96 * 1024;
+constexpr size_t BATCH_SMEM_BUDGET = 108 * 1024;  // two blocks per SM
+// blocks that share an instance of this many element-local nodes: at least 2,048
+// nodes each.  Measured on 160 instances of 4^2..32^2 elements, p = 4, 6, 8, two
+// steps (the largest has 83 k nodes): see the figures at k_batch_bdf2
+inline int batch_cluster(long long nodes) { return nodes >= 16384 ? 8 : nodes >= 8192 ? 4 : nodes >= 4096 ? 2 : 1; }
 
 struct BatchInst {
     DevMesh m;
@@ -43,11 +49,13 @@ struct BatchInst {
     double* r64;       // 2 planes
     double* Y64;       // 2 planes
     float* x32;        // 2 planes
+    const float4* fac4;  // per-node data of the stage solver (k_cg_prep)
+    const float* nnw;
     SolveOut* out;
     int* step;         // steps taken
     int* status;       // 0 running, 1 stopped (a stage solve failed)
     long long* iters;  // inner iterations over all steps
-    int kmax;          // elements per pass of the element kernels
+    int kmax, kmax64;  // elements per pass of the stage solver and of its FP64 residual
 };
 
 struct BatchArgs {
@@ -61,15 +69,18 @@ struct BatchArgs {
     int max_sweeps, fdm;
 };
 
+// elements per pass for an instance of E elements in clusters of C blocks
 template <int N>
-size_t batch_smem_n(int kmax);
+void batch_pass(int E, int C, int* kmax, int* kmax64);
 template <int N>
-cudaError_t batch_prepare(size_t smem, int* per_sm);
+size_t batch_smem_n(int kmax, int kmax64);
 template <int N>
-cudaError_t batch_launch_step(const BatchArgs& ba, const DevMesh& m0, int grid, size_t smem, cudaStream_t st);
+cudaError_t batch_prepare(size_t smem, bool fdm, int* per_sm);
 template <int N>
-cudaError_t batch_launch_probe(const BatchInst* inst, const int* list, int nlist, int kmax, int reps, float* sink,
-                               int grid, cudaStream_t st);
+cudaError_t batch_prep_instance(const DevMesh& m, void* fac, float* wt, cudaStream_t st);
+template <int N>
+cudaError_t batch_launch_step(const BatchArgs& ba, const DevMesh& m0, int grid, int cluster, size_t smem,
+                              cudaStream_t st);
 
 }  // namespace semgb
 
@@ -82,26 +93,29 @@ namespace semgb {
 
 template <int N>
 __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned char* smraw, double* red,
-                              MinresScal<float>& sc, double* sweep_state, float* fdmS, float* fdmL,
+                              MinresScal<float>& sc, double* sweep_state, float* fdmS, float* fdmL, Team& tm,
                               const EoD<N, double>& et, const CgTab<N>& tab)
 {
     constexpr int NN = N * N;
     const DevMesh& m = I.m;
     const long long n = m.n;
     const int k = *I.step;
-    if (*I.status) return;
+    if (*I.status) return;  // the same in every block of the cluster
+    // this block's elements
+    const int eb = (int)((long long)tm.rank * m.E / tm.size), ee = (int)((long long)(tm.rank + 1) * m.E / tm.size);
+    const long long nb = (long long)eb * NN, ne = (long long)ee * NN;
     double* hnew = I.hist[k & 1];
     const double* hold = I.hist[(k + 1) & 1];
     // proj(p) (galerkin.hpp:42-57 via schrodinger.hpp:69-78): mass * p per
     // element, assembled and masked; the imaginary plane negated
-    for (long long idx = threadIdx.x; idx < n; idx += blockDim.x) {
+    for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
         const double ms = m.mass[idx];
         I.Y64[idx] = ms * I.p[idx];
         I.Y64[n + idx] = ms * I.p[n + idx];
     }
-    __syncthreads();
+    team_barrier<TEAM_CLUSTER>(tm);
     const double c0 = -1.0 / 3.0, c1 = 4.0 / 3.0;  // schrodinger.hpp:102
-    for (long long idx = threadIdx.x; idx < n; idx += blockDim.x) {
+    for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
         const int e = (int)(idx / NN);
         const int node = (int)(idx - (long long)e * NN);
         const NodeInfo ni = node_info<N>(m, e, node % N, node / N);
@@ -113,7 +127,7 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
             I.b[c * n + idx] = (k == 0) ? v : c0 * hold[c * n + idx] + c1 * v;
         }
     }
-    __syncthreads();
+    team_barrier<TEAM_CLUSTER>(tm);
     // stage solve Res(alpha) p = b from p (schrodinger.hpp:97,104), alpha = dt
     // on the first step, 2 dt / 3 after (schrodinger.hpp:98-99)
     SolveArgs a{};
@@ -129,9 +143,10 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
     a.tol = ba.tol;
     a.x_is_zero = 0;
     a.kmax = I.kmax;
+    a.kmax64 = I.kmax64;
     a.rel_to_b = 0;
     a.timeout_ns = 0;
-    a.sync = nullptr;  // block-local
+    a.sync = nullptr;  // block-local MINRES
     a.out = I.out;
     MixedArgs mx{};
     mx.inner_tol = ba.inner_tol;
@@ -144,26 +159,51 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
     mx.x32[0] = I.x32;
     mx.x32[1] = I.x32 + n;
     mx.pot32 = I.pot32;
+    mx.fac4 = I.fac4;
+    mx.nnw = I.nnw;
     mx.pinv32 = nullptr;
     mx.fdm = ba.fdm;
     mx.fused = 0;
     mx.outer_scale = ba.outer_scale;
     mx.adaptive = 1;
-    mixed_solve<N, OP_RES, MIXED_BATCH>(m, a, I.w, mx, 0, m.E, true, smraw, red, sc, sweep_state, fdmS, fdmL, et,
-                                     &tab);
+    int done = 0;
+    bool minres = !ba.fdm;
+    if (ba.fdm) {
+        CgRefine r{};
+        cg_refine<N, TEAM_CLUSTER>(m, a, I.w, mx, eb, ee, smraw, fdmL, et, tab, tm, r);
+        done = r.inner;
+        minres = r.fallback;
+        a.maxit -= done;
+        a.r0_given = r.r0;
+        if (tm.rank == 0 && threadIdx.x == 0) {
+            I.out->success = r.conv ? 1 : 0;
+            I.out->n_iter = r.inner;
+            I.out->residual = r.rn;
+            I.out->inner_iters = r.inner;
+            I.out->sweeps = r.sweeps;
+        }
+    }
+    if (minres) {  // no preconditioner, or the conjugate gradients gave up: the whole instance on one block
+        if (tm.rank == 0) {
+            a.kmax = a.kmax64 = I.kmax64;
+            mixed_solve<N, OP_RES, MIXED_BATCH>(m, a, I.w, mx, 0, m.E, true, smraw, red, sc, sweep_state, fdmS, fdmL,
+                                                et);
+        }
+        team_barrier<TEAM_CLUSTER>(tm);
+    }
     // unmask(p) (schrodinger.hpp:105-106): owner copies are never written here
-    for (long long idx = threadIdx.x; idx < n; idx += blockDim.x) {
+    for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
         const int e = (int)(idx / NN);
         const int node = (int)(idx - (long long)e * NN);
         const long long src = ni_gather_src(m, node_info<N>(m, e, node % N, node / N), e, idx);
         if (src != idx) {
-            I.p[idx] = I.p[src];
-            I.p[n + idx] = I.p[n + src];
+            I.p[idx] = __ldcg(I.p + src);
+            I.p[n + idx] = __ldcg(I.p + n + src);
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        *I.iters += I.out->n_iter;
+    team_barrier<TEAM_CLUSTER>(tm);
+    if (tm.rank == 0 && threadIdx.x == 0) {
+        *I.iters += I.out->n_iter + (minres ? done : 0);
         if (!I.out->success) *I.status = 1;
         *I.step = k + 1;
     }
@@ -171,7 +211,8 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
 
 // one time step of every instance in ba.order (all of degree N)
 template <int N>
-__global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_bdf2(BatchArgs ba, const __grid_constant__ EoD<N, double> et, const __grid_constant__ CgTab<N> tab)
+__global__ void __launch_bounds__(BATCH_TPB_PLAIN, 1)
+    k_batch_bdf2(BatchArgs ba, const __grid_constant__ EoD<N, double> et, const __grid_constant__ CgTab<N> tab)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[34];
@@ -179,87 +220,78 @@ __global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_bdf2(BatchArgs ba, const
     __shared__ double sweep_state[3];
     __shared__ float fdmS[N * N], fdmL[N];
     __shared__ __align__(16) unsigned char ibuf[sizeof(BatchInst)];
-    __shared__ int next;
+    __shared__ unsigned long long next;
     BatchInst& I = *reinterpret_cast<BatchInst*>(ibuf);
+    Team tm{nullptr, 0, nullptr, 0, cluster_rank(), cluster_size()};
     for (;;) {
-        if (threadIdx.x == 0) next = atomicAdd(ba.queue, 1);
-        __syncthreads();
-        const int q = next;
+        if (tm.rank == 0 && threadIdx.x == 0) {
+            const int q = atomicAdd(ba.queue, 1);
+            next = (unsigned long long)q;
+            for (int r = 1; r < tm.size; ++r) cluster_put(&next, r, (unsigned long long)q);
+        }
+        team_barrier<TEAM_CLUSTER>(tm);
+        const int q = (int)next;
         if (q >= ba.n) break;
         if (threadIdx.x == 0) I = ba.inst[ba.order[q]];
         __syncthreads();
-        bdf2_instance<N>(I, ba, smraw, red, sc, sweep_state, fdmS, fdmL, et, tab);
-        __syncthreads();
+        bdf2_instance<N>(I, ba, smraw, red, sc, sweep_state, fdmS, fdmL, tm, et, tab);
+        team_barrier<TEAM_CLUSTER>(tm);  // `next` and the instance read, before rank 0 takes another
     }
-}
-
-// staging-capacity probe: every block takes instances of the probed degree
-// and runs `reps` block-local FP32 Res applies with capacity kmax
-template <int N>
-__global__ void __launch_bounds__(BATCH_TPB, 1) k_batch_probe(const BatchInst* inst, const int* list, int nlist,
-                                                               int kmax, int reps, float* sink)
-{
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ __align__(16) unsigned char ibuf[sizeof(BatchInst)];
-    BatchInst& I = *reinterpret_cast<BatchInst*>(ibuf);
-    float* sm = (float*)smraw;
-    for (int q = blockIdx.x; q < nlist; q += gridDim.x) {
-        if (threadIdx.x == 0) I = inst[list[q]];
-        __syncthreads();
-        const DevMesh& m = I.m;
-        const Fac<float> fac = fac_of<float>(m);
-        load_dmat_raw<N, float>(sm, m);
-        __syncthreads();
-        const long long n = m.n;
-        float* Y = I.w.Y[0];
-        for (int r = 0; r < reps; ++r)
-            for (int e0 = 0; e0 < m.E; e0 += kmax)
-                apply_range<N, float, OP_RES>(
-                    sm, kmax, nullptr, fac, I.pot32, 0.01f, e0, min(kmax, m.E - e0),
-                    [&](int, int, int, long long flat, float* u) {
-                        u[0] = I.w.L[0][flat];
-                        u[1] = I.w.L[0][n + flat];
-                    },
-                    [&](int, int, int, long long flat, const float* o) {
-                        Y[flat] = o[0];
-                        Y[n + flat] = o[1];
-                    });
-        if (threadIdx.x == 0 && sink) sink[0] = Y[0];
-        __syncthreads();
-    }
+    team_barrier<TEAM_CLUSTER>(tm);  // no block leaves while another may still write its shared memory
 }
 
 template <int N>
-size_t batch_smem_n(int kmax)
+void batch_pass(int E, int C, int* kmax, int* kmax64)
 {
-    return std::max(range_smem_bytes<N, double, OP_RES>(kmax), cg_smem_bytes<N>(kmax));
+    const int share = (E + C - 1) / C;
+    int k = std::max(1, std::min(share, BATCH_TPB / N));  // a line per thread
+    while (k > 1 && cg_smem_bytes<N>(k) > BATCH_SMEM_BUDGET) --k;
+    const int passes = (share + k - 1) / k;
+    *kmax = (share + passes - 1) / passes;
+    int k6 = std::max(1, std::min(share, BATCH_TPB / N));
+    while (k6 > 1 && range_smem_bytes<N, double, OP_RES>(k6) > BATCH_SMEM_BUDGET) --k6;
+    *kmax64 = k6;
+}
+
+template <int N>
+size_t batch_smem_n(int kmax, int kmax64)
+{
+    return std::max(range_smem_bytes<N, double, OP_RES>(kmax64), cg_smem_bytes<N>(kmax));
 }
 
 // shared-memory opt-in and resident blocks per SM of the step kernel
 template <int N>
-cudaError_t batch_prepare(size_t smem, int* per_sm)
+cudaError_t batch_prepare(size_t smem, bool fdm, int* per_sm)
 {
     cudaError_t e = cudaFuncSetAttribute(k_batch_bdf2<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_batch_bdf2<N>, BATCH_TPB, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_batch_bdf2<N>, fdm ? BATCH_TPB : BATCH_TPB_PLAIN,
+                                                         smem);
 }
 
 template <int N>
-cudaError_t batch_launch_step(const BatchArgs& ba, const DevMesh& m0, int grid, size_t smem, cudaStream_t st)
+cudaError_t batch_prep_instance(const DevMesh& m, void* fac, float* wt, cudaStream_t st)
 {
-    k_batch_bdf2<N><<<grid, BATCH_TPB, smem, st>>>(ba, eo_d_table<N, double>(m0.Dh), cg_table<N>(m0));
+    k_cg_prep<N><<<(int)std::min<long long>((m.n + 255) / 256, 1024), 256, 0, st>>>(m, (float4*)fac, wt);
     return cudaGetLastError();
 }
 
 template <int N>
-cudaError_t batch_launch_probe(const BatchInst* inst, const int* list, int nlist, int kmax, int reps, float* sink,
-                               int grid, cudaStream_t st)
+cudaError_t batch_launch_step(const BatchArgs& ba, const DevMesh& m0, int grid, int cluster, size_t smem,
+                              cudaStream_t st)
 {
-    const size_t sm = batch_smem_n<N>(kmax);
-    cudaError_t e = cudaFuncSetAttribute(k_batch_probe<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    k_batch_probe<N><<<grid, BATCH_TPB, sm, st>>>(inst, list, nlist, kmax, reps, sink);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid * cluster);
+    cfg.blockDim = dim3(ba.fdm ? BATCH_TPB : BATCH_TPB_PLAIN);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_batch_bdf2<N>, ba, eo_d_table<N, double>(m0.Dh), cg_table<N>(m0));
 }
 
 }  // namespace semgb
@@ -268,10 +300,10 @@ cudaError_t batch_launch_probe(const BatchInst* inst, const int* list, int nlist
 
 #define SEM_BATCH_INSTANTIATE(NV)                                                                        \
     namespace semgb {                                                                                    \
-    template size_t batch_smem_n<NV>(int);                                                               \
-    template cudaError_t batch_prepare<NV>(size_t, int*);                                                \
-    template cudaError_t batch_launch_step<NV>(const BatchArgs&, const DevMesh&, int, size_t,            \
+    template void batch_pass<NV>(int, int, int*, int*);                                                  \
+    template size_t batch_smem_n<NV>(int, int);                                                          \
+    template cudaError_t batch_prepare<NV>(size_t, bool, int*);                                          \
+    template cudaError_t batch_prep_instance<NV>(const DevMesh&, void*, float*, cudaStream_t);           \
+    template cudaError_t batch_launch_step<NV>(const BatchArgs&, const DevMesh&, int, int, size_t,       \
                                                  cudaStream_t);                                          \
-    template cudaError_t batch_launch_probe<NV>(const BatchInst*, const int*, int, int, int, float*, int, \
-                                                cudaStream_t);                                           \
     }

@@ -32,15 +32,69 @@
 
 namespace semgb {
 
-// All-reduce of K per-thread FP32 partials over the team that solves one mesh:
-// a cooperative grid (gs) behind one grid barrier, or one block (gs null).
-// Warp sums in FP32, FP64 from there on, every sum in one fixed order.
-// partials: [slot][K][grid], consecutive reductions alternate slots
-template <int K>
-__device__ __forceinline__ void team_sum(const float (&v)[K], double* partials, int slot, GridSync* gs, long long tmo,
-                                         bool& ok, double (&out)[K])
+// ------------------------------------------------------------------- teams
+// The blocks that solve one mesh together: a cooperative grid (one mesh), or a
+// thread-block cluster (one instance of a batch; a cluster of one is a block).
+enum TeamKind : int { TEAM_GRID = 0, TEAM_CLUSTER = 1 };
+struct Team {
+    GridSync* gs;      // grid
+    long long tmo;
+    double* partials;  // grid: [slot][K][grid] partial sums
+    int slot;          // alternates
+    int rank, size;
+};
+__device__ __forceinline__ int cluster_rank()
 {
-    __shared__ double ts[K][33];
+    int r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ int cluster_size()
+{
+    int r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+// every thread of every block of the cluster; orders their memory accesses
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_put(void* p, int rank, unsigned long long v)
+{
+    unsigned la = (unsigned)__cvta_generic_to_shared(p), ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(la), "r"(rank));
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ra), "l"(v) : "memory");
+}
+template <int TEAM>
+__device__ __forceinline__ bool team_barrier(Team& t)
+{
+    if (TEAM == TEAM_GRID) return grid_barrier(t.gs, t.tmo);
+    if (t.size > 1) cluster_sync();
+    else __syncthreads();
+    return true;
+}
+
+// (hi, lo) += (h, l): hi + lo carries twice FP32's precision (TwoSum, D. E.
+// Knuth, The Art of Computer Programming 2, 4.2.2).  FP64 additions and
+// conversions take 64 cycles each on GB300 and would dominate a reduction.
+__device__ __forceinline__ void two_add(float& hi, float& lo, float h, float l)
+{
+    const float s = __fadd_rn(hi, h), t = __fadd_rn(s, -hi);
+    const float e = __fadd_rn(__fadd_rn(hi, -__fadd_rn(s, -t)), __fadd_rn(h, -t));
+    hi = s;
+    lo = __fadd_rn(lo, __fadd_rn(l, e));
+}
+
+// All-reduce of K per-thread FP32 partials over the team: warp sums in FP32,
+// pairs (hi, lo) from there on, every sum in one fixed order.  Consecutive
+// reductions alternate slots.
+constexpr int TEAM_MAX_CLUSTER = 8;
+template <int TEAM, int K>
+__device__ __forceinline__ bool team_sum(const float (&v)[K], Team& tm, float (&out)[K])
+{
+    __shared__ float ts[K][33];
+    __shared__ f2_t cs[2][K][TEAM_MAX_CLUSTER];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     float a[K];
 #pragma unroll
@@ -52,38 +106,137 @@ __device__ __forceinline__ void team_sum(const float (&v)[K], double* partials, 
     __syncthreads();
     if (lane == 0)
 #pragma unroll
-        for (int k = 0; k < K; ++k) ts[k][wid] = (double)a[k];
+        for (int k = 0; k < K; ++k) ts[k][wid] = a[k];
     __syncthreads();
+    float hi[K], lo[K];
+    auto tree = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                two_add(hi[k], lo[k], __shfl_down_sync(0xffffffffu, hi[k], o), __shfl_down_sync(0xffffffffu, lo[k], o));
+    };
+    const int slot = tm.slot;
+    tm.slot ^= 1;
     const int G = gridDim.x;
-    double* p = partials + (size_t)slot * K * G;
+    f2_t* p = (f2_t*)tm.partials + (size_t)slot * K * G;
     if (wid == 0) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            double s = lane < nw ? ts[k][lane] : 0.0;
+            hi[k] = lane < nw ? ts[k][lane] : 0.f;
+            lo[k] = 0.f;
+        }
+        tree();
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-            if (lane == 0) {
-                if (gs) p[(size_t)k * G + blockIdx.x] = s;
-                else ts[k][32] = s;
+        for (int k = 0; k < K; ++k) {
+            const f2_t w = f2pack(hi[k], lo[k]);
+            if (TEAM == TEAM_GRID) {
+                if (lane == 0) p[(size_t)k * G + blockIdx.x] = w;
+            } else if (tm.size == 1) {
+                if (lane == 0) ts[k][32] = hi[k] + lo[k];
+            } else {
+                const f2_t w0 = __shfl_sync(0xffffffffu, w, 0);
+                if (lane < tm.size) cluster_put(&cs[slot][k][tm.rank], lane, w0);
             }
         }
     }
-    ok = true;
-    if (gs) {
-        ok = grid_barrier(gs, tmo);
-        if (wid == 0)
+    bool ok = true;
+    if (TEAM == TEAM_GRID || tm.size > 1) {
+        ok = team_barrier<TEAM>(tm);
+        if (wid == 0) {
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                double s = 0.0;
-                for (int q = lane; q < G; q += 32) s += __ldcg(p + (size_t)k * G + q);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-                if (lane == 0) ts[k][32] = s;
+                hi[k] = lo[k] = 0.f;
+                if (TEAM == TEAM_GRID) {
+                    for (int q = lane; q < G; q += 32) {
+                        float h, l;
+                        f2unpack(__ldcg(p + (size_t)k * G + q), h, l);
+                        two_add(hi[k], lo[k], h, l);
+                    }
+                } else if (lane < tm.size) {
+                    f2unpack(cs[slot][k][lane], hi[k], lo[k]);
+                }
             }
+            tree();
+            if (lane == 0)
+#pragma unroll
+                for (int k = 0; k < K; ++k) ts[k][32] = hi[k] + lo[k];
+        }
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; ++k) out[k] = ts[k][32];
+    return ok;
+}
+// the same of two FP64 values (the refinement's norms)
+template <int TEAM>
+__device__ __forceinline__ bool team_sum64(double v0, double v1, Team& tm, double& r0, double& r1)
+{
+    __shared__ double ts[2][33];
+    __shared__ double cs[2][2][TEAM_MAX_CLUSTER];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    auto tree = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            v0 += __shfl_down_sync(0xffffffffu, v0, o);
+            v1 += __shfl_down_sync(0xffffffffu, v1, o);
+        }
+    };
+    tree();
+    __syncthreads();
+    if (lane == 0) {
+        ts[0][wid] = v0;
+        ts[1][wid] = v1;
+    }
+    __syncthreads();
+    const int slot = tm.slot;
+    tm.slot ^= 1;
+    const int G = gridDim.x;
+    double* p = tm.partials + (size_t)slot * 2 * G;
+    if (wid == 0) {
+        v0 = lane < nw ? ts[0][lane] : 0.0;
+        v1 = lane < nw ? ts[1][lane] : 0.0;
+        tree();
+        if (TEAM == TEAM_GRID) {
+            if (lane == 0) {
+                p[blockIdx.x] = v0;
+                p[G + blockIdx.x] = v1;
+            }
+        } else {
+            const double w0 = __shfl_sync(0xffffffffu, v0, 0), w1 = __shfl_sync(0xffffffffu, v1, 0);
+            if (tm.size > 1) {
+                if (lane < tm.size) {
+                    cluster_put(&cs[slot][0][tm.rank], lane, (unsigned long long)__double_as_longlong(w0));
+                    cluster_put(&cs[slot][1][tm.rank], lane, (unsigned long long)__double_as_longlong(w1));
+                }
+            } else if (lane == 0) {
+                cs[slot][0][0] = w0;
+                cs[slot][1][0] = w1;
+            }
+        }
+    }
+    const bool ok = team_barrier<TEAM>(tm);
+    if (wid == 0) {
+        v0 = v1 = 0.0;
+        if (TEAM == TEAM_GRID) {
+            for (int q = lane; q < G; q += 32) {
+                v0 += __ldcg(p + q);
+                v1 += __ldcg(p + G + q);
+            }
+        } else if (lane < tm.size) {
+            v0 = cs[slot][0][lane];
+            v1 = cs[slot][1][lane];
+        }
+        tree();
+        if (lane == 0) {
+            ts[0][32] = v0;
+            ts[1][32] = v1;
+        }
+    }
+    __syncthreads();
+    r0 = ts[0][32];
+    r1 = ts[1][32];
+    return ok;
 }
 
 // coefficient tables of the FP32 line passes (kernel parameter)
@@ -101,12 +254,30 @@ inline CgTab<N> cg_table(const DevMesh& m)
     return t;
 }
 
-// shared memory of a pass over kmax elements: three planes of pairs, three of
-// factors
+// shared memory of a pass over kmax elements: the factors {g11, -g12, g22, mass}
+// and three planes of pairs
 template <int N>
 __host__ __device__ constexpr size_t cg_smem_bytes(int kmax)
 {
-    return (size_t)kmax * line_es(N) * (3 * sizeof(f2_t) + 3 * sizeof(float));
+    return (size_t)kmax * line_es(N) * (sizeof(float4) + 3 * sizeof(f2_t));
+}
+
+// Per-node data of the streaming iteration, built once per mesh: the factors in
+// one 16-byte load, and the Neumann-Neumann weight (1 / copies, 0 on a Dirichlet
+// boundary), negative on copies that are not the owner
+template <int N>
+__global__ void k_cg_prep(DevMesh m, float4* __restrict__ fac, float* __restrict__ wt)
+{
+    constexpr int NN = N * N;
+    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < m.n;
+         idx += (long long)gridDim.x * blockDim.x) {
+        const int e = (int)(idx / NN);
+        const int node = (int)(idx - (long long)e * NN);
+        const NodeInfo ni = node_info<N>(m, e, node % N, node / N);
+        const float w = nn_weight<N, float>(m, ni, e);
+        fac[idx] = make_float4(m.g11f[idx], -m.g12f[idx], m.g22f[idx], m.massf[idx]);
+        wt[idx] = ni_owner(ni) ? w : -w;
+    }
 }
 
 // the three operator passes on staged elements (all threads; leading and
@@ -114,7 +285,7 @@ __host__ __device__ constexpr size_t cg_smem_bytes(int kmax)
 // D_xi^T f1 + D_eta^T f2 (the weak Laplacian) of both components
 template <int N>
 __device__ __forceinline__ void cg_laplace(const EoD<N, f2_t>& t, const f2_t* su, f2_t* s1, f2_t* s2,
-                                           const float* sg, int gst, int ne)
+                                           const float4* sg, int ne)
 {
     constexpr int ES = line_es(N);
     const LineNe nb = line_ne(ne);
@@ -143,7 +314,8 @@ __device__ __forceinline__ void cg_laplace(const EoD<N, f2_t>& t, const f2_t* su
         for (int k = 0; k < N; ++k) {
             const int q = o + k * N;
             const f2_t ur = s1[q];
-            const f2_t g11 = f2dup(sg[q]), g12 = f2dup(-sg[gst + q]), g22 = f2dup(sg[2 * gst + q]);
+            const float4 g = sg[q];
+            const f2_t g11 = f2dup(g.x), g12 = f2dup(g.y), g22 = f2dup(g.z);
             s1[q] = f2fma(g12, us[k], f2mul(g11, ur));
             us[k] = f2fma(g12, ur, f2mul(g22, us[k]));
         }
@@ -235,6 +407,61 @@ __device__ __forceinline__ void cg_fdm(const EoS<N, f2_t>& t, f2_t* s, const flo
     }
 }
 
+// Assembly of the ring copies (continuous format, dss_value's sums) of ne
+// staged elements from e0 on, in place: s holds the block's own element values
+// Y every block's.  One task per ring node, so that the
+// dependent table and value loads of a pass are all in flight at once and the
+// loops over all nodes stay free of branches.
+template <int N>
+__device__ __forceinline__ void cg_ring(const DevMesh& m, const f2_t* Y, f2_t* s, int e0, int ne)
+{
+    constexpr int R = 4 * (N - 1), ES = line_es(N);
+#pragma unroll 2
+    for (int t = threadIdx.x; t < ne * R; t += blockDim.x) {
+        const int le = t / R, r = t - le * R;
+        const int sc = r / (N - 1), h = r - sc * (N - 1);  // h = 0: the corner the side starts at
+        const int i = sc == 0 ? h : sc == 1 ? N - 1 : sc == 2 ? N - 1 - h : 0;
+        const int j = sc == 0 ? 0 : sc == 1 ? h : sc == 2 ? N - 1 : N - 1 - h;
+        const int e = e0 + le;
+        const int fl = __ldg(m.flags + e);
+        f2_t* v = s + le * ES + j * N + i;
+        if (h != 0) {
+            const int sb = __ldg(m.side_base + 4 * e + sc), ss = __ldg(m.side_step + 4 * e + sc);
+            if ((fl >> (4 + sc)) & 1) {  // Dirichlet boundary
+                *v = 0ull;
+            } else if (!((fl >> (16 + sc)) & 1)) {
+                const long long q = (long long)sb + (long long)((sc & 1) ? j : i) * ss;
+                *v = f2add(*v, __ldcg(Y + q));
+            }
+        } else {
+            const int4* cl = reinterpret_cast<const int4*>(m.corner_nb + (size_t)(4 * e + sc) * CORNER_NB_MAX);
+            const int4 qa = __ldg(cl), qb = __ldg(cl + 1);
+            const int q[CORNER_NB_MAX] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+            f2_t sum = 0ull;  // csum = 0, then += in connected_elements order
+            if ((fl >> (12 + sc)) & 1) {
+            } else if (q[0] == -2) {  // more copies than the table holds
+                const int node = __ldg(m.corner_node + 4 * e + sc);
+                const int q0 = __ldg(m.node_ptr + node), q1 = __ldg(m.node_ptr + node + 1);
+                for (int k = q0; k < q1; ++k) {
+                    const int f = __ldg(m.node_flat + k);
+                    sum = f2add(sum, __ldcg(Y + f));
+                }
+            } else {
+                f2_t w[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) w[k] = q[k] >= 0 ? __ldcg(Y + q[k]) : 0ull;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (q[k] >= 0) sum = f2add(sum, w[k]);
+#pragma unroll
+                for (int k = 4; k < CORNER_NB_MAX; ++k)
+                    if (q[k] >= 0) sum = f2add(sum, __ldcg(Y + q[k]));
+            }
+            *v = sum;
+        }
+    }
+}
+
 // scalar state of the recurrence, identical on every thread (FP32; the
 // right-hand side is scaled to unit norm)
 struct CgScal {
@@ -276,91 +503,100 @@ struct CgOut {
     bool usable;  // the correction is finite
 };
 
-// Solves A d = b for the block's element range [eb, ee) (a team of blocks: a
-// cooperative grid, gs != nullptr, or one block).  rhs(flat, c) is the
-// right-hand side scaled to unit norm (continuous format).  The correction
-// (continuous format, scaled like b) is left in xo.  w: L[0] r, L[1] p, Y[0]
-// Y, Y[1] Zl.  Returns false when a wait timed out.
-template <int N, class Rhs>
-__device__ __forceinline__ bool cg_core(unsigned char* smraw, int kmax, const DevMesh& m,
-                                        const CgTab<N>& tab, const float* __restrict__ pot, float alpha, int eb,
-                                        int ee, const KrylovWork<float>& w, GridSync* gs, long long tmo, int& slot,
-                                        Rhs&& rhs, float* const* xo, int maxit, float tol_rel, const float* lam,
-                                        CgOut& res)
+// Solves A d = b for the block's element range [eb, ee) of its team's mesh.
+// rhs(flat) is the right-hand side pair scaled to unit norm (continuous format).
+// The correction (continuous format, scaled like b) is left in X.  Vectors are
+// arrays of n pairs: r, p, Y (element output of A p), Zl (weighted local
+// solves).  Returns false when a wait timed out.
+template <int N, int TEAM, class Rhs>
+__device__ __forceinline__ bool cg_core(unsigned char* smraw, int kmax, const DevMesh& m, const CgTab<N>& tab,
+                                        const float4* __restrict__ fac, const float* __restrict__ nnw,
+                                        const float* __restrict__ pot, float alpha, int eb, int ee,
+                                        const KrylovWork<float>& w, Team& tm, Rhs&& rhs, f2_t* __restrict__ X,
+                                        int maxit, float tol_rel, const float* lam, CgOut& res)
 {
     constexpr int NN = N * N;
     constexpr int ES = line_es(N);
-    const long long n = m.n;
-    const int gst = kmax * ES;
-    f2_t* su = (f2_t*)smraw;
-    f2_t* s1 = su + gst;
-    f2_t* s2 = s1 + gst;
-    float* sg = (float*)(s2 + gst);
-    float* R = w.L[0];
-    float* Pv = w.L[1];
-    float* Y = w.Y[0];
-    float* Zl = w.Y[1];
+    constexpr int U = 4;  // nodes a thread has in flight
+    float4* sg = (float4*)smraw;
+    f2_t* su = (f2_t*)(sg + kmax * ES);
+    f2_t* s1 = su + kmax * ES;
+    f2_t* s2 = s1 + kmax * ES;
+    float* sw = (float*)s2;  // Phase B: weights
+    f2_t* __restrict__ const R = (f2_t*)w.L[0];
+    f2_t* __restrict__ const P = (f2_t*)w.L[1];
+    f2_t* const Y = (f2_t*)w.Y[0];
+    f2_t* const Zl = (f2_t*)w.Y[1];
     CgScal sc{};
-    bool ok = true;
     res.it = 0;
     res.conv = false;
     res.usable = true;
     if (maxit < 1) return true;
     // Phase B of every iteration (first: r = b)
-    auto phase_b = [&](bool first, double (&out)[3]) {
+    auto phase_b = [&](bool first, float (&out)[3]) -> bool {
         float rz0 = 0.f, rz1 = 0.f, rr = 0.f;
+        const f2_t na0 = f2dup(-sc.a0), cross = f2pack(sc.a1, -sc.a1);
         for (int e0 = eb; e0 < ee; e0 += kmax) {
             const int ne = min(kmax, ee - e0);
             const int total = ne * NN;
+            const long long base = (long long)e0 * NN;
+            if (!first) {  // the assembled A p
 #pragma unroll 4
-            for (int t = threadIdx.x; t < total; t += blockDim.x) {
-                const int le = t / NN;
-                const int node = t - le * NN;
-                const int e = e0 + le;
-                const long long flat = (long long)e * NN + node;
-                const NodeInfo ni = node_info<N>(m, e, node % N, node / N);
-                float r0, r1;
-                if (first) {
-                    r0 = rhs(flat, 0);
-                    r1 = rhs(flat, 1);
-                } else {
-                    const float q0 = dss_value<N, float, DSS_CONT>(m, Y, ni, e, flat);
-                    const float q1 = dss_value<N, float, DSS_CONT>(m, Y + n, ni, e, flat);
-                    r0 = R[flat] - fmaf(sc.a0, q0, -sc.a1 * q1);
-                    r1 = R[n + flat] - fmaf(sc.a0, q1, sc.a1 * q0);
+                for (int t = threadIdx.x; t < total; t += blockDim.x) su[t + t / NN * (ES - NN)] = __ldcg(Y + base + t);
+                __syncthreads();
+                cg_ring<N>(m, Y, su, e0, ne);
+                __syncthreads();
+            }
+            for (int t0 = threadIdx.x; t0 < total; t0 += U * blockDim.x) {
+                f2_t r[U];
+                float wt[U];
+#pragma unroll
+                for (int h = 0; h < U; ++h) {  // every load of the group before its stores
+                    const int t = t0 + h * blockDim.x;
+                    if (t < total) {
+                        r[h] = first ? rhs(base + t) : R[base + t];
+                        wt[h] = __ldg(nnw + base + t);
+                    }
                 }
-                R[flat] = r0;
-                R[n + flat] = r1;
-                if (ni_owner(ni)) rr = fmaf(r0, r0, fmaf(r1, r1, rr));
-                const float wt = nn_weight<N, float>(m, ni, e);
-                su[le * ES + node] = f2pack(wt * r0, wt * r1);
+#pragma unroll
+                for (int h = 0; h < U; ++h) {
+                    const int t = t0 + h * blockDim.x;
+                    if (t >= total) continue;
+                    const int q = t + t / NN * (ES - NN);
+                    if (!first) {  // r -= a A p
+                        float q0, q1;
+                        const f2_t qv = su[q];
+                        f2unpack(qv, q0, q1);
+                        r[h] = f2fma(cross, f2pack(q1, q0), f2fma(na0, qv, r[h]));
+                    }
+                    R[base + t] = r[h];
+                    float r0, r1;
+                    f2unpack(r[h], r0, r1);
+                    if (wt[h] > 0.f) rr = fmaf(r0, r0, fmaf(r1, r1, rr));
+                    const float wa = fabsf(wt[h]);
+                    su[q] = f2mul(f2dup(wa), r[h]);
+                    sw[q] = wa;
+                }
             }
             __syncthreads();
             cg_fdm<N>(tab.S, su, lam, alpha, ne, [&](int le) { return __ldg(m.fdm_el + e0 + le); }, rz0, rz1);
             __syncthreads();
+#pragma unroll 4
             for (int t = threadIdx.x; t < total; t += blockDim.x) {
-                const int le = t / NN;
-                const int node = t - le * NN;
-                const int e = e0 + le;
-                const long long flat = (long long)e * NN + node;
-                const float wt = nn_weight<N, float>(m, node_info<N>(m, e, node % N, node / N), e);
-                float a, b;
-                f2unpack(su[le * ES + node], a, b);
-                Zl[flat] = wt * a;
-                Zl[n + flat] = -wt * b;
+                const int q = t + t / NN * (ES - NN);
+                const float wa = sw[q];
+                Zl[base + t] = f2mul(f2pack(wa, -wa), su[q]);
             }
             __syncthreads();
         }
         const float v[3] = {rz0, rz1, rr};
-        team_sum<3>(v, w.partials, slot, gs, tmo, ok, out);
-        slot ^= 1;
+        return team_sum<TEAM, 3>(v, tm, out);
     };
-    double o3[3], o2[2];
-    phase_b(true, o3);
-    if (!ok) return false;
-    sc.rho0 = (float)o3[0];
-    sc.rho1 = (float)o3[1];
-    const float bb = (float)o3[2];
+    float o3[3], o2[2];
+    if (!phase_b(true, o3)) return false;
+    sc.rho0 = o3[0];
+    sc.rho1 = o3[1];
+    const float bb = o3[2];
     sc.best = bb;
     if (!(bb > 0.f)) {  // nothing to solve (or a NaN right-hand side: the caller sees |b|)
         res.conv = bb == 0.f;
@@ -374,75 +610,78 @@ __device__ __forceinline__ bool cg_core(unsigned char* smraw, int kmax, const De
         const bool first = it == 1;
         // ---- Phase A
         float d0 = 0.f, d1 = 0.f;
+        const f2_t b0 = f2dup(sc.b0), bx = f2pack(sc.b1, -sc.b1), a0 = f2dup(sc.a0), ax = f2pack(sc.a1, -sc.a1);
         for (int e0 = eb; e0 < ee; e0 += kmax) {
             const int ne = min(kmax, ee - e0);
             const int total = ne * NN;
+            const long long base = (long long)e0 * NN;
 #pragma unroll 4
-            for (int t = threadIdx.x; t < total; t += blockDim.x) {
-                const int le = t / NN;
-                const int node = t - le * NN;
-                const int e = e0 + le;
-                const long long flat = (long long)e * NN + node;
-                const NodeInfo ni = node_info<N>(m, e, node % N, node / N);
-                const int q = le * ES + node;
-                sg[q] = __ldg(m.g11f + flat);
-                sg[gst + q] = __ldg(m.g12f + flat);
-                sg[2 * gst + q] = __ldg(m.g22f + flat);
-                float p0 = dss_value<N, float, DSS_CONT>(m, Zl, ni, e, flat);
-                float p1 = dss_value<N, float, DSS_CONT>(m, Zl + n, ni, e, flat);
-                float x0 = 0.f, x1 = 0.f;
-                if (!first) {
-                    const float a = Pv[flat], b = Pv[n + flat];
-                    x0 = fmaf(sc.a0, a, sc.a1 * b);
-                    x1 = fmaf(sc.a0, b, -sc.a1 * a);
-                    if (it > 2) {
-                        x0 += xo[0][flat];
-                        x1 += xo[1][flat];
-                    }
-                    p0 += fmaf(sc.b0, a, sc.b1 * b);
-                    p1 += fmaf(sc.b0, b, -sc.b1 * a);
-                    xo[0][flat] = x0;
-                    xo[1][flat] = x1;
-                }
-                Pv[flat] = p0;
-                Pv[n + flat] = p1;
-                su[q] = f2pack(p0, p1);
+            for (int t = threadIdx.x; t < total; t += blockDim.x) {  // the assembled z, the factors
+                const int q = t + t / NN * (ES - NN);
+                const f2_t z = __ldcg(Zl + base + t);
+                const float4 g = __ldg(fac + base + t);
+                su[q] = z;
+                sg[q] = g;
             }
             __syncthreads();
-            cg_laplace<N>(tab.D, su, s1, s2, sg, gst, ne);
+            cg_ring<N>(m, Zl, su, e0, ne);
+            __syncthreads();
+            for (int t0 = threadIdx.x; t0 < total; t0 += U * blockDim.x) {
+                f2_t pv[U], xv[U];
+#pragma unroll
+                for (int h = 0; h < U; ++h) {
+                    const int t = t0 + h * blockDim.x;
+                    if (t < total && !first) {
+                        pv[h] = P[base + t];
+                        xv[h] = it > 2 ? X[base + t] : 0ull;
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < U; ++h) {
+                    const int t = t0 + h * blockDim.x;
+                    if (t >= total) continue;
+                    const int q = t + t / NN * (ES - NN);
+                    f2_t z = su[q];
+                    if (!first) {  // x += a p, p = z + beta p
+                        float a, b;
+                        f2unpack(pv[h], a, b);
+                        const f2_t swp = f2pack(b, a);
+                        X[base + t] = f2fma(ax, swp, f2fma(a0, pv[h], xv[h]));
+                        z = f2fma(bx, swp, f2fma(b0, pv[h], z));
+                    }
+                    P[base + t] = z;
+                    su[q] = z;
+                }
+            }
+            __syncthreads();
+            cg_laplace<N>(tab.D, su, s1, s2, sg, ne);
             __syncthreads();
 #pragma unroll 4
             for (int t = threadIdx.x; t < total; t += blockDim.x) {
-                const int le = t / NN;
-                const int node = t - le * NN;
-                const long long flat = (long long)(e0 + le) * NN + node;
-                const float ms = __ldg(m.massf + flat);
-                const float mv = ms * __ldg(pot + flat);
+                const int q = t + t / NN * (ES - NN);
+                const float ms = sg[q].w;
+                const float mv = ms * __ldg(pot + base + t);
                 float u0, u1, l0, l1;
-                f2unpack(su[le * ES + node], u0, u1);
-                f2unpack(s1[le * ES + node], l0, l1);
+                f2unpack(su[q], u0, u1);
+                f2unpack(s1[q], l0, l1);
                 const float q0 = ms * u0 + alpha * (l1 + mv * u1);
                 const float q1 = alpha * (l0 + mv * u0) - ms * u1;
                 d0 = fmaf(u0, q0, fmaf(u1, q1, d0));
                 d1 = fmaf(u0, q1, fmaf(-u1, q0, d1));
-                Y[flat] = q0;
-                Y[n + flat] = q1;
+                Y[base + t] = f2pack(q0, q1);
             }
             __syncthreads();
         }
         const float v2[2] = {d0, d1};
-        team_sum<2>(v2, w.partials, slot, gs, tmo, ok, o2);
-        slot ^= 1;
-        if (!ok) return false;
-        if (!cg_step(sc, (float)o2[0], (float)o2[1])) {
+        if (!team_sum<TEAM, 2>(v2, tm, o2)) return false;
+        if (!cg_step(sc, o2[0], o2[1])) {
             --it;
             good = false;
             break;
         }
         // ---- Phase B
-        phase_b(false, o3);
-        if (!ok) return false;
-        const float rr = (float)o3[2];
+        if (!phase_b(false, o3)) return false;
+        const float rr = o3[2];
         if (!isfinite(rr)) {
             good = false;
             break;
@@ -457,26 +696,146 @@ __device__ __forceinline__ bool cg_core(unsigned char* smraw, int kmax, const De
         } else if (it - sc.best_it >= CG_STALL) {
             break;
         }
-        if (it < maxit) good = cg_beta(sc, (float)o3[0], (float)o3[1]);
+        if (it < maxit) good = cg_beta(sc, o3[0], o3[1]);
     }
     res.it = it;
     res.usable = good && it > 0;
     // x += a p of the last iteration
     if (res.usable) {
+        const f2_t a0 = f2dup(sc.a0), ax = f2pack(sc.a1, -sc.a1);
         const long long nb = (long long)eb * NN, ne = (long long)ee * NN;
+#pragma unroll 2
         for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
-            const float a = Pv[idx], b = Pv[n + idx];
-            float x0 = fmaf(sc.a0, a, sc.a1 * b), x1 = fmaf(sc.a0, b, -sc.a1 * a);
-            if (it > 1) {
-                x0 += xo[0][idx];
-                x1 += xo[1][idx];
-            }
-            xo[0][idx] = x0;
-            xo[1][idx] = x1;
+            const f2_t pv = P[idx];
+            const f2_t x = it > 1 ? X[idx] : 0ull;
+            float a, b;
+            f2unpack(pv, a, b);
+            X[idx] = f2fma(ax, f2pack(b, a), f2fma(a0, pv, x));
         }
     }
     __syncthreads();
     return true;
+}
+
+// FP64 iterative refinement around cg_core for the block's range of its team's
+// mesh: r = b - A x in FP64 (true residual, continuous format); stop when
+// |r| < scale (tol |r0| + tol) (the reference's criterion, minres.hpp:92; with
+// rel_to_b |b| in the place of |r0|); else solve A d = r to the inner tolerance
+// and add d to x on owner copies.  res.fallback: the inner iteration broke
+// down, stalled or did not halve the true residual, and MINRES should go on
+// from x.  Returns false when a wait timed out.
+struct CgRefine {
+    int sweeps, inner;
+    bool conv, fallback;
+    double rn, r0;
+};
+template <int N, int TEAM>
+__device__ __forceinline__ bool cg_refine(const DevMesh& m, const SolveArgs& a, const KrylovWork<float>& w,
+                                          const MixedArgs& mx, int eb, int ee, unsigned char* smraw, float* lam,
+                                          const EoD<N, double>& et, const CgTab<N>& tab, Team& tm, CgRefine& res)
+{
+    constexpr int NN = N * N;
+    double* sm64 = (double*)smraw;
+    const Fac<double> fac64 = fac_of<double>(m);
+    const double* b0 = (const double*)a.b[0];
+    const double* b1 = (const double*)a.b[1];
+    double* x0 = (double*)a.x[0];
+    double* x1 = (double*)a.x[1];
+    double* const Y0 = mx.Y64[0];
+    double* const Y1 = mx.Y64[1];
+    const long long nb = (long long)eb * NN, ne = (long long)ee * NN;
+    f2_t* const X = (f2_t*)mx.x32[0];
+    res.sweeps = res.inner = 0;
+    res.conv = res.fallback = false;
+    double last_rn = 0.0;
+    for (int l = threadIdx.x; l < N; l += blockDim.x) lam[l] = m.fdmL32[l];
+    for (;;) {
+        const bool applied = res.sweeps > 0 || !a.x_is_zero;
+        if (applied) {
+            __syncthreads();  // the staging area overlays the inner solve's
+            load_dmat_raw<N, double>(sm64, m);
+            __syncthreads();
+            for (int e0 = eb; e0 < ee; e0 += a.kmax64)
+                apply_range<N, double, OP_RES>(
+                    sm64, a.kmax64, &et, fac64, (const double*)a.pot, a.alpha, e0, min(a.kmax64, ee - e0),
+                    [&](int e, int i, int j, long long flat, double* u) {
+                        const long long src = ni_gather_src(m, node_info<N>(m, e, i, j), e, flat);
+                        u[0] = x0[src];
+                        u[1] = x1[src];
+                    },
+                    [&](int, int, int, long long flat, const double* o) {
+                        Y0[flat] = o[0];
+                        Y1[flat] = o[1];
+                    });
+            if (!team_barrier<TEAM>(tm)) return false;
+        }
+        double part = 0.0, partb = 0.0;
+        const bool want_b = res.sweeps == 0 && a.rel_to_b;
+#pragma unroll 2
+        for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
+            const int e = (int)(idx / NN);
+            const int node = (int)(idx - (long long)e * NN);
+            const NodeInfo ni = node_info<N>(m, e, node % N, node / N);
+            const long long src = ni_gather_src(m, ni, e, idx);
+            const double bv0 = b0[src], bv1 = b1[src];
+            double r0 = bv0, r1 = bv1;
+            if (applied) {
+                r0 -= dss_value<N, double, DSS_CONT>(m, Y0, ni, e, idx);
+                r1 -= dss_value<N, double, DSS_CONT>(m, Y1, ni, e, idx);
+            }
+            mx.r64[0][idx] = r0;
+            mx.r64[1][idx] = r1;
+            if (ni_owner(ni)) {
+                part = fma(r0, r0, fma(r1, r1, part));
+                if (want_b) partb = fma(bv0, bv0, fma(bv1, bv1, partb));
+            }
+        }
+        double rr = 0.0, bbv = 0.0;
+        if (!team_sum64<TEAM>(part, partb, tm, rr, bbv)) return false;
+        const double rn = sqrt(rr);
+        if (res.sweeps == 0) res.r0 = a.r0_given > 0.0 ? a.r0_given : want_b ? sqrt(bbv) : rn;
+        res.rn = rn;
+        const double thr = mx.outer_scale * (a.tol * res.r0 + a.tol);
+        res.conv = rn < thr;
+        if (res.conv || res.sweeps >= mx.max_sweeps || res.inner >= a.maxit || !(rn == rn)) return true;
+        if (res.sweeps > 0 && !(rn < 0.5 * last_rn)) {
+            res.fallback = true;
+            return true;
+        }
+        last_rn = rn;
+        // the inner solve reduces by inner_tol, or (last sweep) by CG_MARGIN of
+        // what the outer test still needs: a good initial guess then saves
+        // iterations, not sweeps
+        double itol = mx.inner_tol;
+        if (mx.adaptive) itol = fmax(itol, fmin(CG_MARGIN * thr / rn, 0.5));
+        const double inv = 1.0 / rn;
+        const double* r64a = mx.r64[0];
+        const double* r64b = mx.r64[1];
+        CgOut cr{};
+        if (!cg_core<N, TEAM>(smraw, a.kmax, m, tab, mx.fac4, mx.nnw, mx.pot32, (float)a.alpha, eb, ee, w, tm,
+                              [&](long long flat) {
+                                  return f2pack((float)(r64a[flat] * inv), (float)(r64b[flat] * inv));
+                              },
+                              X, min(mx.inner_maxit, a.maxit - res.inner), (float)itol, lam, cr))
+            return false;
+        res.inner += cr.it;
+        ++res.sweeps;
+        if (cr.usable) {  // x += d
+#pragma unroll 4
+            for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
+                if (!(__ldg(mx.nnw + idx) > 0.f)) continue;
+                float d0, d1;
+                f2unpack(X[idx], d0, d1);
+                x0[idx] += (double)d0 * rn;
+                x1[idx] += (double)d1 * rn;
+            }
+        }
+        if (!team_barrier<TEAM>(tm)) return false;
+        if (!(cr.usable && cr.conv) && res.inner < a.maxit) {
+            res.fallback = true;
+            return true;
+        }
+    }
 }
 
 }  // namespace semgb

@@ -211,7 +211,7 @@ static int grid_1d(long long n) { return (int)std::min<long long>((n + 255) / 25
 
 // dynamic shared memory a persistent solver block may use for staging
 static const size_t kSolverSmemBudget = 160 * 1024;
-static const size_t kCgSmemBudget = 2 * 108 * 1024;
+static const size_t kCgSmemBudget = 222 * 1024;
 static const size_t kK64SmemBudget = 224 * 1024;
 // all-reduce words of the FP64 solvers: two sets of at most 160 lines
 static const size_t kSlotWords = 2 * 160 * RESIDENT_SLOT_STRIDE;
@@ -344,6 +344,7 @@ struct sem_ctx {
     std::vector<double> Drow_host;         // D row-major (DevMesh::Dh)
     std::vector<double> S_host;            // preconditioner basis row-major (DevMesh::Sh)
     unsigned res_epoch = 0;                // last epoch on the resident solver's exchange words (0: clear them)
+    bool cg_ready = false;                 // "cg_fac" and "cg_wt" hold the mesh's data
     unsigned kr_epoch = 0;                 // the same for the FP64 solvers' reduction words
     std::vector<double> coords;            // [n_nodes][2]
     std::vector<int> elements;             // [E][4]
@@ -1489,7 +1490,7 @@ static int run_mixed(sem_ctx* c, int op, const double* pot, double alpha, double
         SEM_CUDA(cudaGetLastError());
         mx.pinv32 = pinv;
     }
-    int grid = 0, kmax = 1, rst = 0;
+    int grid = 0, kmax = 1, kmax64 = 0, rst = 0;
     size_t smem = 0;
     bool resident = false;
     if (mx.fdm && c->resident)
@@ -1535,13 +1536,29 @@ static int run_mixed(sem_ctx* c, int op, const double* pot, double alpha, double
             }
         } else {
             dispatch_n(c->N, [&](auto nv) {
-                grid = solver_plan<decltype(nv)::value>(op, mx.fdm ? SOLVE_MIXED_FDM : SOLVE_MIXED, c->E, c->sms,
-                                                        mx.fdm ? kCgSmemBudget : kSolverSmemBudget, &kmax, &smem);
+                const int kind = mx.minres ? SOLVE_MINRES_FDM : mx.fdm ? SOLVE_MIXED_FDM : SOLVE_MIXED;
+                grid = solver_plan<decltype(nv)::value>(op, kind, c->E, c->sms,
+                                                        kind == SOLVE_MIXED_FDM ? kCgSmemBudget : kSolverSmemBudget,
+                                                        &kmax, &kmax64, &smem);
                 return cudaSuccess;
             });
             if (grid <= 0) return fail(SEM_ERR_CUDA, "could not size the cooperative grid");
+            if (mx.fdm && !mx.minres && !mx.fac4) {  // per-node data of the streaming form, once per context
+                void* fac = nullptr;
+                float* wt = nullptr;
+                if ((s = wsbuf(c, "cg_fac", sizeof(float4) * c->n, &fac)) || (s = wsget(c, "cg_wt", c->n, &wt)))
+                    return s;
+                if (!c->cg_ready)
+                    SEM_LAUNCH(dispatch_n(c->N, [&](auto nv) {
+                        return launch_cg_prep<decltype(nv)::value>(c->dm, fac, wt, c->stream);
+                    }));
+                c->cg_ready = true;
+                mx.fac4 = (const float4*)fac;
+                mx.nnw = wt;
+            }
         }
         a.kmax = kmax;
+        a.kmax64 = kmax64;
         SEM_CUDA(cudaMemsetAsync(sync, 0, sizeof(GridSync), c->stream));
         SEM_CUDA(cudaMemsetAsync(out, 0, sizeof(SolveOut), c->stream));
         if (c->profile) SEM_CUDA(cudaEventRecord(c->ev[0], c->stream));
@@ -1566,11 +1583,10 @@ static int run_mixed(sem_ctx* c, int op, const double* pot, double alpha, double
         c->stats.fp64_applies += c->h_out->sweeps + 1;
         res->n_iter += done_it;
         *sweeps = c->h_out->sweeps + done_sweeps;
-        if (!resident) return SEM_OK;
-        c->res_epoch = c->h_out->epoch;
+        if (resident) c->res_epoch = c->h_out->epoch;
         if (!c->h_out->fallback) return SEM_OK;
-        // the resident iteration broke down, stalled or did not help: go on
-        // from its solution on the staged kernel, MINRES only
+        // the conjugate gradient iteration broke down, stalled or did not help: go on
+        // from its solution on the staged kernel with MINRES
         done_it = res->n_iter;
         done_sweeps = *sweeps;
         resident = false;
@@ -1598,15 +1614,15 @@ static int run_krylov(sem_ctx* c, int op, const double* pot, double alpha, doubl
     SolveOut* out = nullptr;
     int s = krylov_work(c, nc, &w, &sync, &out);
     if (s) return s;
-    int grid = 0, kmax = 1;
+    int grid = 0, kmax = 1, kmax64 = 0;
     size_t smem = 0;
     int resident = 1;
     dispatch_n(c->N, [&](auto nv) {
         constexpr int NV = decltype(nv)::value;
-        grid = solver_plan<NV>(op, SOLVE_FP64_RES, c->E, c->sms, kK64SmemBudget, &kmax, &smem);
+        grid = solver_plan<NV>(op, SOLVE_FP64_RES, c->E, c->sms, kK64SmemBudget, &kmax, &kmax64, &smem);
         if (grid <= 0) {
             resident = 0;
-            grid = solver_plan<NV>(op, SOLVE_FP64, c->E, c->sms, kK64SmemBudget, &kmax, &smem);
+            grid = solver_plan<NV>(op, SOLVE_FP64, c->E, c->sms, kK64SmemBudget, &kmax, &kmax64, &smem);
         }
         return cudaSuccess;
     });

@@ -125,7 +125,7 @@ struct SolveOut {
     int status;      // 0 or SEM_ERR_DEVICE_WAIT
     int inner_iters; // mixed mode: total FP32 iterations
     int sweeps;      // mixed mode: refinement sweeps
-    int fallback;    // resident kernel: the inner solver gave up, continue with MINRES
+    int fallback;    // element-preconditioned kernels: the inner solver gave up, continue with MINRES
     unsigned epoch;  // resident and FP64 kernels: last epoch used on the exchange words
     double r0;       // mixed mode: the norm the stopping test is relative to
 };
@@ -154,6 +154,7 @@ struct SolveArgs {
     double tol;
     int x_is_zero;
     int kmax;         // elements staged per pass (solver_plan)
+    int kmax64;       // mixed solvers: elements per pass of the FP64 residual
     int resident;     // FP64 solvers: the vectors stay in shared memory (SOLVE_FP64_RES)
     int rel_to_b;     // mixed solver: stop on |r| < tol |b| + tol instead of tol |r_0| + tol
                       // (the same test when x_0 = 0; used with warm starts)
@@ -175,7 +176,9 @@ struct MixedArgs {
     const float* pot32;  // FP32 copy of the potential (V or c)
     const float* pinv32; // diagonal preconditioner P^-1 (continuous format), or null
     int fdm;             // element fast-diagonalisation preconditioner (Res only; uses KrylovWork::Z)
-    int minres;          // with fdm: MINRES from the first sweep on
+    int minres;          // with fdm: MINRES (the conjugate gradients gave up)
+    const float4* fac4;  // fdm: per-node factors {g11, -g12, g22, mass} and signed weights (k_cg_prep)
+    const float* nnw;
     int fused;           // inner solve with the single-barrier MINRES iteration (Res only)
     double outer_scale;  // refinement stops at |r| < outer_scale * (tol |r0| + tol)
     int adaptive;        // inner tolerance of a sweep no tighter than the outer test needs
@@ -261,9 +264,12 @@ cudaError_t launch_learn(const DevMesh& m, const LearnArgs& a, cudaStream_t st);
 // launch_solver runs MINRES (op OP_RES/OP_HELM), PCG (OP_LAPLACE) or, when
 // mx is given, the mixed-precision refinement.  work points to a
 // KrylovWork<double> (FP64 solvers) or KrylovWork<float> (mixed).
-enum SolveKind : int { SOLVE_FP64 = 0, SOLVE_MIXED = 1, SOLVE_MIXED_FDM = 2, SOLVE_FP64_RES = 3 };
+enum SolveKind : int { SOLVE_FP64 = 0, SOLVE_MIXED = 1, SOLVE_MIXED_FDM = 2, SOLVE_FP64_RES = 3, SOLVE_MINRES_FDM = 4 };
 template <int N>
-int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax, size_t* smem);
+int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax, int* kmax64, size_t* smem);
+// per-node data of the streaming element-preconditioned solver: fac n float4, wt n floats
+template <int N>
+cudaError_t launch_cg_prep(const DevMesh& m, void* fac, float* wt, cudaStream_t st);
 template <int N>
 cudaError_t launch_solver(const DevMesh& m, const SolveArgs& a, const void* work, const MixedArgs* mx,
                           int grid, size_t smem, cudaStream_t st);

@@ -791,7 +791,8 @@ cudaError_t launch_learn(const DevMesh& m, const LearnArgs& a, cudaStream_t st)
                                             const ZList&, double*, cudaStream_t);                    \
     template cudaError_t launch_update<NV>(const DevMesh&, const double*, const ZList&, double*,     \
                                            cudaStream_t);                                            \
-    template int solver_plan<NV>(int, int, int, int, size_t, int*, size_t*);                         \
+    template int solver_plan<NV>(int, int, int, int, size_t, int*, int*, size_t*);                   \
+    template cudaError_t launch_cg_prep<NV>(const DevMesh&, void*, float*, cudaStream_t);            \
     template cudaError_t launch_learn<NV>(const DevMesh&, const LearnArgs&, cudaStream_t);           \
     template cudaError_t launch_solver<NV>(const DevMesh&, const SolveArgs&, const void*,            \
                                            const MixedArgs*, int, size_t, cudaStream_t);             \

@@ -11,6 +11,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <limits>
 
@@ -718,11 +719,8 @@ __device__ __forceinline__ bool minres_core_fused(T* sm, int kmax, double* red, 
 // whole instance (a.sync == nullptr: block barriers and block reductions).
 // Returns false when a wait timed out.  `leader` writes a.out.
 //
-// With the element preconditioner (FDM kinds) the inner solver is the
-// complex-symmetric conjugate gradient iteration of cg_core, whose
-// correction is taken when it is finite; when it breaks down, stalls or fails
-// to halve the true residual, the remaining sweeps use the preconditioned
-// MINRES, which cannot break down.
+// The element-preconditioned stage solves run on cg_refine (sem_cg.cuh); here
+// their preconditioned MINRES takes over when that iteration gives up.
 enum MixedKind : int {
     MIXED_PLAIN = 0,  // no or diagonal preconditioner
     MIXED_BATCH = 1,  // batched instances: no preconditioner or the element one
@@ -733,7 +731,7 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
                                             const MixedArgs& mx, int eb, int ee, bool leader,
                                             unsigned char* smraw, double* red, MinresScal<float>& sc,
                                             double* sweep_state, float* fdmS, float* fdmL,
-                                            const EoD<N, double>& et, const CgTab<N>* tab = nullptr)
+                                            const EoD<N, double>& et)
 {
     static_assert(KIND == MIXED_PLAIN || OP == OP_RES, "the element preconditioner is the stage operator's");
     constexpr int NN = N * N;
@@ -750,8 +748,6 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
     bool ok = true;
     int sweep = 0, inner_total = 0;
     bool conv = false;
-    bool cg = KIND != MIXED_PLAIN && mx.fdm && !mx.minres;  // the same on every thread
-    double last_rn = 0.0;
     for (;;) {
         // ---- FP64 residual r = unmask(b) - DSS(A_local(unmask(x)))
         const bool applied = (sweep > 0) || !a.x_is_zero;
@@ -759,9 +755,9 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
             __syncthreads();  // the staging area overlays the inner solve's
             load_dmat_raw<N, double>(sm64, m);
             __syncthreads();
-            for (int e0 = eb; e0 < ee; e0 += kmax)
+            for (int e0 = eb; e0 < ee; e0 += a.kmax64)
                 apply_range<N, double, OP>(
-                    sm64, kmax, &et, fac64, pot64, a.alpha, e0, min(kmax, ee - e0),
+                    sm64, a.kmax64, &et, fac64, pot64, a.alpha, e0, min(a.kmax64, ee - e0),
                     [&](int e, int i, int j, long long flat, double* u) {
                         const long long src = ni_gather_src(m, node_info<N>(m, e, i, j), e, flat);
 #pragma unroll
@@ -821,40 +817,9 @@ __device__ __forceinline__ bool mixed_solve(const DevMesh& m, const SolveArgs& a
         double itol = mx.inner_tol;
         if (mx.adaptive) {
             const double need = mx.outer_scale * (a.tol * sweep_state[0] + a.tol) / sweep_state[1];
-            itol = fmax(itol, fmin((cg ? CG_MARGIN : 0.3) * need, 0.5));
+            itol = fmax(itol, fmin(0.3 * need, 0.5));
         }
-        if constexpr (KIND != MIXED_PLAIN) {
-            const double rn = sweep_state[1];
-            if (cg && sweep > 0 && !(rn < 0.5 * last_rn)) cg = false;
-            last_rn = rn;
-            if (mx.fdm) {
-                load_fdm_basis<N, float>(fdmS, fdmL, m);
-                __syncthreads();
-            }
-            if (cg) {
-                const double inv = 1.0 / rn;
-                CgOut cr{};
-                if (!cg_core<N>(smraw, kmax, m, *tab, mx.pot32, (float)a.alpha, eb, ee, w, a.sync, a.timeout_ns, slot,
-                                [&](long long flat, int c) -> float { return (float)(r64c[c][flat] * inv); }, mx.x32,
-                                budget, (float)itol, fdmL, cr))
-                    return false;
-                inner_total += cr.it;
-                ++sweep;
-                if (cr.usable) {  // x += d (FP64, owner copies)
-#pragma unroll 4
-                    for (long long idx = nb + threadIdx.x; idx < ne; idx += blockDim.x) {
-                        const int e = (int)(idx / NN);
-                        const int node = (int)(idx - (long long)e * NN);
-                        if (!ni_owner(node_info<N>(m, e, node % N, node / N))) continue;
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) xp[c][idx] += (double)mx.x32[c][idx] * rn;
-                    }
-                }
-                cg = cr.usable && cr.conv;
-                if (!grid_barrier(a.sync, a.timeout_ns)) return false;
-                continue;
-            }
-        }
+        if (KIND != MIXED_PLAIN && mx.fdm) load_fdm_basis<N, float>(fdmS, fdmL, m);
         load_dmat_raw<N, float>(sm32, m);
         __syncthreads();
         auto rhs = [&](const NodeInfo&, int, long long flat, int c) -> float { return (float)r64c[c][flat]; };
@@ -927,12 +892,10 @@ __global__ void __launch_bounds__(SOLVER_TPB, 1)
                                     nullptr, et);
 }
 
-// the same with the element preconditioner
-constexpr int CG_TPB = 256;
+// the element-preconditioned MINRES (after the conjugate gradients gave up)
 template <int N>
-__global__ void __launch_bounds__(CG_TPB, 2)
-    k_cg_mixed(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ EoD<N, double> et,
-               const __grid_constant__ CgTab<N> tab)
+__global__ void __launch_bounds__(SOLVER_TPB, 1)
+    k_minres_fdm(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ EoD<N, double> et)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[34];
@@ -942,7 +905,37 @@ __global__ void __launch_bounds__(CG_TPB, 2)
     int eb, ee;
     block_range(m.E, eb, ee);
     mixed_solve<N, OP_RES, MIXED_FDM>(m, a, w, mx, eb, ee, blockIdx.x == 0, smraw, red, sc, sweep_state, fdmS, fdmL,
-                                      et, &tab);
+                                      et);
+}
+
+// the element-preconditioned stage solve (streaming form)
+// Threads and blocks per SM: measured per iteration at 192x192, 100x100 and
+// 64x64, p = 8: 269, 83, 57 us; 128 x 5: 290, 102, 91; 256 x 3 (80 registers,
+// spills): 247, 94, 67; before the vectors were interleaved as pairs and the
+// factors packed in 16 bytes (then 209, 55, 38)
+constexpr int CG_TPB = 256, CG_BLOCKS = 2;
+template <int N>
+__global__ void __launch_bounds__(CG_TPB, CG_BLOCKS)
+    k_cg_mixed(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ EoD<N, double> et,
+               const __grid_constant__ CgTab<N> tab)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ float lam[N];
+    int eb, ee;
+    block_range(m.E, eb, ee);
+    Team tm{a.sync, a.timeout_ns, w.partials, 0, (int)blockIdx.x, (int)gridDim.x};
+    CgRefine r{};
+    if (!cg_refine<N, TEAM_GRID>(m, a, w, mx, eb, ee, smraw, lam, et, tab, tm, r)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.out->success = r.conv ? 1 : 0;
+        a.out->n_iter = r.inner;
+        a.out->residual = r.rn;
+        a.out->status = 0;
+        a.out->inner_iters = r.inner;
+        a.out->sweeps = r.sweeps;
+        a.out->fallback = r.fallback ? 1 : 0;
+        a.out->r0 = r.r0;
+    }
 }
 
 // ------------------------------------------------------------- launchers
@@ -957,16 +950,15 @@ size_t solver_smem(int op, int kind, int kmax)
                : op == OP_HELM ? k64_smem_bytes<N, OP_HELM>(kmax, r)
                                : k64_smem_bytes<N, OP_LAPLACE>(kmax, r);
     }
-    const bool two = (op == OP_RES);
-    const size_t d = two ? range_smem_bytes<N, double, OP_RES>(kmax) : range_smem_bytes<N, double, OP_HELM>(kmax);
-    const size_t c = kind == SOLVE_MIXED_FDM ? cg_smem_bytes<N>(kmax) : 0;
-    return d > c ? d : c;
+    if (kind == SOLVE_MIXED_FDM) return cg_smem_bytes<N>(kmax);
+    return op == OP_RES ? range_smem_bytes<N, double, OP_RES>(kmax) : range_smem_bytes<N, double, OP_HELM>(kmax);
 }
 
 template <int N>
 static const void* solver_fn(int op, int kind)
 {
     if (kind == SOLVE_MIXED_FDM) return (const void*)k_cg_mixed<N>;
+    if (kind == SOLVE_MINRES_FDM) return (const void*)k_minres_fdm<N>;
     if (kind == SOLVE_MIXED)
         return op == OP_RES ? (const void*)k_minres_mixed<N, OP_RES> : (const void*)k_minres_mixed<N, OP_HELM>;
     if (kind == SOLVE_FP64_RES)
@@ -988,30 +980,52 @@ inline int k64_threads(int N, int nc, int share)
     return v >= top ? top : v < 128 ? 128 : (v + 31) / 32 * 32;
 }
 
-// Plan a cooperative launch: one block per SM (fewer for small meshes), two
-// smaller ones for the element-preconditioned kernel on meshes that give each
-// SM several passes, so that one block's loads overlap the other's passes,
-// and the largest staging capacity kmax <= the block's element count that
-// fits in smem_budget bytes per SM.  Returns the grid, or 0 on failure (for
-// SOLVE_FP64_RES also when the block's elements do not fit in one pass).
+// elements of one element-preconditioned pass: one line per thread
 template <int N>
-int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_out, size_t* smem_out)
+constexpr int cg_pass()
+{
+    return CG_TPB / N;
+}
+
+// Plan a cooperative launch: one block per SM (fewer for small meshes), for the
+// element-preconditioned kernel as many of its small blocks per SM as the mesh
+// fills with a pass each (a block alternates between loading a pass and the
+// line contractions behind block barriers, so only other blocks of the SM hide
+// its memory latency), and the largest staging capacities
+// kmax <= the block's element count that fit smem_budget bytes per SM.
+// Returns the grid, or 0 on failure (for SOLVE_FP64_RES also when the block's
+// elements do not fit in one pass).
+template <int N>
+int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_out, int* kmax64_out,
+                size_t* smem_out)
 {
     const bool fdm = kind == SOLVE_MIXED_FDM;
-    int per = 1;
-    if (fdm && (long long)E * N * N >= 4096ll * sms) per = 2;
     const bool f64 = kind == SOLVE_FP64 || kind == SOLVE_FP64_RES;
+    int per = 1;
+    if (fdm) {
+        per = E / (sms * cg_pass<N>());
+        per = per < 1 ? 1 : per > CG_BLOCKS ? CG_BLOCKS : per;
+        smem_budget = smem_budget / CG_BLOCKS;
+    }
     if (f64 && sms > 32 * K64_MAXQ) sms = 32 * K64_MAXQ;
     int grid = E < per * sms ? E : per * sms;
     if (grid < 1) grid = 1;
     int kmax = (E + grid - 1) / grid;
     const int share = kmax;
     if (kind == SOLVE_FP64_RES && solver_smem<N>(op, kind, kmax) > smem_budget) return 0;  // does not fit
-    while (kmax > 1 && solver_smem<N>(op, kind, kmax) > smem_budget / per)
-        kmax = kind != SOLVE_MIXED ? kmax - 1 : (kmax + 1) / 2;
-    if (kind != SOLVE_MIXED)  // even passes
+    if (fdm && kmax > cg_pass<N>()) kmax = cg_pass<N>();
+    while (kmax > 1 && solver_smem<N>(op, kind, kmax) > smem_budget)
+        kmax = fdm || f64 ? kmax - 1 : (kmax + 1) / 2;
+    if (fdm || f64)  // even passes
         kmax = (share + (share + kmax - 1) / kmax - 1) / ((share + kmax - 1) / kmax);
-    const size_t smem = solver_smem<N>(op, kind, kmax);
+    size_t smem = solver_smem<N>(op, kind, kmax);
+    int kmax64 = kmax;
+    if (fdm) {
+        while (kmax64 > 1 && range_smem_bytes<N, double, OP_RES>(kmax64) > (smem > smem_budget ? smem : smem_budget))
+            --kmax64;
+        const size_t s64 = range_smem_bytes<N, double, OP_RES>(kmax64);
+        if (s64 > smem) smem = s64;
+    }
     const void* fn = solver_fn<N>(op, kind);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
     int per_sm = 0;
@@ -1019,10 +1033,21 @@ int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_
                                                       smem) != cudaSuccess ||
         per_sm < 1)
         return 0;
-    if (grid > per_sm * sms) grid = per_sm * sms;
+    if (grid > per_sm * sms) {  // fewer blocks per SM: the passes cover the rest
+        grid = per_sm * sms;
+    }
     *kmax_out = kmax;
+    *kmax64_out = kmax64;
     *smem_out = smem;
     return grid;
+}
+
+template <int N>
+cudaError_t launch_cg_prep(const DevMesh& m, void* fac, float* wt, cudaStream_t st)
+{
+    const int grid = (int)std::min<long long>((m.n + 255) / 256, 152 * 32);
+    k_cg_prep<N><<<grid, 256, 0, st>>>(m, (float4*)fac, wt);
+    return cudaGetLastError();
 }
 
 template <int N>
@@ -1031,7 +1056,10 @@ cudaError_t launch_solver(const DevMesh& m, const SolveArgs& a, const void* work
 {
     DevMesh mm = m;
     SolveArgs aa = a;
-    const int kind = !mx ? (a.resident ? SOLVE_FP64_RES : SOLVE_FP64) : mx->fdm ? SOLVE_MIXED_FDM : SOLVE_MIXED;
+    const int kind = !mx          ? (a.resident ? SOLVE_FP64_RES : SOLVE_FP64)
+                     : mx->minres ? SOLVE_MINRES_FDM
+                     : mx->fdm    ? SOLVE_MIXED_FDM
+                                  : SOLVE_MIXED;
     const void* fn = solver_fn<N>(a.op, kind);
     if (!m.Dh || !m.Sh) return cudaErrorInvalidValue;
     EoD<N, double> et = eo_d_table<N, double>(m.Dh);
