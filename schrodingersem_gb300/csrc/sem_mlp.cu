@@ -42,6 +42,7 @@ struct GemmArgs {
     int ldc;
     const float* bias;     // optional, length N
     int relu;              // ReLU epilogue
+    const float* mask;     // optional, like C: 0 where the mask is not positive (ReLU backward)
     int accumulate;        // C += result
     __nv_bfloat16* Cbf;    // optional BF16 copy of the output
 };
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g)
                     if (g.accumulate) v += g.C[(long long)m * g.ldc + nn];
                     if (g.bias) v += g.bias[nn];
                     if (g.relu) v = fmaxf(v, 0.f);
+                    if (g.mask && !(g.mask[(long long)m * g.ldc + nn] > 0.f)) v = 0.f;
                     g.C[(long long)m * g.ldc + nn] = v;
                     if (g.Cbf) g.Cbf[(long long)m * g.ldc + nn] = __float2bfloat16(v);
                 }
@@ -221,41 +223,89 @@ __device__ __forceinline__ void tc_chunk(const void* X, int bf, long long base, 
     }
 }
 
-template <int BN>
-__device__ __forceinline__ void tc_stage(const GemmArgs& g, unsigned char* sA, unsigned char* sB, int m0, int n0,
-                                         int k0)
+// One operand of a K tile, rows [row0, row0 + R) x [k0, k0 + TC_BK), in two
+// steps so that the loads of a tile are in flight while the one before it is
+// multiplied: load brings this thread's share into registers as BF16 pairs,
+// store writes it to the staged layout.  Zero past the matrix edges.
+//  - K contiguous (sk == 1): 16-byte chunks, 8 consecutive k of one row.
+//  - rows contiguous (the transposed operands of the weight gradients): a thread
+//    takes 8 rows x 8 k, one vector load per k over 8 consecutive rows, and
+//    transposes the block in registers; it stores its rows starting from its
+//    lane's so that the eight lanes of a store phase hit different banks.
+//    (Chunks along k cost 8 scalar loads each, uncoalesced: 150 us for a
+//    1024-row gradient GEMM.)
+template <int R>
+__device__ __forceinline__ void tc_load(const void* X, int bf, long long sr, long long sk, int rows, int K, int row0,
+                                        int k0, uint32_t (&w)[8][4])
 {
-    // 16-byte chunks: 8 consecutive k of one row; every thread issues all of
-    // its chunks' loads before its shared-memory stores
-    constexpr int NQ = ((TC_M + BN) * (TC_BK / 8) + TC_THREADS - 1) / TC_THREADS;
-    uint32_t w[NQ][4];
+    if (sr == 1 && sk != 1) {
+        const int mb = threadIdx.x % (R / 8), kb = threadIdx.x / (R / 8);
+        const int r = row0 + mb * 8, nr = min(8, rows - r);
 #pragma unroll
-    for (int i = 0; i < NQ; ++i) {
-        const int q = threadIdx.x + i * TC_THREADS;
-        const bool isA = q < TC_M * (TC_BK / 8);
-        const int qq = isA ? q : q - TC_M * (TC_BK / 8);
-        const int r = qq >> 3, kc = qq & 7;
-        const int k = k0 + kc * 8;
-        const int row = (isA ? m0 : n0) + r;
-        const bool in = isA ? (row < g.M) : (row < g.N);
-        const int kvalid = in ? min(8, g.K - k) : 0;
-        if (kvalid <= 0) {
-            w[i][0] = w[i][1] = w[i][2] = w[i][3] = 0u;
-            continue;
+        for (int q = 0; q < 8; ++q) {
+            const int k = k0 + kb * 8 + q;
+            const int valid = (kb < TC_BK / 8 && k < K) ? nr : 0;
+            if (valid <= 0) {
+                w[q][0] = w[q][1] = w[q][2] = w[q][3] = 0u;
+            } else if (!bf && valid >= 8 && (((uintptr_t)((const float*)X + r + (long long)k * sk)) & 15) == 8) {
+                const float2* p = (const float2*)((const float*)X + r + (long long)k * sk);  // 8-byte aligned rows
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const float2 v = __ldg(p + h);
+                    w[q][h] = pack_bf16(__float2bfloat16(v.x), __float2bfloat16(v.y));
+                }
+            } else {
+                tc_chunk(X, bf, r + (long long)k * sk, 1, valid, w[q]);
+            }
         }
-        if (isA)
-            tc_chunk(g.A, g.a_bf16, (long long)row * g.sa_m + (long long)k * g.sa_k, g.sa_k, kvalid, w[i]);
-        else
-            tc_chunk(g.B, g.b_bf16, (long long)k * g.sb_k + (long long)row * g.sb_n, g.sb_k, kvalid, w[i]);
+        return;
     }
 #pragma unroll
-    for (int i = 0; i < NQ; ++i) {
+    for (int i = 0; i < R / 16; ++i) {
         const int q = threadIdx.x + i * TC_THREADS;
-        const bool isA = q < TC_M * (TC_BK / 8);
-        const int qq = isA ? q : q - TC_M * (TC_BK / 8);
-        const int r = qq >> 3, kc = qq & 7;
-        unsigned char* dst = (isA ? sA + tc_off(TC_M, r, kc * 8) : sB + tc_off(BN, r, kc * 8));
-        *(uint4*)dst = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+        const int r = q >> 3, k = k0 + (q & 7) * 8;
+        const int kvalid = row0 + r < rows ? min(8, K - k) : 0;
+        if (kvalid <= 0)
+            w[i][0] = w[i][1] = w[i][2] = w[i][3] = 0u;
+        else
+            tc_chunk(X, bf, (long long)(row0 + r) * sr + (long long)k * sk, sk, kvalid, w[i]);
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void tc_store(long long sr, long long sk, unsigned char* dst, uint32_t (&w)[8][4])
+{
+    if (sr == 1 && sk != 1) {
+        const int mb = threadIdx.x % (R / 8), kb = threadIdx.x / (R / 8);
+        if (kb >= TC_BK / 8) return;
+        uint32_t t[8][4];  // row j: k pairs
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+                t[j][h] = __byte_perm(w[2 * h][j >> 1], w[2 * h + 1][j >> 1], (j & 1) ? 0x7632 : 0x5410);
+        const int rot = threadIdx.x & 7;  // t[j] := row (j + rot) & 7
+#pragma unroll
+        for (int s = 1; s < 8; s <<= 1) {
+            uint32_t u[8][4];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int h = 0; h < 4; ++h) u[j][h] = (rot & s) ? t[(j + s) & 7][h] : t[j][h];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int h = 0; h < 4; ++h) t[j][h] = u[j][h];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            *(uint4*)(dst + tc_off(R, mb * 8 + ((j + rot) & 7), kb * 8)) = make_uint4(t[j][0], t[j][1], t[j][2], t[j][3]);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < R / 16; ++i) {
+        const int q = threadIdx.x + i * TC_THREADS;
+        *(uint4*)(dst + tc_off(R, q >> 3, (q & 7) * 8)) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
     }
 }
 
@@ -290,6 +340,9 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
     const int nk = (g.K + TC_BK - 1) / TC_BK;
     bool ok = true;
     int issued = 0;  // K chunks whose MMAs thread 0 has committed
+    uint32_t wa[8][4], wb[8][4];
+    tc_load<TC_M>(g.A, g.a_bf16, g.sa_m, g.sa_k, g.M, g.K, m0, 0, wa);
+    tc_load<BN>(g.B, g.b_bf16, g.sb_n, g.sb_k, g.N, g.K, n0, 0, wb);
     for (int kt = 0; kt < nk && ok; ++kt) {
         const int b = kt & 1;
         if (kt >= 2) ok = mbar_wait(&bar[b], (uint32_t)(((kt - 2) >> 1) & 1), timeout_ns);
@@ -297,7 +350,12 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
             ok = false;
             break;
         }
-        tc_stage<BN>(g, sA(b), sB(b), m0, n0, kt * TC_BK);
+        tc_store<TC_M>(g.sa_m, g.sa_k, sA(b), wa);
+        tc_store<BN>(g.sb_n, g.sb_k, sB(b), wb);
+        if (kt + 1 < nk) {
+            tc_load<TC_M>(g.A, g.a_bf16, g.sa_m, g.sa_k, g.M, g.K, m0, (kt + 1) * TC_BK, wa);
+            tc_load<BN>(g.B, g.b_bf16, g.sb_n, g.sb_k, g.N, g.K, n0, (kt + 1) * TC_BK, wb);
+        }
         fence_proxy_async_smem();  // the staged tile is read by the tensor cores (async proxy)
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -341,12 +399,13 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
                 // every load of the chunk (bias, accumulated C) before its
                 // first store: the stores may alias them as far as the
                 // compiler knows, which would serialise load after store
-                float cin[16], bin[16];
+                float cin[16], bin[16], min_[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     const int nn = n0 + c0 + j;
                     const bool in = nn < g.N;
                     cin[j] = (in && g.accumulate) ? g.C[(long long)m * g.ldc + nn] : 0.f;
+                    min_[j] = (in && g.mask) ? __ldg(g.mask + (long long)m * g.ldc + nn) : 1.f;
                     bin[j] = (in && g.bias) ? __ldg(g.bias + nn) : 0.f;
                 }
 #pragma unroll
@@ -357,6 +416,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
                     if (g.accumulate) v += cin[j];
                     if (g.bias) v += bin[j];
                     if (g.relu) v = fmaxf(v, 0.f);
+                    if (!(min_[j] > 0.f)) v = 0.f;
                     g.C[(long long)m * g.ldc + nn] = v;
                     if (g.Cbf) g.Cbf[(long long)m * g.ldc + nn] = __float2bfloat16(v);
                 }
@@ -389,71 +449,66 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
 // rounding points and MMA shapes as the per-layer GEMMs (M = 128, K = 16
 // steps in order), so the results agree with them.  Shapes: H <= 256 and
 // H, d_out <= 256; otherwise the per-layer GEMMs run.
-constexpr int MF_BUF = 48 * 1024;  // one staging buffer: A chunk (16 KB) + B chunk (<= 32 KB)
-constexpr int MF_H = 64 * 1024;    // hidden activations, 128 rows x 256 K BF16
-constexpr size_t MF_SMEM = 2 * (size_t)MF_BUF + MF_H;
+//
+// The weights come as packed images (k_pack_weights): per 64-wide K chunk the
+// staged operand itself, so one thread brings a chunk with one bulk copy, three
+// chunks in flight; only the features are staged by threads, their loads one
+// chunk ahead.  Staging every chunk through registers, four 16-byte loads at a
+// time, took 90 us for 4,096 rows (14 chunks of 6 us on 32 SMs).
+constexpr int MF_NB = 3;             // weight chunks in flight
+constexpr int MF_BB = 32 * 1024;     // one weight chunk: at most 256 rows x 64 K BF16
+constexpr int MF_AB = 16 * 1024;     // one feature chunk: 128 rows x 64 K BF16
+constexpr int MF_H = 64 * 1024;      // hidden activations, 128 rows x 256 K BF16
+constexpr size_t MF_SMEM = MF_NB * (size_t)MF_BB + 2 * (size_t)MF_AB + MF_H;
+static_assert(MF_SMEM >= 128 * 256 * sizeof(float), "the output tile overlays the staging buffers");
 
 struct MlpArgs {
     int rows, d_in, H, d_out;
     const __nv_bfloat16* x;       // rows x d_in
-    const __nv_bfloat16* WT[3];   // [out][in]
+    const unsigned char* img[3];  // packed weight chunks
     const float* b[3];
     float* out;                   // rows x d_out
 };
 
-__device__ __forceinline__ int mf_round16(int n) { return (n + 15) & ~15; }
+__host__ __device__ __forceinline__ int mf_round16(int n) { return (n + 15) & ~15; }
 
-// stage K chunk k0 of layer l: B rows [0, nrows_pad) of WT (rows >= n are
-// zero), and for layer 1 the A rows of the CTA's x tile
-__device__ __forceinline__ void mf_stage(const MlpArgs& a, int l, int m0, int k0, unsigned char* buf)
+// img: per K chunk of 64 the canonical layout of rows n (padded to 16 with
+// zeros) of W^T: element (n, k) of chunk c = W[c*64 + k][n], W row-major [K][N]
+__global__ void k_pack_weights(int K, int N, const __nv_bfloat16* __restrict__ W, unsigned char* __restrict__ img)
 {
-    const int K = l == 0 ? a.d_in : a.H;
-    const int n = l == 2 ? a.d_out : a.H;
-    const int npad = mf_round16(n);
-    const __nv_bfloat16* W = l == 0 ? a.WT[0] : l == 1 ? a.WT[1] : a.WT[2];  // no runtime index into the parameters
-    unsigned char* sA = buf;
-    unsigned char* sB = buf + TC_M * TC_BK * 2;
-    const int nqa = l == 0 ? TC_M * (TC_BK / 8) : 0;
-    const int nq = nqa + npad * (TC_BK / 8);
-    for (int q0 = threadIdx.x; q0 < nq; q0 += 4 * TC_THREADS) {
-        uint32_t w[4][4];
+    const int npad = mf_round16(N), groups = (K + TC_BK - 1) / TC_BK * (TC_BK / 8);
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npad * groups; t += gridDim.x * blockDim.x) {
+        const int kg = t / npad, n = t - kg * npad;
+        uint32_t w[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int q = q0 + u * TC_THREADS;
-            w[u][0] = w[u][1] = w[u][2] = w[u][3] = 0u;
-            if (q >= nq) continue;
-            const bool isA = q < nqa;
-            const int qq = isA ? q : q - nqa;
-            const int r = qq >> 3, kc = qq & 7;
-            const int k = k0 + kc * 8;
-            const int row = isA ? m0 + r : r;
-            const bool in = isA ? row < a.rows : row < n;
-            const int kvalid = in ? min(8, K - k) : 0;
-            if (kvalid <= 0) continue;
-            if (isA)
-                tc_chunk(a.x, 1, (long long)row * a.d_in + k, 1, kvalid, w[u]);
-            else
-                tc_chunk(W, 1, (long long)row * K + k, 1, kvalid, w[u]);
+        for (int h = 0; h < 4; ++h) {
+            const int k = kg * 8 + 2 * h;
+            const __nv_bfloat16 z = __float2bfloat16(0.f);
+            w[h] = pack_bf16(n < N && k < K ? W[(long long)k * N + n] : z, n < N && k + 1 < K ? W[(long long)(k + 1) * N + n] : z);
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int q = q0 + u * TC_THREADS;
-            if (q >= nq) continue;
-            const bool isA = q < nqa;
-            const int qq = isA ? q : q - nqa;
-            const int r = qq >> 3, kc = qq & 7;
-            unsigned char* dst = isA ? sA + tc_off(TC_M, r, kc * 8) : sB + tc_off(npad, r, kc * 8);
-            *(uint4*)dst = make_uint4(w[u][0], w[u][1], w[u][2], w[u][3]);
-        }
+        const int c = kg / (TC_BK / 8), kc = (kg - c * (TC_BK / 8)) * 8;
+        *(uint4*)(img + (size_t)c * npad * TC_BK * 2 + tc_off(npad, n, kc)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
+}
+
+__device__ __forceinline__ void tc_ld16(uint32_t addr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
 }
 
 __global__ void __launch_bounds__(TC_THREADS) k_mlp_fwd(MlpArgs a, long long timeout_ns)
 {
     extern __shared__ __align__(1024) unsigned char msm[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t full[MF_NB], done[MF_NB];  // chunk arrived / its MMAs complete
     __shared__ uint32_t tmem_base;
-    unsigned char* hbuf = msm + 2 * MF_BUF;
+    __shared__ float sbias[3 * 256];
+    unsigned char* abuf = msm + MF_NB * MF_BB;
+    unsigned char* hbuf = abuf + 2 * MF_AB;
     const int m0 = blockIdx.x * TC_M;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0) {
@@ -463,98 +518,136 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_fwd(MlpArgs a, long long tim
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int i = 0; i < MF_NB; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&done[i], 1);
+        }
         mbar_fence_init();
+    }
+    for (int t = threadIdx.x; t < 256; t += TC_THREADS) {
+        sbias[t] = t < a.H ? __ldg(a.b[0] + t) : 0.f;
+        sbias[256 + t] = t < a.H ? __ldg(a.b[1] + t) : 0.f;
+        sbias[512 + t] = t < a.d_out ? __ldg(a.b[2] + t) : 0.f;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = tmem_base;
-    bool ok = true;
-    int g = 0;  // K chunks issued so far (all layers): buffer g & 1
-    const int row = m0 + warp * 32 + lane;
-    for (int l = 0; l < 3 && ok; ++l) {
-        const int K = l == 0 ? a.d_in : a.H;
-        const int n = l == 2 ? a.d_out : a.H;
-        const int npad = mf_round16(n);
-        const uint32_t idesc = tc_idesc(TC_M, npad);
-        const uint32_t acc_col = l == 1 ? 256u : 0u;
-        const int nk = (K + TC_BK - 1) / TC_BK;
-        for (int kt = 0; kt < nk && ok; ++kt, ++g) {
-            const int b = g & 1;
-            unsigned char* buf = msm + (size_t)b * MF_BUF;
-            if (g >= 2) ok = mbar_wait(&bar[b], (uint32_t)(((g - 2) >> 1) & 1), timeout_ns);
-            if (!__syncthreads_and(ok)) {
-                ok = false;
-                break;
-            }
-            mf_stage(a, l, m0, kt * TC_BK, buf);
-            fence_proxy_async_smem();
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t b0 = smem_addr(buf + TC_M * TC_BK * 2);
-                // layer 1: A from the staged chunk; layers 2 and 3: from H
-                const uint32_t a0 = l == 0 ? smem_addr(buf) : smem_addr(hbuf) + (uint32_t)(kt * 4) * (TC_M * 32);
+    const int nk1 = (a.d_in + TC_BK - 1) / TC_BK, nk2 = (a.H + TC_BK - 1) / TC_BK;  // chunks of layer 1; of 2 and 3
+    const int total = nk1 + 2 * nk2;
+    int issued = 0, waited = 0, committed = 0;  // thread 0: bulk copies issued and waited for, chunks committed
+    auto bulk = [&](int g) {  // thread 0: weight chunk g into buffer g % MF_NB
+        const int l = g < nk1 ? 0 : g < nk1 + nk2 ? 1 : 2;
+        const int kt = g - (l == 0 ? 0 : l == 1 ? nk1 : nk1 + nk2);
+        const uint32_t bytes = (uint32_t)mf_round16(l == 2 ? a.d_out : a.H) * TC_BK * 2;
+        const unsigned char* src = (l == 0 ? a.img[0] : l == 1 ? a.img[1] : a.img[2]) + (size_t)kt * bytes;
+        mbar_arrive_tx(&full[g % MF_NB], bytes);
+        bulk_load(msm + (size_t)(g % MF_NB) * MF_BB, src, bytes, &full[g % MF_NB]);
+        issued = g + 1;
+    };
+    // thread 0: the MMAs of chunk g, then the copy that reuses chunk g - 1's buffer
+    auto step = [&](int g, int l, int kt) -> bool {
+        const int K = l == 0 ? a.d_in : a.H, npad = mf_round16(l == 2 ? a.d_out : a.H);
+        if (!mbar_wait(&full[g % MF_NB], (uint32_t)((g / MF_NB) & 1), timeout_ns)) return false;
+        waited = g + 1;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t idesc = tc_idesc(TC_M, npad), acc = taddr + (l == 1 ? 256u : 0u);
+        const uint32_t b0 = smem_addr(msm + (size_t)(g % MF_NB) * MF_BB);
+        // layer 1: A from the staged chunk; layers 2 and 3: from H
+        const uint32_t a0 = l == 0 ? smem_addr(abuf + (kt & 1) * MF_AB) : smem_addr(hbuf) + (uint32_t)(kt * 4) * (TC_M * 32);
 #pragma unroll
-                for (int ks = 0; ks < TC_BK / 16; ++ks) {
-                    if (kt * TC_BK + ks * 16 >= mf_round16(K)) break;
-                    const uint64_t ad = tc_desc(a0 + ks * TC_M * 32, 128, 256);
-                    const uint64_t bd = tc_desc(b0 + ks * npad * 32, 128, 256);
-                    const uint32_t accf = (kt > 0 || ks > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(taddr + acc_col),
-                        "l"(ad), "l"(bd), "r"(idesc), "r"(accf)
-                        : "memory");
-                }
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                        smem_addr(&bar[b]))
-                    : "memory");
-            }
+        for (int ks = 0; ks < TC_BK / 16; ++ks) {
+            if (kt * TC_BK + ks * 16 >= mf_round16(K)) break;
+            const uint64_t ad = tc_desc(a0 + ks * TC_M * 32, 128, 256);
+            const uint64_t bd = tc_desc(b0 + ks * npad * 32, 128, 256);
+            const uint32_t accf = (kt > 0 || ks > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(acc),
+                "l"(ad), "l"(bd), "r"(idesc), "r"(accf)
+                : "memory");
         }
-        if (!ok) break;
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_addr(&done[g % MF_NB]))
+                     : "memory");
+        committed = g + 1;
+        if (g >= 1 && g + 2 < total) {
+            if (!mbar_wait(&done[(g - 1) % MF_NB], (uint32_t)(((g - 1) / MF_NB) & 1), timeout_ns)) return false;
+            bulk(g + 2);
+        }
+        return true;
+    };
+    if (threadIdx.x == 0)
+        for (int g = 0; g < MF_NB && g < total; ++g) bulk(g);
+    bool ok = true;
+    int g = 0;  // chunks so far
+    uint32_t w[8][4];
+    tc_load<TC_M>(a.x, 1, a.d_in, 1, a.rows, a.d_in, m0, 0, w);
+    for (int l = 0; l < 3 && ok; ++l) {
+        const int n = l == 2 ? a.d_out : a.H;
+        const int nk = l == 0 ? nk1 : nk2;
+        if (l == 0) {
+            for (int kt = 0; kt < nk; ++kt) {
+                // the feature buffer's previous chunk (the barrier's next use
+                // is chunk kt + 1, issued after this iteration's block barrier)
+                if (kt >= 2) ok = mbar_wait(&done[(kt - 2) % MF_NB], (uint32_t)(((kt - 2) / MF_NB) & 1), timeout_ns);
+                if (!__syncthreads_and(ok)) {
+                    ok = false;
+                    break;
+                }
+                tc_store<TC_M>(a.d_in, 1, abuf + (kt & 1) * MF_AB, w);
+                if (kt + 1 < nk) tc_load<TC_M>(a.x, 1, a.d_in, 1, a.rows, a.d_in, m0, (kt + 1) * TC_BK, w);
+                fence_proxy_async_smem();
+                __syncthreads();
+                if (threadIdx.x == 0) ok = step(kt, 0, kt);
+            }
+        } else if (threadIdx.x == 0) {
+            for (int kt = 0; kt < nk && ok; ++kt) ok = step(g + kt, l, kt);
+        }
+        if (!__syncthreads_and(ok)) {
+            ok = false;
+            break;
+        }
+        g += nk;
         // the layer's last commit covers every MMA issued before it
-        ok = mbar_wait(&bar[(g - 1) & 1], (uint32_t)(((g - 1) >> 1) & 1), timeout_ns);
+        ok = mbar_wait(&done[(g - 1) % MF_NB], (uint32_t)(((g - 1) / MF_NB) & 1), timeout_ns);
         ok = __syncthreads_and(ok) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (!ok) break;
-        // epilogue: 16 accumulator columns at a time
-        for (int c0 = 0; c0 < n; c0 += 16) {
-            uint32_t r[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                "[%16];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15])
-                : "r"(taddr + acc_col + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0)
-                : "memory");
+        // epilogue: 32 accumulator columns at a time
+        const uint32_t tcol = taddr + (l == 1 ? 256u : 0u) + ((uint32_t)(warp * 32) << 16);
+        const int rl = warp * 32 + lane;
+        const float* bias = sbias + l * 256;
+        float* so = (float*)msm;  // layer 3: the output tile, rows of n (every staging buffer is free)
+        for (int c0 = 0; c0 < n; c0 += 32) {
+            uint32_t r[2][16];
+            tc_ld16(tcol + (uint32_t)c0, r[0]);
+            const bool two = c0 + 16 < n;
+            if (two) tc_ld16(tcol + (uint32_t)c0 + 16u, r[1]);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const float* bias = l == 0 ? a.b[0] : l == 1 ? a.b[1] : a.b[2];
-            float bv[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) bv[j] = (c0 + j < n) ? __ldg(bias + c0 + j) : 0.f;
-            if (l < 2) {
-                // ReLU, BF16, into H at (row - m0, k = c0 + j); columns >= n
-                // (up to the 16-aligned K of the next layer) hold zeros
-                uint32_t pk[8];
+            for (int h = 0; h < 2; ++h) {
+                if (h == 1 && !two) break;
+                const int c = c0 + 16 * h;
+                if (l < 2) {
+                    // ReLU, BF16, into H at (row - m0, k = c + j); columns >= n
+                    // (up to the 16-aligned K of the next layer) hold zeros
+                    uint32_t pk[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const float v0 = (c0 + 2 * j < n) ? fmaxf(__uint_as_float(r[2 * j]) + bv[2 * j], 0.f) : 0.f;
-                    const float v1 =
-                        (c0 + 2 * j + 1 < n) ? fmaxf(__uint_as_float(r[2 * j + 1]) + bv[2 * j + 1], 0.f) : 0.f;
-                    pk[j] = pack_bf16(__float2bfloat16(v0), __float2bfloat16(v1));
+                    for (int j = 0; j < 8; ++j) {
+                        const float v0 = (c + 2 * j < n) ? fmaxf(__uint_as_float(r[h][2 * j]) + bias[c + 2 * j], 0.f) : 0.f;
+                        const float v1 = (c + 2 * j + 1 < n)
+                                             ? fmaxf(__uint_as_float(r[h][2 * j + 1]) + bias[c + 2 * j + 1], 0.f)
+                                             : 0.f;
+                        pk[j] = pack_bf16(__float2bfloat16(v0), __float2bfloat16(v1));
+                    }
+                    *(uint4*)(hbuf + tc_off(TC_M, rl, c)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                    *(uint4*)(hbuf + tc_off(TC_M, rl, c + 8)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (c + j < n) so[rl * n + c + j] = __uint_as_float(r[h][j]) + bias[c + j];
                 }
-                const int rl = warp * 32 + lane;
-                *(uint4*)(hbuf + tc_off(TC_M, rl, c0)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                *(uint4*)(hbuf + tc_off(TC_M, rl, c0 + 8)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            } else if (row < a.rows) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (c0 + j < n) a.out[(long long)row * n + c0 + j] = __uint_as_float(r[j]) + bv[j];
             }
         }
         if (l < 2) {
@@ -564,14 +657,25 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_fwd(MlpArgs a, long long tim
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        } else {
+            // the tile's rows are contiguous in the output
+            __syncthreads();
+            const int nv = min(TC_M, a.rows - m0) * n;
+            float* o = a.out + (long long)m0 * n;
+            if (((uintptr_t)o & 15) == 0) {
+                for (int t = threadIdx.x; t < nv / 4; t += TC_THREADS) ((float4*)o)[t] = ((const float4*)so)[t];
+                for (int t = (nv & ~3) + threadIdx.x; t < nv; t += TC_THREADS) o[t] = so[t];
+            } else {
+                for (int t = threadIdx.x; t < nv; t += TC_THREADS) o[t] = so[t];
+            }
         }
     }
-    if (!ok) {
-        if (threadIdx.x == 0) atomicExch(&g_tc_err, 1);
-        // g K chunks were committed (a chunk counts once its MMAs are
-        // issued): one more bounded wait on the last commit before the
-        // tensor memory is freed
-        if (g > 0) mbar_wait(&bar[(g - 1) & 1], (uint32_t)(((g - 1) >> 1) & 1), timeout_ns);
+    if (!ok && threadIdx.x == 0) {
+        atomicExch(&g_tc_err, 1);
+        // copies still in flight, and the last committed MMAs, before the
+        // shared and tensor memory go (bounded)
+        for (int q = waited; q < issued; ++q) mbar_wait(&full[q % MF_NB], (uint32_t)((q / MF_NB) & 1), timeout_ns);
+        if (committed > 0) mbar_wait(&done[(committed - 1) % MF_NB], (uint32_t)(((committed - 1) / MF_NB) & 1), timeout_ns);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -608,21 +712,23 @@ cudaError_t gemm(const GemmArgs& g, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// dY := dY * (Y > 0)  (ReLU backward, in place on the FP32 gradient)
-__global__ void k_relu_back(long long n, const float* __restrict__ y, float* __restrict__ dy)
+// column sums: db[j] = sum_i dY[i][j].  32 columns x 32 row groups per block
+// (one thread per column took 60 us for 1024 rows), fixed order
+__global__ void __launch_bounds__(1024) k_colsum(int M, int N, const float* __restrict__ dy, float* __restrict__ db)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        if (!(y[i] > 0.f)) dy[i] = 0.f;
-}
-
-// column sums: db[j] = sum_i dY[i][j]  (one thread per column, fixed order)
-__global__ void k_colsum(int M, int N, const float* __restrict__ dy, float* __restrict__ db)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
+    __shared__ float sm[32][33];
+    const int c = threadIdx.x & 31, r = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + c;
     float s = 0.f;
-    for (int i = 0; i < M; ++i) s += dy[(long long)i * N + j];
-    db[j] = s;
+    if (j < N)
+#pragma unroll 8
+        for (int i = r; i < M; i += 32) s += dy[(long long)i * N + j];
+    sm[r][c] = s;
+    __syncthreads();
+    float v = sm[c][r];  // row groups of column r of the block
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (c == 0 && blockIdx.x * 32 + r < N) db[blockIdx.x * 32 + r] = v;
 }
 
 // mean-squared-error gradient: d = (pred - target) * 2 / (M * n_out); loss partial sums
@@ -688,6 +794,10 @@ struct sem_learner {
     // rebuilt before a forward pass whenever the weights changed
     __nv_bfloat16* WbfT[3] = {};
     bool wt_dirty = true;
+    // packed weight chunks of the fused inference pass (k_pack_weights), rebuilt
+    // before it whenever the weights changed
+    unsigned char* img[3] = {};
+    bool img_dirty = true;
     int rows_cap = 0;
     float *h1 = nullptr, *h2 = nullptr, *out = nullptr, *d2 = nullptr, *d1 = nullptr, *dout = nullptr;
     __nv_bfloat16 *h1bf = nullptr, *h2bf = nullptr;
@@ -762,6 +872,8 @@ extern "C" int sem_learner_create(sem_learner** out, int d_in, int hidden, int d
         for (float** p : bb) LCUDA(cudaMalloc(p, nb * 4));
         LCUDA(cudaMalloc(&L->Wbf[l], nw * 2));
         LCUDA(cudaMalloc(&L->WbfT[l], nw * 2));
+        if (hidden <= 256 && d_out <= 256)  // the fused inference pass
+            LCUDA(cudaMalloc(&L->img[l], (size_t)((L->din(l) + TC_BK - 1) / TC_BK) * mf_round16(L->dout_(l)) * TC_BK * 2));
         LCUDA(cudaMemcpy(L->W[l], w.data(), nw * 4, cudaMemcpyHostToDevice));
         LCUDA(cudaMemset(L->mW[l], 0, nw * 4));
         LCUDA(cudaMemset(L->vW[l], 0, nw * 4));
@@ -786,6 +898,7 @@ extern "C" int sem_learner_destroy(sem_learner* L)
             if (p) cudaFree(p);
         if (L->Wbf[l]) cudaFree(L->Wbf[l]);
         if (L->WbfT[l]) cudaFree(L->WbfT[l]);
+        if (L->img[l]) cudaFree(L->img[l]);
     }
     float* f2[] = {L->h1, L->h2, L->out, L->d2, L->d1, L->dout};
     for (float* p : f2)
@@ -830,7 +943,7 @@ extern "C" int sem_learner_set_params(sem_learner* L, int l, const float* W, con
     if (W) {
         LCUDA(cudaMemcpy(L->W[l], W, nw * 4, cudaMemcpyHostToDevice));
         k_to_bf16<<<g1d(nw), 256, 0, L->stream>>>(nw, L->W[l], L->Wbf[l]);
-        L->wt_dirty = true;
+        L->wt_dirty = L->img_dirty = true;
         LCUDA(cudaGetLastError());
     }
     if (b) LCUDA(cudaMemcpy(L->b[l], b, (size_t)L->dout_(l) * 4, cudaMemcpyHostToDevice));
@@ -863,8 +976,15 @@ static bool fused_forward_ok(const sem_learner* L)
 // inference: x (rows x d_in, BF16) -> out (rows x d_out, FP32) in one launch
 static int forward_fused(sem_learner* L, int rows, const __nv_bfloat16* x, float* out)
 {
-    int s = refresh_wt(L);
-    if (s) return s;
+    if (L->img_dirty) {
+        for (int l = 0; l < 3; ++l) {
+            k_pack_weights<<<g1d((long long)mf_round16(L->dout_(l)) * ((L->din(l) + 7) / 8)), 256, 0, L->stream>>>(
+                L->din(l), L->dout_(l), L->Wbf[l], L->img[l]);
+        }
+        LCUDA(cudaGetLastError());
+        L->img_dirty = false;
+        L->forward_launches += 3;
+    }
     MlpArgs a{};
     a.rows = rows;
     a.d_in = L->d_in;
@@ -873,7 +993,7 @@ static int forward_fused(sem_learner* L, int rows, const __nv_bfloat16* x, float
     a.x = x;
     a.out = out;
     for (int l = 0; l < 3; ++l) {
-        a.WT[l] = L->WbfT[l];
+        a.img[l] = L->img[l];
         a.b[l] = L->b[l];
     }
     LCUDA(cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MF_SMEM));
@@ -941,14 +1061,13 @@ extern "C" int sem_learner_train_step(sem_learner* L, int rows, const void* x_bf
     g.B = L->dout; g.sb_k = L->d_out; g.sb_n = 1; g.b_bf16 = 0;
     g.C = L->gW[2]; g.ldc = L->d_out;
     LCUDA(gemm(g, L->stream));
-    k_colsum<<<(L->d_out + 127) / 128, 128, 0, L->stream>>>(rows, L->d_out, L->dout, L->gb[2]);
+    k_colsum<<<(L->d_out + 31) / 32, 1024, 0, L->stream>>>(rows, L->d_out, L->dout, L->gb[2]);
     g = GemmArgs{};
     g.M = rows; g.N = L->H; g.K = L->d_out;
     g.A = L->dout; g.sa_m = L->d_out; g.sa_k = 1; g.a_bf16 = 0;
     g.B = L->Wbf[2]; g.sb_k = 1; g.sb_n = L->d_out; g.b_bf16 = 1;
-    g.C = L->d2; g.ldc = L->H;
+    g.C = L->d2; g.ldc = L->H; g.mask = L->h2;
     LCUDA(gemm(g, L->stream));
-    k_relu_back<<<g1d((long long)rows * L->H), 256, 0, L->stream>>>((long long)rows * L->H, L->h2, L->d2);
     // layer 2
     g = GemmArgs{};
     g.M = L->H; g.N = L->H; g.K = rows;
@@ -956,14 +1075,13 @@ extern "C" int sem_learner_train_step(sem_learner* L, int rows, const void* x_bf
     g.B = L->d2; g.sb_k = L->H; g.sb_n = 1; g.b_bf16 = 0;
     g.C = L->gW[1]; g.ldc = L->H;
     LCUDA(gemm(g, L->stream));
-    k_colsum<<<(L->H + 127) / 128, 128, 0, L->stream>>>(rows, L->H, L->d2, L->gb[1]);
+    k_colsum<<<(L->H + 31) / 32, 1024, 0, L->stream>>>(rows, L->H, L->d2, L->gb[1]);
     g = GemmArgs{};
     g.M = rows; g.N = L->H; g.K = L->H;
     g.A = L->d2; g.sa_m = L->H; g.sa_k = 1; g.a_bf16 = 0;
     g.B = L->Wbf[1]; g.sb_k = 1; g.sb_n = L->H; g.b_bf16 = 1;
-    g.C = L->d1; g.ldc = L->H;
+    g.C = L->d1; g.ldc = L->H; g.mask = L->h1;
     LCUDA(gemm(g, L->stream));
-    k_relu_back<<<g1d((long long)rows * L->H), 256, 0, L->stream>>>((long long)rows * L->H, L->h1, L->d1);
     // layer 1
     g = GemmArgs{};
     g.M = L->d_in; g.N = L->H; g.K = rows;
@@ -971,11 +1089,11 @@ extern "C" int sem_learner_train_step(sem_learner* L, int rows, const void* x_bf
     g.B = L->d1; g.sb_k = L->H; g.sb_n = 1; g.b_bf16 = 0;
     g.C = L->gW[0]; g.ldc = L->H;
     LCUDA(gemm(g, L->stream));
-    k_colsum<<<(L->H + 127) / 128, 128, 0, L->stream>>>(rows, L->H, L->d1, L->gb[0]);
+    k_colsum<<<(L->H + 31) / 32, 1024, 0, L->stream>>>(rows, L->H, L->d1, L->gb[0]);
     LCUDA(cudaGetLastError());
     if (lr > 0.f) {
         ++L->adam_t;
-        L->wt_dirty = true;
+        L->wt_dirty = L->img_dirty = true;
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.f - std::pow(b1, (float)L->adam_t), c2 = 1.f - std::pow(b2, (float)L->adam_t);
         for (int l = 0; l < 3; ++l) {
