@@ -37,6 +37,7 @@ struct GemmArgs {
     int a_bf16;            // A is __nv_bfloat16 (else float)
     const void* B;
     long long sb_k, sb_n;  // B(k,n) = B[k*sb_k + n*sb_n]
+    int vec_a, vec_b;      // tcgen05 kernel: load widths (tc_vec; set by gemm())
     int b_bf16;
     float* C;              // C[m*ldc + n] (FP32)
     int ldc;
@@ -179,48 +180,48 @@ __device__ __forceinline__ uint32_t tc_off(int R, int r, int k)
     return (uint32_t)((k >> 4) * (R * 32) + (r >> 3) * 256 + ((k >> 3) & 1) * 128 + (r & 7) * 16 + (k & 7) * 2);
 }
 
-// 8 consecutive values of one operand row (K-contiguous when stride 1),
-// packed as 4 BF16 pairs; vector loads when the row run is aligned and in range
-__device__ __forceinline__ void tc_chunk(const void* X, int bf, long long base, long long sk, int kvalid,
-                                         uint32_t (&w)[4])
+// 8 consecutive BF16 values as 4 packed words by loads of VB bytes (p so
+// aligned); no branch inside, so a run of these keeps every load in flight
+template <int VB>
+__device__ __forceinline__ void tc_chunk(const __nv_bfloat16* p, bool in, uint32_t (&w)[4])
 {
-    if (sk == 1 && kvalid >= 8) {
-        if (bf) {
-            const __nv_bfloat16* p = (const __nv_bfloat16*)X + base;
-            const uintptr_t a = (uintptr_t)p;
-            if ((a & 15) == 0) {
-                const uint4 v = __ldg((const uint4*)p);
-                w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-                return;
-            }
-            if ((a & 7) == 0) {
-                const uint2 v0 = __ldg((const uint2*)p), v1 = __ldg((const uint2*)p + 1);
-                w[0] = v0.x; w[1] = v0.y; w[2] = v1.x; w[3] = v1.y;
-                return;
-            }
-            if ((a & 3) == 0) {
+    w[0] = w[1] = w[2] = w[3] = 0u;
+    if constexpr (VB == 16) {
+        if (in) {
+            const uint4 v = __ldg((const uint4*)p);
+            w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        }
+    } else if constexpr (VB == 8) {
+        if (in) {
+            const uint2 v0 = __ldg((const uint2*)p), v1 = __ldg((const uint2*)p + 1);
+            w[0] = v0.x; w[1] = v0.y; w[2] = v1.x; w[3] = v1.y;
+        }
+    } else if constexpr (VB == 4) {
+        if (in) {
 #pragma unroll
-                for (int h = 0; h < 4; ++h) w[h] = __ldg((const unsigned int*)p + h);
-                return;
-            }
-        } else {
-            const float* p = (const float*)X + base;
-            if (((uintptr_t)p & 15) == 0) {
-                const float4 v0 = __ldg((const float4*)p), v1 = __ldg((const float4*)p + 1);
-                w[0] = pack_bf16(__float2bfloat16(v0.x), __float2bfloat16(v0.y));
-                w[1] = pack_bf16(__float2bfloat16(v0.z), __float2bfloat16(v0.w));
-                w[2] = pack_bf16(__float2bfloat16(v1.x), __float2bfloat16(v1.y));
-                w[3] = pack_bf16(__float2bfloat16(v1.z), __float2bfloat16(v1.w));
-                return;
-            }
+            for (int h = 0; h < 4; ++h) w[h] = __ldg((const unsigned int*)p + h);
+        }
+    } else {
+        if (in) {
+            const unsigned short* u = (const unsigned short*)p;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) w[h] = (uint32_t)__ldg(u + 2 * h) | ((uint32_t)__ldg(u + 2 * h + 1) << 16);
         }
     }
+}
+// the first n < 8 of them
+__device__ __forceinline__ void tc_chunk_part(const __nv_bfloat16* p, int n, uint32_t (&w)[4])
+{
+    const unsigned short* u = (const unsigned short*)p;
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        const float v0 = (2 * h < kvalid) ? ld_any(X, base + (long long)(2 * h) * sk, bf) : 0.f;
-        const float v1 = (2 * h + 1 < kvalid) ? ld_any(X, base + (long long)(2 * h + 1) * sk, bf) : 0.f;
-        w[h] = pack_bf16(__float2bfloat16(v0), __float2bfloat16(v1));
-    }
+    for (int h = 0; h < 4; ++h)
+        w[h] = (2 * h < n ? (uint32_t)__ldg(u + 2 * h) : 0u) | (2 * h + 1 < n ? (uint32_t)__ldg(u + 2 * h + 1) << 16 : 0u);
+}
+// host: the widest of 16, 8, 4, 2 bytes that divides the address of every row
+inline int tc_vec(const void* p, long long ld)
+{
+    const unsigned long long a = (unsigned long long)(uintptr_t)p | (unsigned long long)(ld * 2);
+    return (a & 15) == 0 ? 16 : (a & 7) == 0 ? 8 : (a & 3) == 0 ? 4 : 2;
 }
 
 // One operand of a K tile, rows [row0, row0 + R) x [k0, k0 + TC_BK), in two
@@ -232,50 +233,52 @@ __device__ __forceinline__ void tc_chunk(const void* X, int bf, long long base, 
 //    takes 8 rows x 8 k, one vector load per k over 8 consecutive rows, and
 //    transposes the block in registers; it stores its rows starting from its
 //    lane's so that the eight lanes of a store phase hit different banks.
-//    (Chunks along k cost 8 scalar loads each, uncoalesced: 150 us for a
-//    1024-row gradient GEMM.)
-template <int R>
-__device__ __forceinline__ void tc_load(const void* X, int bf, long long sr, long long sk, int rows, int K, int row0,
-                                        int k0, uint32_t (&w)[8][4])
+//    (Chunks along k cost 8 scalar loads each, uncoalesced.)
+// The load width is chosen once per operand on the host: choosing it chunk by
+// chunk put every load behind a branch and a register merge, one L2 latency per
+// chunk, 8.7 us per K tile.
+template <int R, int VB>
+__device__ __forceinline__ void tc_load_v(const __nv_bfloat16* X, bool trans, long long ld, int rows, int K, int row0,
+                                          int k0, uint32_t (&w)[8][4])
 {
-    if (sr == 1 && sk != 1) {
+    if (trans) {
         const int mb = threadIdx.x % (R / 8), kb = threadIdx.x / (R / 8);
         const int r = row0 + mb * 8, nr = min(8, rows - r);
+        const __nv_bfloat16* p = X + r + (long long)(k0 + kb * 8) * ld;
+        const int nkq = kb < TC_BK / 8 ? K - (k0 + kb * 8) : 0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = k0 + kb * 8 + q;
-            const int valid = (kb < TC_BK / 8 && k < K) ? nr : 0;
-            if (valid <= 0) {
-                w[q][0] = w[q][1] = w[q][2] = w[q][3] = 0u;
-            } else if (!bf && valid >= 8 && (((uintptr_t)((const float*)X + r + (long long)k * sk)) & 15) == 8) {
-                const float2* p = (const float2*)((const float*)X + r + (long long)k * sk);  // 8-byte aligned rows
+        for (int q = 0; q < 8; ++q) tc_chunk<VB>(p + q * ld, q < nkq && nr == 8, w[q]);
+        if (nr > 0 && nr < 8)
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const float2 v = __ldg(p + h);
-                    w[q][h] = pack_bf16(__float2bfloat16(v.x), __float2bfloat16(v.y));
-                }
-            } else {
-                tc_chunk(X, bf, r + (long long)k * sk, 1, valid, w[q]);
-            }
-        }
+            for (int q = 0; q < 8; ++q)
+                if (q < nkq) tc_chunk_part(p + q * ld, nr, w[q]);
         return;
     }
+    const int k = k0 + (threadIdx.x & 7) * 8, nk = min(8, K - k);
+    const __nv_bfloat16* p = X + (long long)(row0 + (threadIdx.x >> 3)) * ld + k;
+    const int r0 = row0 + (threadIdx.x >> 3);
 #pragma unroll
-    for (int i = 0; i < R / 16; ++i) {
-        const int q = threadIdx.x + i * TC_THREADS;
-        const int r = q >> 3, k = k0 + (q & 7) * 8;
-        const int kvalid = row0 + r < rows ? min(8, K - k) : 0;
-        if (kvalid <= 0)
-            w[i][0] = w[i][1] = w[i][2] = w[i][3] = 0u;
-        else
-            tc_chunk(X, bf, (long long)(row0 + r) * sr + (long long)k * sk, sk, kvalid, w[i]);
-    }
+    for (int i = 0; i < R / 16; ++i) tc_chunk<VB>(p + (long long)(i * 16) * ld, r0 + i * 16 < rows && nk == 8, w[i]);
+    if (nk > 0 && nk < 8)
+#pragma unroll
+        for (int i = 0; i < R / 16; ++i)
+            if (r0 + i * 16 < rows) tc_chunk_part(p + (long long)(i * 16) * ld, nk, w[i]);
+}
+template <int R>
+__device__ __forceinline__ void tc_load(const void* X, int vec, bool trans, long long ld, int rows, int K, int row0,
+                                        int k0, uint32_t (&w)[8][4])
+{
+    const __nv_bfloat16* x = (const __nv_bfloat16*)X;
+    if (vec == 16) tc_load_v<R, 16>(x, trans, ld, rows, K, row0, k0, w);
+    else if (vec == 8) tc_load_v<R, 8>(x, trans, ld, rows, K, row0, k0, w);
+    else if (vec == 4) tc_load_v<R, 4>(x, trans, ld, rows, K, row0, k0, w);
+    else tc_load_v<R, 2>(x, trans, ld, rows, K, row0, k0, w);
 }
 
 template <int R>
-__device__ __forceinline__ void tc_store(long long sr, long long sk, unsigned char* dst, uint32_t (&w)[8][4])
+__device__ __forceinline__ void tc_store(bool trans, unsigned char* dst, uint32_t (&w)[8][4])
 {
-    if (sr == 1 && sk != 1) {
+    if (trans) {
         const int mb = threadIdx.x % (R / 8), kb = threadIdx.x / (R / 8);
         if (kb >= TC_BK / 8) return;
         uint32_t t[8][4];  // row j: k pairs
@@ -341,8 +344,10 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
     bool ok = true;
     int issued = 0;  // K chunks whose MMAs thread 0 has committed
     uint32_t wa[8][4], wb[8][4];
-    tc_load<TC_M>(g.A, g.a_bf16, g.sa_m, g.sa_k, g.M, g.K, m0, 0, wa);
-    tc_load<BN>(g.B, g.b_bf16, g.sb_n, g.sb_k, g.N, g.K, n0, 0, wb);
+    const bool ta = g.sa_k != 1, tb = g.sb_k != 1;  // rows contiguous
+    const long long lda = ta ? g.sa_k : g.sa_m, ldb = tb ? g.sb_k : g.sb_n;
+    tc_load<TC_M>(g.A, g.vec_a, ta, lda, g.M, g.K, m0, 0, wa);
+    tc_load<BN>(g.B, g.vec_b, tb, ldb, g.N, g.K, n0, 0, wb);
     for (int kt = 0; kt < nk && ok; ++kt) {
         const int b = kt & 1;
         if (kt >= 2) ok = mbar_wait(&bar[b], (uint32_t)(((kt - 2) >> 1) & 1), timeout_ns);
@@ -350,11 +355,11 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
             ok = false;
             break;
         }
-        tc_store<TC_M>(g.sa_m, g.sa_k, sA(b), wa);
-        tc_store<BN>(g.sb_n, g.sb_k, sB(b), wb);
+        tc_store<TC_M>(ta, sA(b), wa);
+        tc_store<BN>(tb, sB(b), wb);
         if (kt + 1 < nk) {
-            tc_load<TC_M>(g.A, g.a_bf16, g.sa_m, g.sa_k, g.M, g.K, m0, (kt + 1) * TC_BK, wa);
-            tc_load<BN>(g.B, g.b_bf16, g.sb_n, g.sb_k, g.N, g.K, n0, (kt + 1) * TC_BK, wb);
+            tc_load<TC_M>(g.A, g.vec_a, ta, lda, g.M, g.K, m0, (kt + 1) * TC_BK, wa);
+            tc_load<BN>(g.B, g.vec_b, tb, ldb, g.N, g.K, n0, (kt + 1) * TC_BK, wb);
         }
         fence_proxy_async_smem();  // the staged tile is read by the tensor cores (async proxy)
         __syncthreads();
@@ -465,6 +470,7 @@ static_assert(MF_SMEM >= 128 * 256 * sizeof(float), "the output tile overlays th
 struct MlpArgs {
     int rows, d_in, H, d_out;
     const __nv_bfloat16* x;       // rows x d_in
+    int vec;                      // its load width (tc_vec)
     const unsigned char* img[3];  // packed weight chunks
     const float* b[3];
     float* out;                   // rows x d_out
@@ -582,7 +588,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_fwd(MlpArgs a, long long tim
     bool ok = true;
     int g = 0;  // chunks so far
     uint32_t w[8][4];
-    tc_load<TC_M>(a.x, 1, a.d_in, 1, a.rows, a.d_in, m0, 0, w);
+    tc_load<TC_M>(a.x, a.vec, false, a.d_in, a.rows, a.d_in, m0, 0, w);
     for (int l = 0; l < 3 && ok; ++l) {
         const int n = l == 2 ? a.d_out : a.H;
         const int nk = l == 0 ? nk1 : nk2;
@@ -595,8 +601,8 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_fwd(MlpArgs a, long long tim
                     ok = false;
                     break;
                 }
-                tc_store<TC_M>(a.d_in, 1, abuf + (kt & 1) * MF_AB, w);
-                if (kt + 1 < nk) tc_load<TC_M>(a.x, 1, a.d_in, 1, a.rows, a.d_in, m0, (kt + 1) * TC_BK, w);
+                tc_store<TC_M>(false, abuf + (kt & 1) * MF_AB, w);
+                if (kt + 1 < nk) tc_load<TC_M>(a.x, a.vec, false, a.d_in, a.rows, a.d_in, m0, (kt + 1) * TC_BK, w);
                 fence_proxy_async_smem();
                 __syncthreads();
                 if (threadIdx.x == 0) ok = step(kt, 0, kt);
@@ -687,14 +693,20 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_fwd(MlpArgs a, long long tim
 // 2 the tcgen05 kernel per layer, 0 the warp-level mma.sync kernel
 int g_gemm_path = 1;
 
-cudaError_t gemm(const GemmArgs& g, cudaStream_t st)
+cudaError_t gemm(const GemmArgs& g0, cudaStream_t st)
 {
-    if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaSuccess;
+    if (g0.M <= 0 || g0.N <= 0 || g0.K <= 0) return cudaSuccess;
     if (g_gemm_path == 0) {
-        dim3 grid((g.N + GT_N - 1) / GT_N, (g.M + GT_M - 1) / GT_M);
-        k_gemm_bf16<<<grid, 128, 0, st>>>(g);
+        dim3 grid((g0.N + GT_N - 1) / GT_N, (g0.M + GT_M - 1) / GT_M);
+        k_gemm_bf16<<<grid, 128, 0, st>>>(g0);
         return cudaGetLastError();
     }
+    // the tensor-core kernel takes BF16 operands with one contiguous direction
+    if (!g0.a_bf16 || !g0.b_bf16 || (g0.sa_m != 1 && g0.sa_k != 1) || (g0.sb_n != 1 && g0.sb_k != 1))
+        return cudaErrorInvalidValue;
+    GemmArgs g = g0;
+    g.vec_a = tc_vec(g.A, g.sa_k != 1 ? g.sa_k : g.sa_m);
+    g.vec_b = tc_vec(g.B, g.sb_k != 1 ? g.sb_k : g.sb_n);
     const long long tmo = 2000000000LL;  // 2 s
     // 64-column tiles when 128-column ones would leave most SMs idle
     const long long mt = (g.M + TC_M - 1) / TC_M;
@@ -733,13 +745,14 @@ __global__ void __launch_bounds__(1024) k_colsum(int M, int N, const float* __re
 
 // mean-squared-error gradient: d = (pred - target) * 2 / (M * n_out); loss partial sums
 __global__ void k_mse(long long n, float scale, const float* __restrict__ pred, const float* __restrict__ tgt,
-                      float* __restrict__ d, double* __restrict__ loss)
+                      float* __restrict__ d, __nv_bfloat16* __restrict__ dbf, double* __restrict__ loss)
 {
     __shared__ double red[34];
     double s = 0.0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float e = pred[i] - tgt[i];
         d[i] = 2.f * scale * e;
+        dbf[i] = __float2bfloat16(2.f * scale * e);
         s += (double)e * e;
     }
     s = block_sum(s, red);
@@ -800,7 +813,7 @@ struct sem_learner {
     bool img_dirty = true;
     int rows_cap = 0;
     float *h1 = nullptr, *h2 = nullptr, *out = nullptr, *d2 = nullptr, *d1 = nullptr, *dout = nullptr;
-    __nv_bfloat16 *h1bf = nullptr, *h2bf = nullptr;
+    __nv_bfloat16 *h1bf = nullptr, *h2bf = nullptr, *d1bf = nullptr, *d2bf = nullptr, *doutbf = nullptr;
     double* loss = nullptr;
     long long adam_t = 0;
     long long forward_launches = 0;  // kernels launched by forward passes
@@ -830,6 +843,9 @@ static int ensure_rows(sem_learner* L, int rows)
         if (*p) cudaFree(*p);
     if (L->h1bf) cudaFree(L->h1bf);
     if (L->h2bf) cudaFree(L->h2bf);
+    if (L->d1bf) cudaFree(L->d1bf);
+    if (L->d2bf) cudaFree(L->d2bf);
+    if (L->doutbf) cudaFree(L->doutbf);
     const size_t r = (size_t)rows;
     LCUDA(cudaMalloc(&L->h1, r * L->H * 4));
     LCUDA(cudaMalloc(&L->h2, r * L->H * 4));
@@ -839,6 +855,9 @@ static int ensure_rows(sem_learner* L, int rows)
     LCUDA(cudaMalloc(&L->dout, r * L->d_out * 4));
     LCUDA(cudaMalloc(&L->h1bf, r * L->H * 2));
     LCUDA(cudaMalloc(&L->h2bf, r * L->H * 2));
+    LCUDA(cudaMalloc(&L->d1bf, r * L->H * 2));
+    LCUDA(cudaMalloc(&L->d2bf, r * L->H * 2));
+    LCUDA(cudaMalloc(&L->doutbf, r * L->d_out * 2));
     L->rows_cap = rows;
     return SEM_OK;
 }
@@ -905,6 +924,9 @@ extern "C" int sem_learner_destroy(sem_learner* L)
         if (p) cudaFree(p);
     if (L->h1bf) cudaFree(L->h1bf);
     if (L->h2bf) cudaFree(L->h2bf);
+    if (L->d1bf) cudaFree(L->d1bf);
+    if (L->d2bf) cudaFree(L->d2bf);
+    if (L->doutbf) cudaFree(L->doutbf);
     if (L->loss) cudaFree(L->loss);
     delete L;
     return SEM_OK;
@@ -991,6 +1013,7 @@ static int forward_fused(sem_learner* L, int rows, const __nv_bfloat16* x, float
     a.H = L->H;
     a.d_out = L->d_out;
     a.x = x;
+    a.vec = tc_vec(x, L->d_in);
     a.out = out;
     for (int l = 0; l < 3; ++l) {
         a.img[l] = L->img[l];
@@ -1052,41 +1075,41 @@ extern "C" int sem_learner_train_step(sem_learner* L, int rows, const void* x_bf
     if (s) return s;
     const long long no = (long long)rows * L->d_out;
     LCUDA(cudaMemsetAsync(L->loss, 0, sizeof(double), L->stream));
-    k_mse<<<g1d(no), 256, 0, L->stream>>>(no, 1.f / (float)no, L->out, target, L->dout, L->loss);
+    k_mse<<<g1d(no), 256, 0, L->stream>>>(no, 1.f / (float)no, L->out, target, L->dout, L->doutbf, L->loss);
     LCUDA(cudaGetLastError());
     // layer 3: gW3 = h2^T dout, gb3 = colsum(dout), d2 = dout W3^T (masked by ReLU)
     GemmArgs g{};
     g.M = L->H; g.N = L->d_out; g.K = rows;
     g.A = L->h2bf; g.sa_m = 1; g.sa_k = L->H; g.a_bf16 = 1;
-    g.B = L->dout; g.sb_k = L->d_out; g.sb_n = 1; g.b_bf16 = 0;
+    g.B = L->doutbf; g.sb_k = L->d_out; g.sb_n = 1; g.b_bf16 = 1;
     g.C = L->gW[2]; g.ldc = L->d_out;
     LCUDA(gemm(g, L->stream));
     k_colsum<<<(L->d_out + 31) / 32, 1024, 0, L->stream>>>(rows, L->d_out, L->dout, L->gb[2]);
     g = GemmArgs{};
     g.M = rows; g.N = L->H; g.K = L->d_out;
-    g.A = L->dout; g.sa_m = L->d_out; g.sa_k = 1; g.a_bf16 = 0;
+    g.A = L->doutbf; g.sa_m = L->d_out; g.sa_k = 1; g.a_bf16 = 1;
     g.B = L->Wbf[2]; g.sb_k = 1; g.sb_n = L->d_out; g.b_bf16 = 1;
-    g.C = L->d2; g.ldc = L->H; g.mask = L->h2;
+    g.C = L->d2; g.ldc = L->H; g.mask = L->h2; g.Cbf = L->d2bf;
     LCUDA(gemm(g, L->stream));
     // layer 2
     g = GemmArgs{};
     g.M = L->H; g.N = L->H; g.K = rows;
     g.A = L->h1bf; g.sa_m = 1; g.sa_k = L->H; g.a_bf16 = 1;
-    g.B = L->d2; g.sb_k = L->H; g.sb_n = 1; g.b_bf16 = 0;
+    g.B = L->d2bf; g.sb_k = L->H; g.sb_n = 1; g.b_bf16 = 1;
     g.C = L->gW[1]; g.ldc = L->H;
     LCUDA(gemm(g, L->stream));
     k_colsum<<<(L->H + 31) / 32, 1024, 0, L->stream>>>(rows, L->H, L->d2, L->gb[1]);
     g = GemmArgs{};
     g.M = rows; g.N = L->H; g.K = L->H;
-    g.A = L->d2; g.sa_m = L->H; g.sa_k = 1; g.a_bf16 = 0;
+    g.A = L->d2bf; g.sa_m = L->H; g.sa_k = 1; g.a_bf16 = 1;
     g.B = L->Wbf[1]; g.sb_k = 1; g.sb_n = L->H; g.b_bf16 = 1;
-    g.C = L->d1; g.ldc = L->H; g.mask = L->h1;
+    g.C = L->d1; g.ldc = L->H; g.mask = L->h1; g.Cbf = L->d1bf;
     LCUDA(gemm(g, L->stream));
     // layer 1
     g = GemmArgs{};
     g.M = L->d_in; g.N = L->H; g.K = rows;
     g.A = x; g.sa_m = 1; g.sa_k = L->d_in; g.a_bf16 = 1;
-    g.B = L->d1; g.sb_k = L->H; g.sb_n = 1; g.b_bf16 = 0;
+    g.B = L->d1bf; g.sb_k = L->H; g.sb_n = 1; g.b_bf16 = 1;
     g.C = L->gW[0]; g.ldc = L->H;
     LCUDA(gemm(g, L->stream));
     k_colsum<<<(L->H + 31) / 32, 1024, 0, L->stream>>>(rows, L->H, L->d1, L->gb[0]);
