@@ -91,17 +91,24 @@ __global__ void k_to_f32(long long n, const double* __restrict__ a, float* __res
 // Projection stage guess (no counterpart in the reference): the previous
 // stage solutions z_j of the same operator and their right-hand sides b_j.
 constexpr int PROJ_MAX = 24;
+constexpr int PTR_MAX = 32;  // a multiple of 8, above PROJ_MAX
 struct PtrList {
     int nz;
-    const double* z[PROJ_MAX + 1];
-    double c[PROJ_MAX + 1];
+    const double* z[PTR_MAX];
+    double c[PTR_MAX];
+    // the kernels load groups of 8 without branches: unused entries repeat the last
+    void pad()
+    {
+        for (int l = nz; nz > 0 && l < PTR_MAX; ++l) z[l] = z[nz - 1];
+    }
 };
 
-// per-block partial sums of b.b_j (j < L.nz) and b.b, laid out
-// part[blk * (PROJ_MAX + 1) + j] (b.b at j = PROJ_MAX); fixed order.  On
-// masked vectors the plain sum equals the reference's unique-DOF dot.
+// out[j] = b.b_j (j < L.nz) and out[PROJ_MAX] = b.b, fixed order.  On masked
+// vectors the plain sum equals the reference's unique-DOF dot.  A branch per
+// vector kept one load in flight: 64 us for 16 vectors of 64x64, p = 8 (85 MB).
 __global__ void __launch_bounds__(256) k_multidot(long long n, const double* __restrict__ b, PtrList L,
-                                                  double* __restrict__ part)
+                                                  double* __restrict__ part, unsigned int* __restrict__ count,
+                                                  double* __restrict__ out)
 {
     double acc[PROJ_MAX + 1];
 #pragma unroll
@@ -111,25 +118,56 @@ __global__ void __launch_bounds__(256) k_multidot(long long n, const double* __r
         const double bv = b[i];
         acc[PROJ_MAX] = fma(bv, bv, acc[PROJ_MAX]);
 #pragma unroll
-        for (int l = 0; l < PROJ_MAX; ++l)
-            if (l < L.nz) acc[l] = fma(bv, __ldg(L.z[l] + i), acc[l]);
+        for (int g = 0; g < PROJ_MAX; g += 8) {
+            if (g >= L.nz) break;
+            double z[8];
+#pragma unroll
+            for (int l = 0; l < 8; ++l) z[l] = __ldg(L.z[g + l] + i);  // unused entries repeat the last vector
+#pragma unroll
+            for (int l = 0; l < 8; ++l)
+                if (g + l < L.nz) acc[g + l] = fma(bv, z[l], acc[g + l]);
+        }
     }
+    // block sums of the used columns, then (last block to arrive) of the blocks
+    // in their order: one short read-back instead of every block's partials
     __shared__ double red[8][PROJ_MAX + 1];
+    __shared__ bool last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int l = 0; l <= PROJ_MAX; ++l) {
+        if (l >= L.nz && l < PROJ_MAX) continue;
         double v = acc[l];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if (lane == 0) red[wid][l] = v;
     }
     __syncthreads();
-    if (threadIdx.x <= PROJ_MAX) {
+    const int t = threadIdx.x;
+    if (t <= PROJ_MAX && (t < L.nz || t == PROJ_MAX)) {
         double v = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[w][threadIdx.x];
-        part[(size_t)blockIdx.x * (PROJ_MAX + 1) + threadIdx.x] = v;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[w][t];
+        part[(size_t)t * gridDim.x + blockIdx.x] = v;
+        __threadfence();
+    }
+    __syncthreads();
+    if (t == 0) {
+        const unsigned int k = atomicAdd(count, 1u);
+        last = k == gridDim.x - 1;
+        if (last) *count = 0u;  // for the next launch
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int l = wid; l <= PROJ_MAX; l += 8) {
+        if (l >= L.nz && l < PROJ_MAX) continue;
+        double v = 0.0;
+        for (int q = lane; q < (int)gridDim.x; q += 32) v += __ldcg(part + (size_t)l * gridDim.x + q);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) out[l] = v;
     }
 }
+
 
 // out = sum_l c_l z_l over up to PROJ_MAX + 1 vectors
 __global__ void k_lincomb_n(long long n, PtrList L, double* __restrict__ out)
@@ -138,8 +176,15 @@ __global__ void k_lincomb_n(long long n, PtrList L, double* __restrict__ out)
          i += (long long)gridDim.x * blockDim.x) {
         double acc = 0.0;
 #pragma unroll
-        for (int l = 0; l <= PROJ_MAX; ++l)
-            if (l < L.nz) acc = fma(L.c[l], __ldg(L.z[l] + i), acc);
+        for (int g = 0; g < PTR_MAX; g += 8) {
+            if (g >= L.nz) break;
+            double z[8];
+#pragma unroll
+            for (int l = 0; l < 8; ++l) z[l] = __ldg(L.z[g + l] + i);
+#pragma unroll
+            for (int l = 0; l < 8; ++l)
+                if (g + l < L.nz) acc = fma(L.c[g + l], z[l], acc);
+        }
         out[i] = acc;
     }
 }
@@ -344,6 +389,7 @@ struct sem_ctx {
     std::vector<double> Drow_host;         // D row-major (DevMesh::Dh)
     std::vector<double> S_host;            // preconditioner basis row-major (DevMesh::Sh)
     unsigned res_epoch = 0;                // last epoch on the resident solver's exchange words (0: clear them)
+    bool proj_count_ready = false;         // "proj_count" starts at zero
     bool cg_ready = false;                 // "cg_fac" and "cg_wt" hold the mesh's data
     unsigned kr_epoch = 0;                 // the same for the FP64 solvers' reduction words
     std::vector<double> coords;            // [n_nodes][2]
@@ -2203,23 +2249,21 @@ static int proj_dots(sem_ctx* c, const double* b, const double* slots, std::vect
     PtrList L{};
     L.nz = c->proj_count;
     for (int j = 0; j < L.nz; ++j) L.z[j] = slots + (size_t)j * 2 * v + v;
-    constexpr int blocks = 256;
-    double* part = nullptr;
+    L.pad();
+    constexpr int blocks = 304;  // two per SM
+    double *part = nullptr, *dev = nullptr;
+    unsigned int* count = nullptr;
     int s = wsget(c, "proj_part", (size_t)blocks * (PROJ_MAX + 1), &part);
-    if (s) return s;
-    k_multidot<<<blocks, 256, 0, c->stream>>>(v, b, L, part);
+    if (s || (s = wsget(c, "proj_out", PROJ_MAX + 1, &dev)) || (s = wsget(c, "proj_count", 1, &count))) return s;
+    if (!c->proj_count_ready) SEM_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned int), c->stream));
+    c->proj_count_ready = true;
+    k_multidot<<<blocks, 256, 0, c->stream>>>(v, b, L, part, count, dev);
     c->stats.kernel_launches++;
     SEM_CUDA(cudaGetLastError());
-    SEM_CUDA(cudaMemcpyAsync(c->h_part, part, sizeof(double) * blocks * (PROJ_MAX + 1), cudaMemcpyDeviceToHost,
-                             c->stream));
+    SEM_CUDA(cudaMemcpyAsync(c->h_part, dev, sizeof(double) * (PROJ_MAX + 1), cudaMemcpyDeviceToHost, c->stream));
     SEM_CUDA(cudaStreamSynchronize(c->stream));
-    d.assign(L.nz, 0.0);
-    double acc = 0.0;
-    for (int q = 0; q < blocks; ++q) {
-        const double* row = c->h_part + (size_t)q * (PROJ_MAX + 1);
-        for (int j = 0; j < L.nz; ++j) d[j] += row[j];
-        acc += row[PROJ_MAX];
-    }
+    d.assign(c->h_part, c->h_part + L.nz);
+    const double acc = c->h_part[PROJ_MAX];
     *bb = acc;
     return SEM_OK;
 }
@@ -2260,6 +2304,7 @@ static int proj_guess(sem_ctx* c, const double* slots, const std::vector<double>
         L.z[j] = slots + (size_t)j * 4 * c->n;
         L.c[j] = cf[j];
     }
+    L.pad();
     k_lincomb_n<<<grid_1d(2 * c->n), 256, 0, c->stream>>>(2 * c->n, L, x0);
     c->stats.kernel_launches++;
     SEM_CUDA(cudaGetLastError());
@@ -2281,6 +2326,7 @@ static int proj_residual(sem_ctx* c, const double* slots, const std::vector<doub
         L.z[j + 1] = slots + (size_t)j * 4 * c->n + 2 * c->n;
         L.c[j + 1] = -cf[j];
     }
+    L.pad();
     k_lincomb_n<<<grid_1d(2 * c->n), 256, 0, c->stream>>>(2 * c->n, L, r);
     c->stats.kernel_launches++;
     SEM_CUDA(cudaGetLastError());

@@ -388,6 +388,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok) {
         const int m = m0 + warp * 32 + lane;
+        const bool vec4 = (g.ldc & 7) == 0 && (((uintptr_t)g.C | (uintptr_t)g.Cbf | (uintptr_t)g.bias | (uintptr_t)g.mask) & 15) == 0;
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 16) {
             uint32_t r[16];
@@ -400,30 +401,64 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
                 : "r"(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0)
                 : "memory");
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (m < g.M) {
-                // every load of the chunk (bias, accumulated C) before its
+            const long long row = (long long)m * g.ldc + n0 + c0;
+            if (m < g.M && vec4 && n0 + c0 + 16 <= g.N) {
+                // 16-byte accesses: a thread's 16 columns of its own row would
+                // otherwise take one store instruction per 4 bytes of 32 rows
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+                float4 x4[3][4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (g.accumulate) x4[0][q] = *(const float4*)(g.C + row + 4 * q);
+                    if (g.bias) x4[1][q] = __ldg((const float4*)(g.bias + n0 + c0) + q);
+                    if (g.mask) x4[2][q] = __ldg((const float4*)(g.mask + row) + q);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float a4[4] = {x4[0][q].x, x4[0][q].y, x4[0][q].z, x4[0][q].w};
+                    const float b4[4] = {x4[1][q].x, x4[1][q].y, x4[1][q].z, x4[1][q].w};
+                    const float m4[4] = {x4[2][q].x, x4[2][q].y, x4[2][q].z, x4[2][q].w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float& u = v[4 * q + j];
+                        if (g.accumulate) u += a4[j];
+                        if (g.bias) u += b4[j];
+                        if (g.relu) u = fmaxf(u, 0.f);
+                        if (g.mask && !(m4[j] > 0.f)) u = 0.f;
+                    }
+                    *(float4*)(g.C + row + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                }
+                if (g.Cbf) {
+                    uint32_t pk[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) pk[j] = pack_bf16(__float2bfloat16(v[2 * j]), __float2bfloat16(v[2 * j + 1]));
+                    *(uint4*)(g.Cbf + row) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                    *(uint4*)(g.Cbf + row + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                }
+            } else if (m < g.M) {
+                // every load of the chunk (bias, mask, accumulated C) before its
                 // first store: the stores may alias them as far as the
                 // compiler knows, which would serialise load after store
                 float cin[16], bin[16], min_[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const int nn = n0 + c0 + j;
-                    const bool in = nn < g.N;
-                    cin[j] = (in && g.accumulate) ? g.C[(long long)m * g.ldc + nn] : 0.f;
-                    min_[j] = (in && g.mask) ? __ldg(g.mask + (long long)m * g.ldc + nn) : 1.f;
-                    bin[j] = (in && g.bias) ? __ldg(g.bias + nn) : 0.f;
+                    const bool in = n0 + c0 + j < g.N;
+                    cin[j] = (in && g.accumulate) ? g.C[row + j] : 0.f;
+                    min_[j] = (in && g.mask) ? __ldg(g.mask + row + j) : 1.f;
+                    bin[j] = (in && g.bias) ? __ldg(g.bias + n0 + c0 + j) : 0.f;
                 }
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const int nn = n0 + c0 + j;
-                    if (nn >= g.N) continue;
+                    if (n0 + c0 + j >= g.N) continue;
                     float v = __uint_as_float(r[j]);
                     if (g.accumulate) v += cin[j];
                     if (g.bias) v += bin[j];
                     if (g.relu) v = fmaxf(v, 0.f);
                     if (!(min_[j] > 0.f)) v = 0.f;
-                    g.C[(long long)m * g.ldc + nn] = v;
-                    if (g.Cbf) g.Cbf[(long long)m * g.ldc + nn] = __float2bfloat16(v);
+                    g.C[row + j] = v;
+                    if (g.Cbf) g.Cbf[row + j] = __float2bfloat16(v);
                 }
             }
         }
