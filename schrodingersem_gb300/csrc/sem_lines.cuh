@@ -15,7 +15,7 @@
 #pragma once
 #include <cstdint>
 #include <cstring>
-
+#include <type_traits>
 
 namespace semgb {
 
@@ -73,40 +73,70 @@ __device__ __forceinline__ float f2y(f2_t v)
 // values a line pass works on: an FP32 pair (both components) or a double
 __device__ __forceinline__ f2_t lv_add(f2_t a, f2_t b) { return f2add(a, b); }
 __device__ __forceinline__ f2_t lv_sub(f2_t a, f2_t b) { return f2sub(a, b); }
-__device__ __forceinline__ f2_t lv_mul(f2_t a, f2_t b) { return f2mul(a, b); }
-__device__ __forceinline__ f2_t lv_fma(f2_t a, f2_t b, f2_t c) { return f2fma(a, b, c); }
 __device__ __forceinline__ double lv_add(double a, double b) { return a + b; }
 __device__ __forceinline__ double lv_sub(double a, double b) { return a - b; }
-__device__ __forceinline__ double lv_mul(double a, double b) { return a * b; }
-__device__ __forceinline__ double lv_fma(double a, double b, double c) { return fma(a, b, c); }
+
+// Table entries of FP32 pairs: both lanes' coefficient, (c, c), for packed FMAs, or
+// one FP32 value for two scalar FMAs.  A packed FMA issues half as often, but its
+// coefficient occupies a register pair that has to be loaded, so the form follows
+// the degree.  Measured per iteration of the stage solver, packed against scalar:
+//   N = 9   64 x 64 elements on chip 15.9 us against 18.5, 192 x 192 streaming 209 against 206
+//   N = 11  30 x 30 on chip 17.5 against 14.6
+//   N = 13  96 x 96 streaming 123 against 96
+//   N = 5   48 x 48 on chip 12.6 against 12.0; N = 6 40 x 40 18.7 against 18.9
+// (the same rounding either way: each lane is one IEEE FP32 FMA)
+template <int N>
+__host__ __device__ constexpr bool eo_packed() { return N >= 8 && N <= 10; }
+template <int N, class V>
+struct EoCoef {
+    using type = double;
+};
+template <int N>
+struct EoCoef<N, f2_t> {
+    using type = typename std::conditional<eo_packed<N>(), f2_t, float>::type;
+};
+__host__ inline void eo_set(double& t, double v) { t = v; }
+__host__ inline void eo_set(float& t, double v) { t = (float)v; }
+__host__ inline void eo_set(f2_t& t, double v)
+{
+    const float f = (float)v;
+    uint32_t u;
+    memcpy(&u, &f, sizeof(u));
+    t = ((f2_t)u << 32) | u;
+}
+__device__ __forceinline__ f2_t lv_cmul(f2_t c, f2_t b) { return f2mul(c, b); }
+__device__ __forceinline__ f2_t lv_cfma(f2_t c, f2_t b, f2_t a) { return f2fma(c, b, a); }
+__device__ __forceinline__ f2_t lv_cmul(float c, f2_t b)
+{
+    float x, y;
+    f2unpack(b, x, y);
+    return f2pack(c * x, c * y);
+}
+__device__ __forceinline__ f2_t lv_cfma(float c, f2_t b, f2_t a)
+{
+    float x, y, u, v;
+    f2unpack(b, x, y);
+    f2unpack(a, u, v);
+    return f2pack(fmaf(c, x, u), fmaf(c, y, v));
+}
+__device__ __forceinline__ double lv_cmul(double c, double b) { return c * b; }
+__device__ __forceinline__ double lv_cfma(double c, double b, double a) { return fma(c, b, a); }
 
 template <int N, class V>
 struct EoD {
     static constexpr int H = N / 2, C = (N + 1) / 2;
-    V P[H * C];  // P(i,k) at [i*C+k]
-    V Q[C * H];  // Q(i,k) at [i*H+k]
+    using K = typename EoCoef<N, V>::type;
+    K P[H * C];  // P(i,k) at [i*C+k]
+    K Q[C * H];  // Q(i,k) at [i*H+k]
 };
 // preconditioner basis, even modes first (fdm_basis orders them so)
 template <int N, class V>
 struct EoS {
     static constexpr int H = N / 2, C = (N + 1) / 2;
-    V E[C * C];  // S(i,k), k even mode, at [i*C+k]
-    V O[H * H];  // S(i,C+k) at [i*H+k]
+    using K = typename EoCoef<N, V>::type;
+    K E[C * C];  // S(i,k), k even mode, at [i*C+k]
+    K O[H * H];  // S(i,C+k) at [i*H+k]
 };
-
-// host: a table entry of type V
-template <class V>
-inline V eo_entry(double v);
-template <>
-inline double eo_entry<double>(double v) { return v; }
-template <>
-inline f2_t eo_entry<f2_t>(double v)
-{
-    const float f = (float)v;
-    uint32_t u;
-    memcpy(&u, &f, sizeof(u));
-    return ((f2_t)u << 32) | u;
-}
 
 // host: tables from D and S, row-major
 template <int N, class V>
@@ -116,9 +146,9 @@ inline EoD<N, V> eo_d_table(const double* D)
     constexpr int H = N / 2, C = (N + 1) / 2;
     for (int i = 0; i < H; ++i)
         for (int k = 0; k < C; ++k)
-            t.P[i * C + k] = eo_entry<V>(k == H ? D[i * N + k] : 0.5 * (D[i * N + k] + D[i * N + N - 1 - k]));
+            eo_set(t.P[i * C + k], k == H ? D[i * N + k] : 0.5 * (D[i * N + k] + D[i * N + N - 1 - k]));
     for (int i = 0; i < C; ++i)
-        for (int k = 0; k < H; ++k) t.Q[i * H + k] = eo_entry<V>(0.5 * (D[i * N + k] - D[i * N + N - 1 - k]));
+        for (int k = 0; k < H; ++k) eo_set(t.Q[i * H + k], 0.5 * (D[i * N + k] - D[i * N + N - 1 - k]));
     return t;
 }
 template <int N, class V>
@@ -127,9 +157,9 @@ inline EoS<N, V> eo_s_table(const double* S)
     EoS<N, V> t;
     constexpr int H = N / 2, C = (N + 1) / 2;
     for (int i = 0; i < C; ++i)
-        for (int k = 0; k < C; ++k) t.E[i * C + k] = eo_entry<V>(S[i * N + k]);
+        for (int k = 0; k < C; ++k) eo_set(t.E[i * C + k], S[i * N + k]);
     for (int i = 0; i < H; ++i)
-        for (int k = 0; k < H; ++k) t.O[i * H + k] = eo_entry<V>(S[i * N + C + k]);
+        for (int k = 0; k < H; ++k) eo_set(t.O[i * H + k], S[i * N + C + k]);
     return t;
 }
 
@@ -149,15 +179,15 @@ __device__ __forceinline__ void eo_d(const EoD<N, V>& t, const V* u, V* o)
     for (int k = 0; k < C; ++k)
 #pragma unroll
         for (int i = 0; i < H; ++i) {
-            const V c = TR ? t.Q[k * H + i] : t.P[i * C + k];
-            a[i] = k == 0 ? lv_mul(c, s[k]) : lv_fma(c, s[k], a[i]);
+            const typename EoCoef<N, V>::type c = TR ? t.Q[k * H + i] : t.P[i * C + k];
+            a[i] = k == 0 ? lv_cmul(c, s[k]) : lv_cfma(c, s[k], a[i]);
         }
 #pragma unroll
     for (int k = 0; k < H; ++k)
 #pragma unroll
         for (int i = 0; i < C; ++i) {
-            const V c = TR ? t.P[k * C + i] : t.Q[i * H + k];
-            b[i] = k == 0 ? lv_mul(c, d[k]) : lv_fma(c, d[k], b[i]);
+            const typename EoCoef<N, V>::type c = TR ? t.P[k * C + i] : t.Q[i * H + k];
+            b[i] = k == 0 ? lv_cmul(c, d[k]) : lv_cfma(c, d[k], b[i]);
         }
 #pragma unroll
     for (int i = 0; i < H; ++i) {
@@ -182,12 +212,12 @@ __device__ __forceinline__ void eo_st(const EoS<N, V>& t, const V* u, V* o)
 #pragma unroll
     for (int i = 0; i < C; ++i)
 #pragma unroll
-        for (int k = 0; k < C; ++k) o[k] = i == 0 ? lv_mul(t.E[k], s[0]) : lv_fma(t.E[i * C + k], s[i], o[k]);
+        for (int k = 0; k < C; ++k) o[k] = i == 0 ? lv_cmul(t.E[k], s[0]) : lv_cfma(t.E[i * C + k], s[i], o[k]);
 #pragma unroll
     for (int i = 0; i < H; ++i)
 #pragma unroll
         for (int k = 0; k < H; ++k)
-            o[C + k] = i == 0 ? lv_mul(t.O[k], d[0]) : lv_fma(t.O[i * H + k], d[i], o[C + k]);
+            o[C + k] = i == 0 ? lv_cmul(t.O[k], d[0]) : lv_cfma(t.O[i * H + k], d[i], o[C + k]);
 }
 
 // u = S t; o may be t
@@ -200,12 +230,12 @@ __device__ __forceinline__ void eo_s(const EoS<N, V>& t, const V* m, V* o)
     for (int k = 0; k < C; ++k)
 #pragma unroll
         for (int i = 0; i < C; ++i)
-            a[i] = k == 0 ? lv_mul(t.E[i * C], m[0]) : lv_fma(t.E[i * C + k], m[k], a[i]);
+            a[i] = k == 0 ? lv_cmul(t.E[i * C], m[0]) : lv_cfma(t.E[i * C + k], m[k], a[i]);
 #pragma unroll
     for (int k = 0; k < H; ++k)
 #pragma unroll
         for (int i = 0; i < H; ++i)
-            b[i] = k == 0 ? lv_mul(t.O[i * H], m[C]) : lv_fma(t.O[i * H + k], m[C + k], b[i]);
+            b[i] = k == 0 ? lv_cmul(t.O[i * H], m[C]) : lv_cfma(t.O[i * H + k], m[C + k], b[i]);
 #pragma unroll
     for (int i = 0; i < H; ++i) {
         o[i] = lv_add(a[i], b[i]);

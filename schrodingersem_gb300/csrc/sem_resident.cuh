@@ -26,7 +26,9 @@
 // thread holds r and x of its row, and the second contraction of the column
 // direction follows the first in the same thread, so an iteration has four
 // block barriers beside the two exchanges.  Measured at 64 x 64 elements,
-// p = 8 (27 elements per SM): see the figures at k_resident.
+// p = 8 (27 elements per SM): 15.9 us per iteration all-in (residual checks and
+// launches included), against 37.7 for the streaming form; two thirds are the
+// latency of the two exchanges and the four barriers, the rest FP32 issue.
 //
 // All-reduce: each block publishes its partials as 64-bit words (FP32 value,
 // 32-bit epoch tag) on its own 128-byte line; every block's first warp polls
@@ -40,14 +42,22 @@
 
 namespace semgb {
 
-constexpr int RES_TPB = 512;
+// one row of both components per thread: 243 rows at 27 elements of p = 8.  With
+// 512 threads half the warps had no row and 128 registers spilled the line
+// contractions: 18.0 us per iteration at 64 x 64 elements of p = 8 against 15.9,
+// 11.8 against 9.7 at 24 x 24, 12.0 against 10.9 at 48 x 48 of p = 4
+constexpr int RES_TPB = 256;
 constexpr int RES_MAXQ = 8;     // words polled per lane: grids up to 256 blocks
 constexpr int RES_PAIRS = 4;    // planes of FP32 pairs: p, q, z, preconditioner symbol
 constexpr int RES_PLANES = 6;   // FP32 planes: g11, -g12, g22, mass, mass V, weight
 constexpr int RES_WSTRIDE = RESIDENT_SLOT_STRIDE;  // all-reduce words 128 bytes apart
-// rows per thread held in registers (N = 5: short rows, two)
-template <int N>
-__host__ __device__ constexpr int res_rows() { return N <= 5 ? 2 : 1; }
+// rows per thread held in registers: 1, 2 or 4, by the block's share
+constexpr int RES_MAXROWS = 4;
+inline int res_rows(int kres, int N)
+{
+    const int r = (kres * N + RES_TPB - 1) / RES_TPB;
+    return r <= 1 ? 1 : r <= 2 ? 2 : r <= RES_MAXROWS ? RES_MAXROWS : 0;
+}
 
 struct ResArgs {
     int st;                     // shared-memory plane length (max elements per block * N^2)
@@ -359,14 +369,13 @@ __device__ __forceinline__ bool res_exchange(const float (&v)[K], const DevMesh&
 // |r| = rn > 0) to |r_it| < tol_rel |r|, at most maxit iterations; adds d to
 // the FP64 solution on owner copies when it is finite.  Returns false when a
 // wait hit its limit.
-template <int N>
+template <int N, int RW>
 __device__ __forceinline__ bool res_inner(const DevMesh& m, const CgTab<N>& tab, const ResPlanes& s, int eb, int ne,
                                           const double* const* r64, double rn, float alpha, const ResArgs& ra,
                                           unsigned& epoch, GridSync* gs, long long tmo, float (*red)[RES_TPB / 32],
                                           float* tot, int maxit, float tol_rel, double* const* xp, CgOut& res)
 {
     constexpr int NN = N * N;
-    constexpr int RW = res_rows<N>();
     const int lines = ne * N;
     const LineNe nb = line_ne(ne);
     res.it = 0;
@@ -620,7 +629,7 @@ __host__ __device__ constexpr size_t res_stage_bytes(int st, int k64)
     const size_t f64 = range_smem_bytes<N, double, OP_RES>(k64);
     return ((pairs > f64 ? pairs : f64) + 15) & ~(size_t)15;
 }
-template <int N>
+template <int N, int RW>
 __global__ void __launch_bounds__(RES_TPB, 1)
     k_resident(DevMesh m, SolveArgs a, KrylovWork<float> w, MixedArgs mx, const __grid_constant__ EoD<N, double> et,
                const __grid_constant__ CgTab<N> tab, ResArgs ra)
@@ -725,7 +734,7 @@ __global__ void __launch_bounds__(RES_TPB, 1)
         last_rn = rn;
         const double* r64c[2] = {mx.r64[0], mx.r64[1]};
         CgOut ir{};
-        if (!res_inner<N>(m, tab, s, eb, ne, r64c, rn, alpha32, ra, epoch, a.sync, a.timeout_ns, redf, tot, budget,
+        if (!res_inner<N, RW>(m, tab, s, eb, ne, r64c, rn, alpha32, ra, epoch, a.sync, a.timeout_ns, redf, tot, budget,
                           (float)itol, xp, ir))
             return;
         inner_total += ir.it;
@@ -763,7 +772,7 @@ bool resident_plan(int E, int sms, size_t smem_budget, int* grid_out, int* st_ou
     if (grid < 1 || grid > 32 * RES_MAXQ) return false;
     const int kres = (E + grid - 1) / grid;
     const int st = kres * NN;
-    if (kres * N > RES_TPB * res_rows<N>()) return false;
+    if (res_rows(kres, N) == 0) return false;
     const size_t fixed = (size_t)st * (sizeof(f2_t) + RES_PLANES * sizeof(float));
     int k64 = kres;
     auto need = [&](int k) { return fixed + res_stage_bytes<N>(st, k); };
@@ -782,7 +791,10 @@ cudaError_t launch_resident(const DevMesh& m, const SolveArgs& a, const KrylovWo
                             int st, unsigned long long* slots, void* xa, void* xb, unsigned epoch0, int grid,
                             size_t smem, cudaStream_t stream)
 {
-    const void* fn = (const void*)k_resident<N>;
+    const int rows = res_rows((m.E + grid - 1) / grid, N);
+    const void* fn = rows == 1   ? (const void*)k_resident<N, 1>
+                     : rows == 2 ? (const void*)k_resident<N, 2>
+                                 : (const void*)k_resident<N, RES_MAXROWS>;
     if (!m.Dh || !m.Sh) return cudaErrorInvalidValue;
     // a per-device function attribute: set on every launch (cheap), so a
     // context on any device of the process gets the opt-in
