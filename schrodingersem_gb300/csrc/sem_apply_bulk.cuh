@@ -730,6 +730,7 @@ __global__ void __launch_bounds__(bulk_tpb_k<T, OP, MG>())
         __syncthreads();
         if (threadIdx.x == 0) issue(b + (long long)S * G, s);
     }
+    ring_release();
     if (threadIdx.x == 0) bulk_wait_all();
 }
 
