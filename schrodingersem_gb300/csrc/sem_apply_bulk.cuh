@@ -270,8 +270,11 @@ __host__ __device__ constexpr bool bulk_f2(int N) { return N <= 11; }
 // and W2 is written out with one bulk store per component.  Every
 // accumulation runs over k in ascending order as in apply_chunk (the
 // one-pass kernel), so both kernels give the same bits.
+// GEO: at most 128 registers (its occupancy is set by them; left alone, the
+// compiler took 113 or 162 with the surrounding code: 261 or 281 us at 559 x 559,
+// p = 8).
 template <int N, typename T, int OP, bool GATHER, bool MG, bool GEO = false>
-__global__ void __launch_bounds__(bulk_tpb_k<T, OP, MG>())
+__global__ void __launch_bounds__(bulk_tpb_k<T, OP, MG>(), GEO && GATHER ? 512 / bulk_tpb_k<T, OP, MG>() : 0)
     k_apply_bulk(DevMesh m, DMat<N, T> D, DMat2<N> D2, const T* __restrict__ pot, T alpha, const T* __restrict__ in0,
                  const T* __restrict__ in1, T* __restrict__ y0, T* __restrict__ y1, int store_bulk, int pair_asm,
                  long long timeout_ns, GeoTab<N> gt)

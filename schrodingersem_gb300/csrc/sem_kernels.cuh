@@ -187,68 +187,65 @@ __global__ void k_dss(DevMesh m, const T* __restrict__ Y, T* __restrict__ out, T
 // order at corners), so the result equals k_dss<MODE> with scale 1 bit for
 // bit.  Element interiors are final as the apply wrote them.
 //
-// Blocks below gp take the side pairs, four of a thread's pairs at a time with
-// their loads issued together; the others the boundary copies and the corners.
 // The pass is bound by its dependent loads (table, values) and by sectors of
-// which it uses one word.  With blocks of their own for the corners (the same
-// low threads did both) and the early launch (3 us of it), the FP32 apply of
-// 301 x 301 elements, p = 8, went from 90.8 to 86.7 us with a cold L2, that of
-// 100 x 100 from 25.3 to 23.2, and an FP64 apply of 8 x 8, p = 4, from 14.3 to 10.3.
+// which it uses one word.  Launched early, with the first tables loaded ahead of
+// the wait, it saves 2 to 4 us: the FP32 apply of 301 x 301 elements, p = 8, went
+// from 90.8 to 86.7 us with a cold L2, that of 559 x 559 from 269 to 263, and an
+// FP64 apply of 8 x 8, p = 4, from 14.3 to 10.3.
 template <int N, typename T, int MODE>
-__global__ void __launch_bounds__(256) k_ring(DevMesh m, long long np, int gp, T* a0, T* a1)
+__global__ void __launch_bounds__(256) k_ring(DevMesh m, long long np, int apart, T* a0, T* a1)
 {
+    const long long nb = m.n_bnd;
+    const long long total = np + nb + m.n_nodes;
     T* planes[2] = {a0, a1};
-    if ((int)blockIdx.x < gp) {
-        const long long stride = (long long)gp * blockDim.x;
-        long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-        int2 pr[4];
-        auto pairs_of = [&](long long i) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long c0 = i0;
+    int2 pr[4];
+    auto pairs_of = [&](long long i) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            pr[q] = i + q * stride < np ? __ldg(m.edge_pairs + i + q * stride) : make_int2(-1, -1);
+    };
+    pairs_of(i0);
+    // the first item after the pairs: its own thread's, or the low threads' again
+    const long long it0 = !apart ? np + c0 : c0 >= np ? c0 : total;
+    if (apart && it0 >= np + nb && it0 < total)  // the corner's row, to L1
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(
+            __cvta_generic_to_global(m.node_nb + (size_t)(it0 - np - nb) * CORNER_NB_MAX)));
+    ring_wait();
+    for (; i0 < np; i0 += 4 * stride, pairs_of(i0)) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            T* a = planes[c];
+            if (!a) continue;
+            T x[4], y[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                pr[q] = i + q * stride < np ? __ldg(m.edge_pairs + i + q * stride) : make_int2(-1, -1);
-        };
-        pairs_of(i0);
-        ring_wait();
-        for (; i0 < np; i0 += 4 * stride, pairs_of(i0)) {
-            T x[2][4], y[2][4];
+                if (pr[q].x >= 0) {
+                    x[q] = a[pr[q].x];
+                    y[q] = a[pr[q].y];
+                }
 #pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (planes[c] && pr[q].x >= 0) {
-                        x[c][q] = planes[c][pr[q].x];
-                        y[c][q] = planes[c][pr[q].y];
-                    }
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (planes[c] && pr[q].x >= 0) {
-                        const T v = x[c][q] + y[c][q];
-                        planes[c][pr[q].x] = v;
-                        planes[c][pr[q].y] = MODE == DSS_MASK ? T(0) : v;
-                    }
+            for (int q = 0; q < 4; ++q)
+                if (pr[q].x >= 0) {
+                    const T v = x[q] + y[q];
+                    a[pr[q].x] = v;
+                    a[pr[q].y] = MODE == DSS_MASK ? T(0) : v;
+                }
         }
-        return;
     }
-    const long long nb = m.n_bnd;
-    const long long total = nb + m.n_nodes;
-    const long long stride = (long long)(gridDim.x - gp) * blockDim.x;
-    const long long it0 = (blockIdx.x - gp) * (long long)blockDim.x + threadIdx.x;
-    if (it0 >= nb && it0 < total)  // the first corner's row, to L1
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(m.node_nb + (size_t)(it0 - nb) * CORNER_NB_MAX)));
-    ring_wait();
     for (long long it = it0; it < total; it += stride) {
-        if (it < nb) {
+        if (it < np + nb) {
             if (MODE == DSS_SUM) continue;
-            const int f = __ldg(m.bnd_flat + it);
+            const int f = __ldg(m.bnd_flat + (it - np));
 #pragma unroll
             for (int q = 0; q < 2; ++q)
                 if (planes[q]) planes[q][f] = T(0);
         } else {
             // corner node: its copies in CSR order from one padded row (two
             // dependent loads: the row, the values), else the CSR
-            const int node = (int)(it - nb);
+            const int node = (int)(it - np - nb);
             const int4* row = reinterpret_cast<const int4*>(m.node_nb + (size_t)node * CORNER_NB_MAX);
             int f[CORNER_NB_MAX];
 #pragma unroll
@@ -750,25 +747,26 @@ template <int N>
 cudaError_t launch_ring(const DevMesh& m, bool fp32, int mode, void* a0, void* a1, bool cross_only,
                         cudaStream_t st)
 {
-    // 152 x 4 blocks of pairs and as many of corners are resident together; small
-    // meshes give each thread one item.  At 301 x 301, p = 8, FP32 the whole apply
-    // took 86.7 us with 4 or 8 blocks per SM, 88.7 with 16 or 32
     const long long np = cross_only ? m.n_pairs_x : m.n_pairs;
-    const int gp = grid_for(np, 256, 152 * 4);
+    // Boundary copies and corners apart from the pairs, on threads of their own,
+    // when all items have a resident thread (8 x 8, p = 4: 10.3 us, 12.3 one after
+    // the other); on larger meshes they follow the pairs on the same threads, whose
+    // sectors they share (559 x 559, p = 8: 263 us, 272 apart)
+    const int apart = np + m.n_bnd + m.n_nodes <= 152 * 2048;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(gp + grid_for((long long)m.n_bnd + m.n_nodes, 256, 152 * 4));
+    cfg.gridDim = dim3(grid_for(np + m.n_bnd + m.n_nodes, 256));
     cfg.blockDim = dim3(256);
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
 #define SEM_RING_CASE(T)                                                                                     \
     switch (mode) {                                                                                          \
-        case DSS_SUM: return cudaLaunchKernelEx(&cfg, k_ring<N, T, DSS_SUM>, m, np, gp, (T*)a0, (T*)a1);     \
-        case DSS_MASK: return cudaLaunchKernelEx(&cfg, k_ring<N, T, DSS_MASK>, m, np, gp, (T*)a0, (T*)a1);   \
-        default: return cudaLaunchKernelEx(&cfg, k_ring<N, T, DSS_CONT>, m, np, gp, (T*)a0, (T*)a1);         \
+        case DSS_SUM: return cudaLaunchKernelEx(&cfg, k_ring<N, T, DSS_SUM>, m, np, apart, (T*)a0, (T*)a1);     \
+        case DSS_MASK: return cudaLaunchKernelEx(&cfg, k_ring<N, T, DSS_MASK>, m, np, apart, (T*)a0, (T*)a1);   \
+        default: return cudaLaunchKernelEx(&cfg, k_ring<N, T, DSS_CONT>, m, np, apart, (T*)a0, (T*)a1);         \
     }
     if (fp32) {
         SEM_RING_CASE(float)

@@ -1,8 +1,9 @@
 """FP64 kernels on parity-split lines, where their dispatch and tiling turn:
-applies on both sides of the size limits (ragged element counts), Krylov solves
-with vectors in shared memory and streamed, from one element to more elements
-than fit; the projection's grouped dot products at basis sizes around the
-groups of 8; network GEMMs whose leading dimensions allow only narrow loads."""
+applies on both sides of the size limits (ragged element counts) and their ring
+pass, Krylov solves with vectors in shared memory and streamed, from one element
+to more elements than fit; the projection's grouped dot products at basis sizes
+around the groups of 8; network GEMMs whose leading dimensions allow only narrow
+loads."""
 import numpy as np
 import pytest
 
@@ -39,6 +40,19 @@ def test_one_component_applies(semlib, oracle, n, p):
     du, dc = ctx.to_device(u), ctx.to_device(c)
     assert rel_err(ctx.apply_laplace(du).cpu().numpy(), om.apply_laplace(u)) <= 1e-12
     assert rel_err(ctx.apply_helmholtz(dc, du).cpu().numpy(), om.apply_helmholtz(c, u)) <= 1e-12
+
+
+# the ring pass gives corners threads of their own up to 311,296 items (3 n^2 + 4 n + 1 at p = 2)
+@pytest.mark.parametrize("n,p", [(3, 2), (321, 2), (322, 2), (330, 2), (140, 8)])
+def test_ring_pass_same_bits(semlib, n, p):
+    """in place of its input an apply is assembled by the gather over all nodes
+    instead of the ring pass: the same sums in the same order"""
+    co, el = structured(n, jitter=0.2, seed=n)
+    ctx = semlib.Context(p, coords=co, elements=el)
+    u = ctx.to_device(np.random.default_rng(n).standard_normal(ctx.shape))
+    out = ctx.apply_laplace(u)
+    ctx.apply_laplace(u, u)
+    assert bool((out == u).all())
 
 
 @pytest.mark.parametrize("n,p", [(1, 4), (40, 1), (13, 8), (5, 15), (13, 16), (64, 8), (100, 8)])
