@@ -58,11 +58,10 @@ WORKLOAD = ("Schroedinger SDIRK4-3 time step, 64x64 jittered quads on [-8,8]^2 (
 DT, TOL, P, NEL = 1e-2, 1e-10, 8, 64
 ORACLE_TOL = 1e-13  # MINRES tolerance of the FP64 accuracy reference runs
 # DRAM bytes (read + write) per launch of the on-chip resident solver kernel
-# (k_minres_resident<9>) inside the timed steps of the headline form: ncu
-# capture summarised in profiles/k_minres_resident_64x64_p8.md (mean of three
-# launches).  The Krylov vectors stay on chip; these bytes are the FP64
-# refinement's fields and the per-launch loads.
-SOLVER_DRAM_BYTES_PER_LAUNCH = 40.94e6
+# (k_resident<9>): ncu capture of one stage solve, summarised in
+# profiles/k_resident_64x64_p8.md.  The Krylov vectors stay on chip; these
+# bytes are the FP64 refinement's fields and the per-launch loads.
+SOLVER_DRAM_BYTES_PER_LAUNCH = 20.55e6
 APPLY_NEL = 559  # 559^2 elements at p = 8: 4473^2 = 20.0 M global nodes
 
 
@@ -598,24 +597,24 @@ FORMS = {
                                           "(its state is just above 1e-8 from the tight solution)"),
     "mixed": ("mixed", 1e-4, 0, 0.5, "FP32-inner MINRES in FP64 iterative refinement (true FP64 residual "
                                      "judged by the reference's criterion), zero stage guess"),
-    "mixed_fdm": ("mixed", 1e-4, 2, 1.0, "FP32-inner MINRES with the element fast-diagonalisation |A|^-1 "
+    "mixed_fdm": ("mixed", 1e-4, 2, 1.0, "FP32-inner CG (complex symmetric) with the element fast-diagonalisation "
                                          "preconditioner in FP64 iterative refinement, zero stage guess"),
-    "mixed_fdm_extrap": ("mixed", 1e-4, 2, 1.0, "FP32-inner MINRES with the element fast-diagonalisation "
+    "mixed_fdm_extrap": ("mixed", 1e-4, 2, 1.0, "FP32-inner CG (complex symmetric) with the element fast-diagonalisation "
                                                 "preconditioner in FP64 iterative refinement, extrapolated stage "
                                                 "guess (test relative to |b|)"),
-    "mixed_fdm_extrap2": ("mixed", 1e-4, 2, 1.0, "FP32-inner MINRES with the element fast-diagonalisation "
+    "mixed_fdm_extrap2": ("mixed", 1e-4, 2, 1.0, "FP32-inner CG (complex symmetric) with the element fast-diagonalisation "
                                                  "preconditioner in FP64 iterative refinement, stage guess "
                                                  "extrapolated quadratically from the last three steps"),
-    "mixed_fdm_learned": ("mixed", 1e-4, 2, 1.0, "FP32-inner MINRES with the element fast-diagonalisation "
+    "mixed_fdm_learned": ("mixed", 1e-4, 2, 1.0, "FP32-inner CG (complex symmetric) with the element fast-diagonalisation "
                                                  "preconditioner in FP64 iterative refinement, stage guess = "
                                                  "linear extrapolation corrected by the BF16 network (trained on "
                                                  "the GPU on stage solves of other initial packets), "
                                                  "residual-minimising step"),
-    "mixed_fdm_proj": ("mixed", 1e-4, 2, 1.0, "FP32-inner MINRES with the element fast-diagonalisation "
+    "mixed_fdm_proj": ("mixed", 1e-4, 2, 1.0, "FP32-inner CG (complex symmetric) with the element fast-diagonalisation "
                                               "preconditioner in FP64 iterative refinement, stage guess = "
                                               "residual-minimising projection onto the last 16 stage solutions "
                                               "(Fischer's successive right-hand sides)"),
-    "mixed_fdm_proj_learned": ("mixed", 1e-4, 2, 1.0, "FP32-inner MINRES with the element fast-diagonalisation "
+    "mixed_fdm_proj_learned": ("mixed", 1e-4, 2, 1.0, "FP32-inner CG (complex symmetric) with the element fast-diagonalisation "
                                                       "preconditioner in FP64 iterative refinement, stage guess = "
                                                       "projection onto the last 16 stage solutions corrected by "
                                                       "the BF16 network (trained on the GPU on stage solves of "
@@ -894,20 +893,20 @@ def run_ours(args):
     sweep = sweep_leg(S, torch, hbm_peak, fp64_peak) if not args.no_sweep else None
     # algorithmic bytes of the dominant kernel (the persistent solver): per
     # Krylov iteration one Res apply (9 words/node) + 13 two-plane vector
-    # words (16 with the element preconditioner: its local solve reads y, r2
-    # and writes y and the local result; the apply pass reads that, writes z
-    # and reads y for beta; Phase B reads z instead of r2 and the previous z
-    # instead of r1); per FP64 refinement sweep one FP64 residual (apply + 5
-    # words)
+    # words (8 for the conjugate gradients with the element preconditioner:
+    # x and r read and written, p written, z written and read, A p read; the
+    # apply counts p in and A p out); per FP64 refinement sweep one FP64
+    # residual (apply + 5 words)
     n = ctx.n
     b64 = n * 8 * (9 + 26)
-    b32 = n * 4 * (9 + (32 if FORMS[head][2] == 2 else 26))
+    b32 = n * 4 * (9 + (16 if FORMS[head][2] == 2 else 26))
     sweeps_total = H["applies64"] if prec == "mixed" else 0
     alg_bytes = H["it64"] * b64 + H["it32"] * b32 + sweeps_total * n * 8 * 14
     achieved = alg_bytes / (H["solver_ms"] / 1e3) / 1e9 if H["solver_ms"] > 0 else None
     resident = H["resident_launches"] > 0
-    kern = ("k_minres_resident<9>" if resident else "k_minres_mixed<9,RES>") if prec == "mixed" \
-        else "k_minres<9,double,RES>"
+    kern = ("k_resident<9>" if resident else "k_cg_mixed<9>" if FORMS[head][2] == 2 else "k_minres_mixed<9,RES>") \
+        if prec == "mixed" \
+        else "k_minres64r<9,RES>"
     it_total = H["it32"] + H["it64"]
     us_per_it = 1e3 * H["solver_ms"] / it_total if it_total else None
     forms_out = {f: {"s_per_step": r["ms"] / 1e3, "minres_tol": r["tol"],
@@ -941,8 +940,8 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                      "frac": (achieved / hbm_peak) if achieved else None,
                      "traffic": SOLVER_DRAM_BYTES_PER_LAUNCH if resident else None,
-                     "traffic_source": "ncu capture of the timed steps' solver launches (constant in this file, "
-                                       "profiles/k_minres_resident_64x64_p8.md)",
+                     "traffic_source": "ncu capture of one stage solve (constant in this file, "
+                                       "profiles/k_resident_64x64_p8.md)",
                      "algorithmic_bytes_per_launch": alg_bytes / max(1, H["solver_launches"]),
                      "launches": H["solver_launches"],
                      "kernel": kern + " (persistent cooperative solver)",

@@ -72,9 +72,12 @@ enum sem_option {
                                     SEM_PRECOND_DIAG (diagonal of |A|) or SEM_PRECOND_FDM
                                     (Schroedinger Res only: per-element |A_e|^-1 by fast
                                     diagonalisation of the element's rectangle approximation,
-                                    summed over elements with 1/multiplicity weights); the
-                                    FP64 outer test on the true residual is unchanged */
-    SEM_OPT_INNER_ITERATION = 8, /* FP32 inner MINRES iteration for Res: 1 (default) one grid
+                                    summed over elements with 1/multiplicity weights; the
+                                    inner iteration is then conjugate gradients on the complex
+                                    form (M + i a L) w = b0 + i b1, which needs a fifth of the
+                                    iterations, with MINRES taking over when it breaks down);
+                                    the FP64 outer test on the true residual is unchanged */
+    SEM_OPT_INNER_ITERATION = 8, /* FP32 inner MINRES iteration for Res (without SEM_PRECOND_FDM): 1 (default) one grid
                                     barrier per iteration (operator product carried by
                                     recurrence), 0 the two-barrier form of the FP64 solver */
     SEM_OPT_REFINE_TOL_SCALE = 9, /* mixed mode stops at |r| < s (tol |r0| + tol), s in (0,1],
@@ -99,7 +102,7 @@ enum sem_option {
                                     FP32 inner solve's vectors on chip (shared memory and
                                     registers; only element-ring copies are exchanged through
                                     global memory) when each SM's share of the mesh fits
-                                    (p = 4, 6, 8, 10; up to 31 elements per SM at p = 8);
+                                    (p = 4, 6, 8, 10; about 50 elements per SM at p = 8);
                                     0 always the staged kernel.  Same FP64 stopping test */
     SEM_OPT_EXTRAP_ORDER = 11,   /* stage guess of SEM_GUESS_EXTRAPOLATE / _LEARNED: 1 (default)
                                     linear 2 z1 - z2, 2 quadratic 3 z1 - 3 z2 + z3 once three

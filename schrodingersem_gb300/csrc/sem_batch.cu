@@ -2,9 +2,8 @@
 // mesh, degree, potential and state) advanced by BDF2 together.  No
 // counterpart in the reference, whose drivers step one mesh
 // (include/openmp_impl/schrodinger.hpp:22-128); each instance follows that
-// driver exactly, with the stage solve of the library's mixed-precision
-// MINRES (FP32 inner iterations, FP64 refinement judged on the true
-// residual).
+// driver exactly, with the library's mixed-precision stage solve (FP32 inner
+// iterations, FP64 refinement judged on the true residual).
 //
 // Execution: see sem_batch.cuh.
 #include <cuda_runtime.h>

@@ -2,9 +2,8 @@
 // mesh, degree, potential and state) advanced by BDF2 together.  No
 // counterpart in the reference, whose drivers step one mesh
 // (include/openmp_impl/schrodinger.hpp:22-128); each instance follows that
-// driver exactly, with the stage solve of the library's mixed-precision
-// MINRES (FP32 inner iterations, FP64 refinement judged on the true
-// residual).
+// driver exactly, with the library's mixed-precision stage solve (FP32 inner
+// iterations, FP64 refinement judged on the true residual).
 //
 // Execution: one persistent launch per time step and group of instances (same
 // degree and cluster size) on forked streams.  A cluster of 1, 2, 4 or 8 blocks
@@ -34,8 +33,9 @@ constexpr int BATCH_MIN_N = 3;  // p = 2
 constexpr int BATCH_MAX_N = 9;  // p = 8
 constexpr size_t BATCH_SMEM_BUDGET = 108 * 1024;  // two blocks per SM
 // blocks that share an instance of this many element-local nodes: at least 2,048
-// nodes each.  Measured on 160 instances of 4^2..32^2 elements, p = 4, 6, 8, two
-// steps (the largest has 83 k nodes): see the figures at k_batch_bdf2
+// nodes each.  Two steps of 160 instances of 4^2..32^2 elements, p = 4, 6, 8 (the
+// largest has 83 k nodes) take 24.8 ms, with one block per instance 152 ms: there
+// the largest instance sets the time
 inline int batch_cluster(long long nodes) { return nodes >= 16384 ? 8 : nodes >= 8192 ? 4 : nodes >= 4096 ? 2 : 1; }
 
 struct BatchInst {

@@ -165,7 +165,7 @@ struct SolveArgs {
 };
 
 // Mixed-precision refinement: FP64 true residual and solution, FP32 inner
-// MINRES (see k_minres_mixed).
+// solve (see k_cg_mixed, k_minres_mixed).
 struct MixedArgs {
     double inner_tol;
     int max_sweeps;

@@ -1,7 +1,7 @@
 // Instantiations of the on-chip resident inner solver (sem_resident.cuh) for
 // the odd N (even degrees p = 4, 6, 8, 10): odd line strides keep the line
 // passes free of shared-memory bank conflicts.  Other degrees use the staged
-// kernel (k_minres_mixed).
+// kernel (k_cg_mixed).
 #include "sem_resident.cuh"
 
 namespace semgb {

@@ -1,6 +1,7 @@
-// Persistent (cooperative) Krylov solvers: MINRES (FP64 or FP32), PCG, and
-// FP64 iterative refinement around an FP32 inner MINRES.  One block per SM,
-// SOLVER_TPB threads; each block owns a contiguous element range and stages
+// Persistent (cooperative) FP64 iterative refinement around an FP32 inner solve:
+// MINRES, or the conjugate gradients of sem_cg.cuh with the element
+// preconditioner (k_cg_mixed, its own block shape).  One block per SM, SOLVER_TPB
+// threads; each block owns a contiguous element range and stages
 // up to kmax of its elements per pass in dynamic shared memory
 // (apply_range).  Grid-wide phases are separated by bounded grid barriers.
 //
