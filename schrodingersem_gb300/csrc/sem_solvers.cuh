@@ -993,7 +993,9 @@ constexpr int cg_pass()
 // fills with a pass each (a block alternates between loading a pass and the
 // line contractions behind block barriers, so only other blocks of the SM hide
 // its memory latency), and the largest staging capacities
-// kmax <= the block's element count that fit smem_budget bytes per SM.
+// kmax <= the block's element count that fit smem_budget bytes per SM and,
+// together with the kernel's own static arrays (4,224 bytes of k_pcg64, 2,176 of
+// k_minres64), the device's limit per block.
 // Returns the grid, or 0 on failure (for SOLVE_FP64_RES also when the block's
 // elements do not fit in one pass).
 template <int N>
@@ -1002,12 +1004,22 @@ int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_
 {
     const bool fdm = kind == SOLVE_MIXED_FDM;
     const bool f64 = kind == SOLVE_FP64 || kind == SOLVE_FP64_RES;
+    const void* fn = solver_fn<N>(op, kind);
+    int dev = 0, optin = 0;
+    cudaFuncAttributes at{};
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
+        cudaGetLastError();  // the caller reports the failure; later calls start clean
+        return 0;
+    }
     int per = 1;
     if (fdm) {
         per = E / (sms * cg_pass<N>());
         per = per < 1 ? 1 : per > CG_BLOCKS ? CG_BLOCKS : per;
         smem_budget = smem_budget / CG_BLOCKS;
     }
+    smem_budget = std::min(smem_budget, (size_t)optin - at.sharedSizeBytes);
     if (f64 && sms > 32 * K64_MAXQ) sms = 32 * K64_MAXQ;
     int grid = E < per * sms ? E : per * sms;
     if (grid < 1) grid = 1;
@@ -1027,13 +1039,14 @@ int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_
         const size_t s64 = range_smem_bytes<N, double, OP_RES>(kmax64);
         if (s64 > smem) smem = s64;
     }
-    const void* fn = solver_fn<N>(op, kind);
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : f64 ? k64_tpb(N) : SOLVER_TPB,
-                                                      smem) != cudaSuccess ||
-        per_sm < 1)
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : f64 ? k64_tpb(N) : SOLVER_TPB,
+                                                      smem) != cudaSuccess) {
+        cudaGetLastError();
         return 0;
+    }
+    if (per_sm < 1) return 0;
     if (grid > per_sm * sms) {  // fewer blocks per SM: the passes cover the rest
         grid = per_sm * sms;
     }
