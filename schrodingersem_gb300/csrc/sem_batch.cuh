@@ -223,6 +223,9 @@ __global__ void __launch_bounds__(BATCH_TPB_PLAIN, 1)
     __shared__ unsigned long long next;
     BatchInst& I = *reinterpret_cast<BatchInst*>(ibuf);
     Team tm{nullptr, 0, nullptr, 0, cluster_rank(), cluster_size()};
+    // a block's shared memory may be written by another one only once the block
+    // is known to run: the barrier comes before rank 0's first store
+    team_barrier<TEAM_CLUSTER>(tm);
     for (;;) {
         if (tm.rank == 0 && threadIdx.x == 0) {
             const int q = atomicAdd(ba.queue, 1);
