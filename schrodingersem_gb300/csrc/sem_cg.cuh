@@ -36,10 +36,15 @@ namespace semgb {
 // The blocks that solve one mesh together: a cooperative grid (one mesh), or a
 // thread-block cluster (one instance of a batch; a cluster of one is a block).
 enum TeamKind : int { TEAM_GRID = 0, TEAM_CLUSTER = 1 };
+// words a block publishes in one reduction, at most: the slots lie this far apart
+// for every reduction, whatever it publishes, so that the words of one slot are
+// never those of the other (a fast block writes the next slot while a slow one
+// still reads this one)
+constexpr int TEAM_WORDS = 3;
 struct Team {
     GridSync* gs;      // grid
     long long tmo;
-    double* partials;  // grid: [slot][K][grid] partial sums
+    double* partials;  // grid: [slot][TEAM_WORDS][grid] partial sums
     int slot;          // alternates
     int rank, size;
 };
@@ -119,7 +124,8 @@ __device__ __forceinline__ bool team_sum(const float (&v)[K], Team& tm, float (&
     const int slot = tm.slot;
     tm.slot ^= 1;
     const int G = gridDim.x;
-    f2_t* p = (f2_t*)tm.partials + (size_t)slot * K * G;
+    static_assert(K <= TEAM_WORDS, "words per slot");
+    f2_t* p = (f2_t*)tm.partials + (size_t)slot * TEAM_WORDS * G;
     if (wid == 0) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
@@ -192,7 +198,7 @@ __device__ __forceinline__ bool team_sum64(double v0, double v1, Team& tm, doubl
     const int slot = tm.slot;
     tm.slot ^= 1;
     const int G = gridDim.x;
-    double* p = tm.partials + (size_t)slot * 2 * G;
+    double* p = tm.partials + (size_t)slot * TEAM_WORDS * G;
     if (wid == 0) {
         v0 = lane < nw ? ts[0][lane] : 0.0;
         v1 = lane < nw ? ts[1][lane] : 0.0;
