@@ -536,6 +536,10 @@ __global__ void __launch_bounds__(k64_tpb(N), 1)
     }
 }
 
+// square of the stopping threshold tol |b| (pcg.hpp:84): a tolerance that is not
+// positive is met by no residual, as it is before squaring
+__device__ __forceinline__ double pcg64_threshold(double tol, double b2) { return tol > 0.0 ? tol * tol * b2 : 0.0; }
+
 // PCG on the Poisson operator (pcg.hpp:59-97, identity preconditioner)
 template <int N>
 __global__ void __launch_bounds__(k64_tpb(N), 1)
@@ -588,7 +592,7 @@ __global__ void __launch_bounds__(k64_tpb(N), 1)
     }
     k64_arrive<2>(v2, sy, part);
     if (!k64_wait<2>(sy, [&](const double (&s)[2]) {
-            thr2 = a.tol * a.tol * s[0];
+            thr2 = pcg64_threshold(a.tol, s[0]);
             rho = s[1];
             rho_prev = 0.0;
             be = 0.0;
@@ -912,7 +916,7 @@ __global__ void __launch_bounds__(k64_tpb(N), 1)
     }
     k64_arrive<2>(v2, sy, part);
     if (!k64_wait<2>(sy, [&](const double (&s)[2]) {
-            thr2 = a.tol * a.tol * s[0];
+            thr2 = pcg64_threshold(a.tol, s[0]);
             rho = s[1];
             rho_prev = 0.0;
             be = 0.0;
