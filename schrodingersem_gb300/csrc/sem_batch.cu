@@ -236,15 +236,12 @@ extern "C" int sem_batch_create(sem_batch** out, int n_inst, const int* p, const
             }
             return cudaSuccess;
         });
-        // one opt-in per kernel: the largest of its groups
-        size_t opt = 0;
-        for (const BatchGroup& h : b->groups)
-            if (h.N == g.N) opt = std::max(opt, h.smem);
         if (e == cudaSuccess)
-            e = dispatch_batch_n(g.N, [&](auto nv) { return batch_prepare<decltype(nv)::value>(opt, true, &per_sm); });
+            e = dispatch_batch_n(g.N,
+                                 [&](auto nv) { return batch_prepare<decltype(nv)::value>(g.smem, true, &per_sm); });
         if (e == cudaSuccess)
             e = dispatch_batch_n(
-                g.N, [&](auto nv) { return batch_prepare<decltype(nv)::value>(opt, false, &per_sm_plain); });
+                g.N, [&](auto nv) { return batch_prepare<decltype(nv)::value>(g.smem, false, &per_sm_plain); });
         if (e != cudaSuccess || per_sm < 1 || per_sm_plain < 1) {
             sem_batch_destroy(b);
             return bfail(SEM_ERR_CUDA, "batched step kernel does not fit");
@@ -359,7 +356,7 @@ static int capture_step(sem_batch* b, const BatchArgs& base)
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        cudaEventRecord(b->fork_ev, cs);
+        cudaError_t le = cudaEventRecord(b->fork_ev, cs);
         for (BatchGroup& gr : b->groups) {
             cudaStreamWaitEvent(gr.fork, b->fork_ev, 0);
             BatchArgs ba = base;
@@ -367,15 +364,20 @@ static int capture_step(sem_batch* b, const BatchArgs& base)
             ba.n = (int)gr.members.size();
             ba.queue = gr.d_queue;
             cudaMemsetAsync(gr.d_queue, 0, sizeof(int), gr.fork);
-            dispatch_batch_n(gr.N, [&](auto nv) {
+            const cudaError_t ke = dispatch_batch_n(gr.N, [&](auto nv) {
                 return batch_launch_step<decltype(nv)::value>(ba, ctx_mesh(b->ctx[gr.members[0]]),
                                                                ba.fdm ? gr.grid : gr.grid_plain,
                                                                ba.fdm ? gr.cluster : 1, gr.smem, gr.fork);
             });
+            if (le == cudaSuccess) le = ke;
             cudaEventRecord(gr.done, gr.fork);
             cudaStreamWaitEvent(cs, gr.done, 0);
         }
         e = cudaStreamEndCapture(cs, &g);
+        if (le != cudaSuccess) {  // the capture's own error says less
+            cudaGetLastError();
+            e = le;
+        }
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph, g, 0);
     if (g) cudaGraphDestroy(g);

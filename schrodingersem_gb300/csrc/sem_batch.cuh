@@ -266,8 +266,8 @@ size_t batch_smem_n(int kmax, int kmax64)
 template <int N>
 cudaError_t batch_prepare(size_t smem, bool fdm, int* per_sm)
 {
-    cudaError_t e = cudaFuncSetAttribute(k_batch_bdf2<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    size_t limit = 0;
+    if (!smem_opt_in_all((const void*)k_batch_bdf2<N>, &limit) || smem > limit) return cudaErrorInvalidConfiguration;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_batch_bdf2<N>, fdm ? BATCH_TPB : BATCH_TPB_PLAIN,
                                                          smem);
 }

@@ -798,8 +798,8 @@ cudaError_t launch_resident(const DevMesh& m, const SolveArgs& a, const KrylovWo
     if (!m.Dh || !m.Sh) return cudaErrorInvalidValue;
     // a per-device function attribute: set on every launch (cheap), so a
     // context on any device of the process gets the opt-in
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    size_t limit = 0;
+    if (!smem_opt_in_all(fn, &limit) || smem > limit) return cudaErrorInvalidConfiguration;
     DevMesh mm = m;
     SolveArgs aa = a;
     KrylovWork<float> ww = w;

@@ -981,6 +981,28 @@ inline int k64_threads(int N, int nc, int share)
     return v >= top ? top : v < 128 ? 128 : (v + 31) / 32 * 32;
 }
 
+// Opts a kernel in to all the dynamic shared memory that a block may have beside
+// its static arrays (*limit, bytes).  The attribute belongs to the kernel and the
+// device, not to a context, so it is never set to what one plan needs: another
+// context's plan for the same kernel may come between a plan and its launch (from
+// another thread, or before an ensemble's step is captured), and lowering it would
+// have that launch refused.
+inline bool smem_opt_in_all(const void* fn, size_t* limit)
+{
+    int dev = 0, optin = 0;
+    cudaFuncAttributes at{};
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncGetAttributes(&at, fn) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)at.sharedSizeBytes) !=
+            cudaSuccess) {
+        cudaGetLastError();  // the caller reports the failure; later calls start clean
+        return false;
+    }
+    *limit = (size_t)optin - at.sharedSizeBytes;
+    return true;
+}
+
 // elements of one element-preconditioned pass: one line per thread
 template <int N>
 constexpr int cg_pass()
@@ -1005,21 +1027,15 @@ int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_
     const bool fdm = kind == SOLVE_MIXED_FDM;
     const bool f64 = kind == SOLVE_FP64 || kind == SOLVE_FP64_RES;
     const void* fn = solver_fn<N>(op, kind);
-    int dev = 0, optin = 0;
-    cudaFuncAttributes at{};
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
-        cudaGetLastError();  // the caller reports the failure; later calls start clean
-        return 0;
-    }
+    size_t limit = 0;
+    if (!smem_opt_in_all(fn, &limit)) return 0;
     int per = 1;
     if (fdm) {
         per = E / (sms * cg_pass<N>());
         per = per < 1 ? 1 : per > CG_BLOCKS ? CG_BLOCKS : per;
         smem_budget = smem_budget / CG_BLOCKS;
     }
-    smem_budget = std::min(smem_budget, (size_t)optin - at.sharedSizeBytes);
+    smem_budget = std::min(smem_budget, limit);
     if (f64 && sms > 32 * K64_MAXQ) sms = 32 * K64_MAXQ;
     int grid = E < per * sms ? E : per * sms;
     if (grid < 1) grid = 1;
@@ -1040,8 +1056,7 @@ int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_
         if (s64 > smem) smem = s64;
     }
     int per_sm = 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : f64 ? k64_tpb(N) : SOLVER_TPB,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : f64 ? k64_tpb(N) : SOLVER_TPB,
                                                       smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
