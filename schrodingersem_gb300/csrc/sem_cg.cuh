@@ -477,21 +477,38 @@ struct CgScal {
     float best;        // smallest |r|^2 so far and the iteration that gave it
     int best_it;
 };
+// the power of two that brings the larger of |a|, |b| to [1, 2).  The quotients
+// below divide by |d|^2; the inner products carry the unit of length (an element's
+// measure to the power -1) and |r|^2, and their squares left FP32's range for
+// element sides above some 1e4 or below 1e-8.  Scaling by powers of two changes
+// no bit of a quotient whose squares did stay in it.
+__device__ __forceinline__ float cg_scale(float a, float b)
+{
+    const int e = (__float_as_int(fmaxf(fabsf(a), fabsf(b))) >> 23) & 255;
+    return __int_as_float(max(254 - e, 1) << 23);
+}
 // a = rho / (p.Ap); false when it is not a finite number
 __device__ __forceinline__ bool cg_step(CgScal& s, float d0, float d1)
 {
+    const float c = cg_scale(d0, d1);
+    d0 *= c;
+    d1 *= c;
+    const float r0 = s.rho0 * c, r1 = s.rho1 * c;
     const float den = fmaf(d0, d0, d1 * d1);
     const float inv = 1.f / den;
-    s.a0 = fmaf(s.rho0, d0, s.rho1 * d1) * inv;
-    s.a1 = fmaf(s.rho1, d0, -s.rho0 * d1) * inv;
+    s.a0 = fmaf(r0, d0, r1 * d1) * inv;
+    s.a1 = fmaf(r1, d0, -r0 * d1) * inv;
     return isfinite(s.a0) && isfinite(s.a1);
 }
+// beta = r.z / rho, rho = r.z
 __device__ __forceinline__ bool cg_beta(CgScal& s, float r0, float r1)
 {
-    const float den = fmaf(s.rho0, s.rho0, s.rho1 * s.rho1);
+    const float c = cg_scale(s.rho0, s.rho1);
+    const float d0 = s.rho0 * c, d1 = s.rho1 * c, q0 = r0 * c, q1 = r1 * c;
+    const float den = fmaf(d0, d0, d1 * d1);
     const float inv = 1.f / den;
-    s.b0 = fmaf(r0, s.rho0, r1 * s.rho1) * inv;
-    s.b1 = fmaf(r1, s.rho0, -r0 * s.rho1) * inv;
+    s.b0 = fmaf(q0, d0, q1 * d1) * inv;
+    s.b1 = fmaf(q1, d0, -q0 * d1) * inv;
     s.rho0 = r0;
     s.rho1 = r1;
     return isfinite(s.b0) && isfinite(s.b1);
