@@ -174,6 +174,7 @@ __device__ void bdf2_instance(const BatchInst& I, const BatchArgs& ba, unsigned 
         done = r.inner;
         minres = r.fallback;
         a.maxit -= done;
+        mx.max_sweeps -= r.sweeps;
         a.r0_given = r.r0;
         if (tm.rank == 0 && threadIdx.x == 0) {
             I.out->success = r.conv ? 1 : 0;

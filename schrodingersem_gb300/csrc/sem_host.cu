@@ -1637,6 +1637,7 @@ static int run_mixed(sem_ctx* c, int op, const double* pot, double alpha, double
         done_sweeps = *sweeps;
         resident = false;
         mx.minres = 1;
+        mx.max_sweeps = c->max_refine - done_sweeps;
         a.x_is_zero = 0;
         a.r0_given = c->h_out->r0;
         a.maxit = maxit - done_it;
