@@ -519,6 +519,17 @@ __device__ __forceinline__ bool cg_beta(CgScal& s, float r0, float r1)
 // large); about 2.5 of 35 iterations
 constexpr double CG_MARGIN = 0.1;
 constexpr int CG_STALL = 200;  // iterations without a smaller residual: give up (MINRES takes over)
+// Whether a sweep left so much of the true residual that MINRES should take over:
+// more than halfway between its inner tolerance and one.  Once a sweep of the
+// solve has reduced it tenfold the iteration is sound on this operator, and a
+// later one that does not has met the rounding of the FP64 residual, which stops
+// MINRES as well and costs it more (64 x 64, p = 8, tol = 1e-16, out of reach:
+// 57 ms with MINRES taking over there)
+__device__ __forceinline__ bool cg_sweep_failed(double rn, double last_rn, double last_itol, bool& sound)
+{
+    sound = sound || rn < 0.1 * last_rn;
+    return !sound && !(rn < 0.5 * (1.0 + last_itol) * last_rn);
+}
 
 struct CgOut {
     int it;
@@ -745,7 +756,7 @@ __device__ __forceinline__ bool cg_core(unsigned char* smraw, int kmax, const De
 // |r| < scale (tol |r0| + tol) (the reference's criterion, minres.hpp:92; with
 // rel_to_b |b| in the place of |r0|); else solve A d = r to the inner tolerance
 // and add d to x on owner copies.  res.fallback: the inner iteration broke
-// down, stalled or did not halve the true residual, and MINRES should go on
+// down, stalled or hardly reduced the true residual, and MINRES should go on
 // from x.  Returns false when a wait timed out.
 struct CgRefine {
     int sweeps, inner;
@@ -770,7 +781,8 @@ __device__ __forceinline__ bool cg_refine(const DevMesh& m, const SolveArgs& a, 
     f2_t* const X = (f2_t*)mx.x32[0];
     res.sweeps = res.inner = 0;
     res.conv = res.fallback = false;
-    double last_rn = 0.0;
+    double last_rn = 0.0, itol = 0.0;
+    bool sound = false;
     for (int l = threadIdx.x; l < N; l += blockDim.x) lam[l] = m.fdmL32[l];
     for (;;) {
         const bool applied = res.sweeps > 0 || !a.x_is_zero;
@@ -821,7 +833,7 @@ __device__ __forceinline__ bool cg_refine(const DevMesh& m, const SolveArgs& a, 
         const double thr = mx.outer_scale * (a.tol * res.r0 + a.tol);
         res.conv = rn < thr;
         if (res.conv || res.sweeps >= mx.max_sweeps || res.inner >= a.maxit || !(rn == rn)) return true;
-        if (res.sweeps > 0 && !(rn < 0.5 * last_rn)) {
+        if (res.sweeps > 0 && cg_sweep_failed(rn, last_rn, itol, sound)) {
             res.fallback = true;
             return true;
         }
@@ -829,7 +841,7 @@ __device__ __forceinline__ bool cg_refine(const DevMesh& m, const SolveArgs& a, 
         // the inner solve reduces by inner_tol, or (last sweep) by CG_MARGIN of
         // what the outer test still needs: a good initial guess then saves
         // iterations, not sweeps
-        double itol = mx.inner_tol;
+        itol = mx.inner_tol;
         if (mx.adaptive) itol = fmax(itol, fmin(CG_MARGIN * thr / rn, 0.5));
         const double inv = 1.0 / rn;
         const double* r64a = mx.r64[0];

@@ -618,7 +618,7 @@ __device__ __forceinline__ bool res_inner(const DevMesh& m, const CgTab<N>& tab,
 // ------------------------------------------------------------------ kernel
 // FP64 iterative refinement (the sweep of mixed_solve: true residual
 // r = b - A x, the reference's stopping test on |r|) around res_inner.  When
-// the inner iteration breaks down, stalls or fails to halve the true residual
+// the inner iteration breaks down, stalls or hardly reduces the true residual
 // the kernel ends with SolveOut::fallback set and the host continues on the
 // staged kernel with MINRES.
 // bytes of the FP64 staging area and, at least, of p, q and z (a multiple of 16)
@@ -657,7 +657,8 @@ __global__ void __launch_bounds__(RES_TPB, 1)
     bool ok = true;
     int sweep = 0, inner_total = 0;
     bool conv = false, fallback = false;
-    double last_rn = 0.0;
+    double last_rn = 0.0, itol = 0.0;
+    bool sound = false;
     for (;;) {
         // ---- FP64 residual r = unmask(b) - DSS(A_local(unmask(x)))
         const bool applied = (sweep > 0) || !a.x_is_zero;
@@ -721,17 +722,17 @@ __global__ void __launch_bounds__(RES_TPB, 1)
         }
         // ---- FP32 inner solve A d = r on chip; x += d
         const int budget = min(mx.inner_maxit, a.maxit - inner_total);
-        double itol = mx.inner_tol;
-        if (mx.adaptive) {
-            const double need = mx.outer_scale * (a.tol * sweep_state[0] + a.tol) / sweep_state[1];
-            itol = fmax(itol, fmin(CG_MARGIN * need, 0.5));
-        }
         const double rn = sweep_state[1];
-        if (sweep > 0 && !(rn < 0.5 * last_rn)) {
+        if (sweep > 0 && cg_sweep_failed(rn, last_rn, itol, sound)) {
             fallback = true;
             break;
         }
         last_rn = rn;
+        itol = mx.inner_tol;
+        if (mx.adaptive) {
+            const double need = mx.outer_scale * (a.tol * sweep_state[0] + a.tol) / sweep_state[1];
+            itol = fmax(itol, fmin(CG_MARGIN * need, 0.5));
+        }
         const double* r64c[2] = {mx.r64[0], mx.r64[1]};
         CgOut ir{};
         if (!res_inner<N, RW>(m, tab, s, eb, ne, r64c, rn, alpha32, ra, epoch, a.sync, a.timeout_ns, redf, tot, budget,
