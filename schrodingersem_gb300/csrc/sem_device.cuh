@@ -901,68 +901,6 @@ __device__ __forceinline__ bool grid_barrier(GridSync* gs, long long timeout_ns)
     return *((volatile int*)&gs->err) == 0;
 }
 
-// all-reduce of one double across the grid: block sums to partials[slot][blk],
-// barrier, then every block sums the partials in the same fixed order.
-__device__ __forceinline__ double grid_sum(double v, double* partials, int slot, GridSync* gs,
-                                           long long timeout_ns, double* red, bool& ok)
-{
-    const double bs = block_sum(v, red);
-    const int G = gridDim.x;
-    // same slot layout as grid_sum2 ([slot][2][grid]) so that consecutive
-    // reductions (alternating slots) never share partial-sum words
-    double* p = partials + (size_t)(2 * slot) * G;
-    if (threadIdx.x == 0) p[blockIdx.x] = bs;
-    ok = grid_barrier(gs, timeout_ns);
-    if (threadIdx.x < 32) {
-        double s = 0.0;
-        for (int q = threadIdx.x; q < G; q += 32) s += __ldcg(p + q);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) red[33] = s;
-    }
-    __syncthreads();
-    const double r = red[33];
-    __syncthreads();
-    return r;
-}
-
-// all-reduce of two doubles behind a single grid barrier; partials laid out
-// [slot][2][grid] (the buffer holds 2 slots x 2 values x grid)
-__device__ __forceinline__ void grid_sum2(double v0, double v1, double* partials, int slot, GridSync* gs,
-                                          long long timeout_ns, double* red, bool& ok, double& r0, double& r1)
-{
-    const double b0 = block_sum(v0, red);
-    const double b1 = block_sum(v1, red);
-    const int G = gridDim.x;
-    double* p0 = partials + (size_t)(slot * 2) * G;
-    double* p1 = p0 + G;
-    if (threadIdx.x == 0) {
-        p0[blockIdx.x] = b0;
-        p1[blockIdx.x] = b1;
-    }
-    ok = grid_barrier(gs, timeout_ns);
-    if (threadIdx.x < 32) {
-        double s0 = 0.0, s1 = 0.0;
-        for (int q = threadIdx.x; q < G; q += 32) {
-            s0 += __ldcg(p0 + q);
-            s1 += __ldcg(p1 + q);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        }
-        if (threadIdx.x == 0) {
-            red[33] = s0;
-            red[32] = s1;
-        }
-    }
-    __syncthreads();
-    r0 = red[33];
-    r1 = red[32];
-    __syncthreads();
-}
-
 __device__ __forceinline__ void block_range(int E, int& eb, int& ee)
 {
     const int G = gridDim.x;

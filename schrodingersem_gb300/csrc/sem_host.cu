@@ -1450,7 +1450,6 @@ static int krylov_work(sem_ctx* c, int nc, KrylovWork<double>* w, GridSync** syn
     }
     for (int k = 0; k < 2; ++k)
         if ((s = wsget(c, yn[k], v, &w->Y[k]))) return s;
-    if ((s = wsget(c, "kr_part", 2 * 152 * 64, &w->partials))) return s;
     if ((s = wsget(c, "kr_slots", kSlotWords, &w->slots))) return s;
     if ((s = wsget(c, "kr_sync", 1, sync))) return s;
     if ((s = wsget(c, "kr_out", 1, out))) return s;

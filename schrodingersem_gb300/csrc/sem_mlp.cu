@@ -6,9 +6,10 @@
 // Model: x (d_in) -> ReLU(x W1 + b1) (H) -> ReLU(. W2 + b2) (H) -> . W3 + b3 (d_out)
 // with row-major activations [rows][features] and weights [in][out].
 //
-// GEMM: C[M][N] = A(M x K) * B(K x N) with generic strides, tiles of 64 x 64
-// staged in shared memory as BF16, computed with mma.sync m16n8k16 (BF16 in,
-// FP32 accumulate); every global access is bounds-checked.
+// GEMM: C[M][N] = A(M x K) * B(K x N), BF16 operands, FP32 accumulation: on the
+// tensor cores by tcgen05 (k_gemm_tc), or (sem_gemm_set_path(0)) with any strides
+// in tiles of 64 x 64 by mma.sync m16n8k16 (k_gemm_bf16).  Every global access is
+// bounds-checked.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -32,13 +33,11 @@ constexpr int GT_M = 64, GT_N = 64, GT_K = 32;
 
 struct GemmArgs {
     int M, N, K;
-    const void* A;
+    const __nv_bfloat16* A;
     long long sa_m, sa_k;  // A(m,k) = A[m*sa_m + k*sa_k]
-    int a_bf16;            // A is __nv_bfloat16 (else float)
-    const void* B;
+    const __nv_bfloat16* B;
     long long sb_k, sb_n;  // B(k,n) = B[k*sb_k + n*sb_n]
     int vec_a, vec_b;      // tcgen05 kernel: load widths (tc_vec; set by gemm())
-    int b_bf16;
     float* C;              // C[m*ldc + n] (FP32)
     int ldc;
     const float* bias;     // optional, length N
@@ -47,11 +46,6 @@ struct GemmArgs {
     int accumulate;        // C += result
     __nv_bfloat16* Cbf;    // optional BF16 copy of the output
 };
-
-__device__ __forceinline__ float ld_any(const void* p, long long i, int bf)
-{
-    return bf ? __bfloat162float(((const __nv_bfloat16*)p)[i]) : ((const float*)p)[i];
-}
 
 __device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi)
 {
@@ -79,14 +73,12 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g)
         for (int t = threadIdx.x; t < GT_M * GT_K; t += blockDim.x) {
             const int r = t / GT_K, c = t - r * GT_K;
             const int m = m0 + r, k = k0 + c;
-            const float v = (m < g.M && k < g.K) ? ld_any(g.A, m * g.sa_m + k * g.sa_k, g.a_bf16) : 0.f;
-            sA[r][c] = __float2bfloat16(v);
+            sA[r][c] = (m < g.M && k < g.K) ? g.A[m * g.sa_m + k * g.sa_k] : __float2bfloat16(0.f);
         }
         for (int t = threadIdx.x; t < GT_N * GT_K; t += blockDim.x) {
             const int r = t / GT_K, c = t - r * GT_K;  // r: n, c: k
             const int n = n0 + r, k = k0 + c;
-            const float v = (n < g.N && k < g.K) ? ld_any(g.B, k * g.sb_k + n * g.sb_n, g.b_bf16) : 0.f;
-            sB[r][c] = __float2bfloat16(v);
+            sB[r][c] = (n < g.N && k < g.K) ? g.B[k * g.sb_k + n * g.sb_n] : __float2bfloat16(0.f);
         }
         __syncthreads();
 #pragma unroll
@@ -145,8 +137,8 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g)
 // The same GEMM on the sm_100-family tensor cores: tcgen05.mma kind::f16
 // (BF16 A and B, FP32 accumulator in tensor memory), M = 128 rows per CTA,
 // N = TC_BN columns, K in steps of 16 from shared-memory operands staged by
-// the CTA's 128 threads (generic strides, FP32 or BF16 sources converted to
-// BF16, zero-filled past the matrix edges) in the canonical K-major layout
+// the CTA's 128 threads (BF16 sources contiguous along K or along their rows,
+// zero-filled past the matrix edges) in the canonical K-major layout
 // without swizzle: 8-row x 16-byte core matrices, the two core matrices of a
 // 16-wide K step 128 bytes apart (leading-dimension offset), consecutive
 // 8-row groups 256 bytes apart (stride-dimension offset).  Two K tiles of 64
@@ -265,10 +257,9 @@ __device__ __forceinline__ void tc_load_v(const __nv_bfloat16* X, bool trans, lo
             if (r0 + i * 16 < rows) tc_chunk_part(p + (long long)(i * 16) * ld, nk, w[i]);
 }
 template <int R>
-__device__ __forceinline__ void tc_load(const void* X, int vec, bool trans, long long ld, int rows, int K, int row0,
+__device__ __forceinline__ void tc_load(const __nv_bfloat16* x, int vec, bool trans, long long ld, int rows, int K, int row0,
                                         int k0, uint32_t (&w)[8][4])
 {
-    const __nv_bfloat16* x = (const __nv_bfloat16*)X;
     if (vec == 16) tc_load_v<R, 16>(x, trans, ld, rows, K, row0, k0, w);
     else if (vec == 8) tc_load_v<R, 8>(x, trans, ld, rows, K, row0, k0, w);
     else if (vec == 4) tc_load_v<R, 4>(x, trans, ld, rows, K, row0, k0, w);
@@ -477,10 +468,10 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(GemmArgs g, long long ti
 
 // ------------------------------------------------ fused forward pass
 // The network's inference pass in one kernel: per CTA 128 rows, the three
-// layers chained through tensor memory and shared memory.  Layer 1 streams
-// its A tile (the BF16 features) and every layer streams its weights
-// (transposed BF16 copies, K contiguous) in 64-wide K chunks through two
-// shared-memory buffers; the hidden activations never leave the SM: the
+// layers chained through tensor memory and shared memory, in 64-wide K chunks.
+// Layer 1 stages its A tile (the BF16 features) through two shared-memory
+// buffers, every layer brings its weights through three (below); the hidden
+// activations never leave the SM: the
 // epilogue of layers 1 and 2 reads the FP32 accumulator with tcgen05.ld,
 // adds the bias, applies ReLU, rounds to BF16 and writes them in the
 // canonical K-major layout as the next layer's A operand (H, all 256 K at
@@ -736,8 +727,8 @@ cudaError_t gemm(const GemmArgs& g0, cudaStream_t st)
         k_gemm_bf16<<<grid, 128, 0, st>>>(g0);
         return cudaGetLastError();
     }
-    // the tensor-core kernel takes BF16 operands with one contiguous direction
-    if (!g0.a_bf16 || !g0.b_bf16 || (g0.sa_m != 1 && g0.sa_k != 1) || (g0.sb_n != 1 && g0.sb_k != 1))
+    // the tensor-core kernel takes operands with one contiguous direction
+    if ((g0.sa_m != 1 && g0.sa_k != 1) || (g0.sb_n != 1 && g0.sb_k != 1))
         return cudaErrorInvalidValue;
     GemmArgs g = g0;
     g.vec_a = tc_vec(g.A, g.sa_k != 1 ? g.sa_k : g.sa_m);
@@ -1071,8 +1062,8 @@ static int forward(sem_learner* L, int rows, const __nv_bfloat16* x)
     // B(k, n) = W[k][n] = WT[n][k]: K contiguous
     GemmArgs g{};
     g.M = rows; g.N = L->H; g.K = L->d_in;
-    g.A = x; g.sa_m = L->d_in; g.sa_k = 1; g.a_bf16 = 1;
-    g.B = L->WbfT[0]; g.sb_k = 1; g.sb_n = L->d_in; g.b_bf16 = 1;
+    g.A = x; g.sa_m = L->d_in; g.sa_k = 1;
+    g.B = L->WbfT[0]; g.sb_k = 1; g.sb_n = L->d_in;
     g.C = L->h1; g.ldc = L->H; g.bias = L->b[0]; g.relu = 1; g.Cbf = L->h1bf;
     LCUDA(gemm(g, L->stream));
     g.K = L->H; g.A = L->h1bf; g.sa_m = L->H;
@@ -1115,36 +1106,36 @@ extern "C" int sem_learner_train_step(sem_learner* L, int rows, const void* x_bf
     // layer 3: gW3 = h2^T dout, gb3 = colsum(dout), d2 = dout W3^T (masked by ReLU)
     GemmArgs g{};
     g.M = L->H; g.N = L->d_out; g.K = rows;
-    g.A = L->h2bf; g.sa_m = 1; g.sa_k = L->H; g.a_bf16 = 1;
-    g.B = L->doutbf; g.sb_k = L->d_out; g.sb_n = 1; g.b_bf16 = 1;
+    g.A = L->h2bf; g.sa_m = 1; g.sa_k = L->H;
+    g.B = L->doutbf; g.sb_k = L->d_out; g.sb_n = 1;
     g.C = L->gW[2]; g.ldc = L->d_out;
     LCUDA(gemm(g, L->stream));
     k_colsum<<<(L->d_out + 31) / 32, 1024, 0, L->stream>>>(rows, L->d_out, L->dout, L->gb[2]);
     g = GemmArgs{};
     g.M = rows; g.N = L->H; g.K = L->d_out;
-    g.A = L->doutbf; g.sa_m = L->d_out; g.sa_k = 1; g.a_bf16 = 1;
-    g.B = L->Wbf[2]; g.sb_k = 1; g.sb_n = L->d_out; g.b_bf16 = 1;
+    g.A = L->doutbf; g.sa_m = L->d_out; g.sa_k = 1;
+    g.B = L->Wbf[2]; g.sb_k = 1; g.sb_n = L->d_out;
     g.C = L->d2; g.ldc = L->H; g.mask = L->h2; g.Cbf = L->d2bf;
     LCUDA(gemm(g, L->stream));
     // layer 2
     g = GemmArgs{};
     g.M = L->H; g.N = L->H; g.K = rows;
-    g.A = L->h1bf; g.sa_m = 1; g.sa_k = L->H; g.a_bf16 = 1;
-    g.B = L->d2bf; g.sb_k = L->H; g.sb_n = 1; g.b_bf16 = 1;
+    g.A = L->h1bf; g.sa_m = 1; g.sa_k = L->H;
+    g.B = L->d2bf; g.sb_k = L->H; g.sb_n = 1;
     g.C = L->gW[1]; g.ldc = L->H;
     LCUDA(gemm(g, L->stream));
     k_colsum<<<(L->H + 31) / 32, 1024, 0, L->stream>>>(rows, L->H, L->d2, L->gb[1]);
     g = GemmArgs{};
     g.M = rows; g.N = L->H; g.K = L->H;
-    g.A = L->d2bf; g.sa_m = L->H; g.sa_k = 1; g.a_bf16 = 1;
-    g.B = L->Wbf[1]; g.sb_k = 1; g.sb_n = L->H; g.b_bf16 = 1;
+    g.A = L->d2bf; g.sa_m = L->H; g.sa_k = 1;
+    g.B = L->Wbf[1]; g.sb_k = 1; g.sb_n = L->H;
     g.C = L->d1; g.ldc = L->H; g.mask = L->h1; g.Cbf = L->d1bf;
     LCUDA(gemm(g, L->stream));
     // layer 1
     g = GemmArgs{};
     g.M = L->d_in; g.N = L->H; g.K = rows;
-    g.A = x; g.sa_m = 1; g.sa_k = L->d_in; g.a_bf16 = 1;
-    g.B = L->d1bf; g.sb_k = L->H; g.sb_n = 1; g.b_bf16 = 1;
+    g.A = x; g.sa_m = 1; g.sa_k = L->d_in;
+    g.B = L->d1bf; g.sb_k = L->H; g.sb_n = 1;
     g.C = L->gW[0]; g.ldc = L->H;
     LCUDA(gemm(g, L->stream));
     k_colsum<<<(L->H + 31) / 32, 1024, 0, L->stream>>>(rows, L->H, L->d1, L->gb[0]);
@@ -1273,8 +1264,8 @@ extern "C" int sem_gemm_bf16(int M, int N, int K, const void* A, const void* B, 
     if (M < 0 || N < 0 || K < 0 || (M && N && K && (!A || !B || !C))) return ctx_fail(SEM_ERR_ARG, "bad gemm");
     GemmArgs g{};
     g.M = M; g.N = N; g.K = K;
-    g.A = A; g.sa_m = K; g.sa_k = 1; g.a_bf16 = 1;
-    g.B = B; g.sb_k = N; g.sb_n = 1; g.b_bf16 = 1;
+    g.A = (const __nv_bfloat16*)A; g.sa_m = K; g.sa_k = 1;
+    g.B = (const __nv_bfloat16*)B; g.sb_k = N; g.sb_n = 1;
     g.C = C; g.ldc = N;
     cudaError_t e = gemm(g, (cudaStream_t)stream);
     if (e != cudaSuccess) return ctx_fail(SEM_ERR_CUDA, cudaGetErrorString(e));

@@ -52,7 +52,8 @@ __device__ __forceinline__ double block_sum_t(T v, double* red)
     return red[32];
 }
 
-// grid all-reduce of up to two T partials (one barrier); see grid_sum2
+// grid all-reduce of up to two T partials behind one barrier: block sums to
+// partials[slot][2][grid], then every block sums them in the same fixed order
 template <typename T>
 __device__ __forceinline__ void grid_sum2_t(T v0, T v1, double* partials, int slot, GridSync* gs, long long tmo,
                                             double* red, bool& ok, double& r0, double& r1)
