@@ -58,10 +58,10 @@ WORKLOAD = ("Schroedinger SDIRK4-3 time step, 64x64 jittered quads on [-8,8]^2 (
 DT, TOL, P, NEL = 1e-2, 1e-10, 8, 64
 ORACLE_TOL = 1e-13  # MINRES tolerance of the FP64 accuracy reference runs
 # DRAM bytes (read + write) per launch of the on-chip resident solver kernel
-# (k_resident<9>): ncu capture of one stage solve, summarised in
-# profiles/k_resident_64x64_p8.md.  The Krylov vectors stay on chip; these
-# bytes are the FP64 refinement's fields and the per-launch loads.
-SOLVER_DRAM_BYTES_PER_LAUNCH = 20.55e6
+# (k_resident<9>), from an ncu capture of one stage solve.  The Krylov vectors
+# stay on chip; these bytes are the FP64 refinement's fields and the per-launch
+# loads.
+SOLVER_DRAM_BYTES_PER_LAUNCH = 39.3e6
 APPLY_NEL = 559  # 559^2 elements at p = 8: 4473^2 = 20.0 M global nodes
 
 
@@ -491,6 +491,17 @@ def measure_apply(ctx, torch, prec, flush, reps, pipeline=1):
     return float(np.median(times))
 
 
+def fp64_apply_ops(N, E):
+    """FP64 instructions per thread of one Res apply as its kernel executes them
+    (csrc/sem_kernels.cuh, lines64: whole lines split by parity where that measured
+    faster, else one thread per node), each one FMA, product or sum: the share of
+    the FP64 pipe is these against half the flops of the measured peak"""
+    H, C, nodes = N // 2, (N + 1) // 2, E * N * N
+    if (N >= 9 and nodes >= 100000) or (N >= 7 and nodes >= 400000):
+        return 2 * (E * N * (8 * H * C + 16 * H + 4 * N) + 4 * nodes)
+    return 2 * nodes * (4 * N + 9)
+
+
 def apply_leg(S, torch, fp64_peak, hbm_peak, reps=20):
     """Res apply on 559x559 jittered quads over [-12,12]^2 at p = 8 (20.0 M
     global nodes, 25.3 M element-local nodes per plane, above L2).
@@ -508,7 +519,8 @@ def apply_leg(S, torch, fp64_peak, hbm_peak, reps=20):
         nb, fl = ctx.n * s * 9, ctx.n * (16 * ctx.N + 23)
         out[prec] = {"ms": ms, "gbs": nb / ms / 1e6, "bytes": nb, "tflops": fl / ms / 1e9, "flops": fl}
     out["fp32"]["frac_hbm"] = out["fp32"]["gbs"] / hbm_peak
-    out["fp64"]["frac_fp64_pipe"] = out["fp64"]["tflops"] / fp64_peak if fp64_peak else None
+    out["fp64"]["frac_fp64_pipe"] = (2 * fp64_apply_ops(ctx.N, ctx.E) / out["fp64"]["ms"] / 1e9 / fp64_peak
+                                     if fp64_peak else None)
     out["fp32_geo"] = geo_row(ctx, measure_apply(ctx, torch, "fp32", flush, reps, pipeline=2), hbm_peak)
     out["fp32_geo"]["speedup_vs_stored_factors"] = out["fp32"]["ms"] / out["fp32_geo"]["ms"]
     ctx.close()
@@ -552,7 +564,8 @@ def sweep_leg(S, torch, hbm_peak, fp64_peak, degrees=range(2, 17), nodes=2e7, re
             else:
                 tf = ctx.n * (16 * ctx.N + 23) / ms / 1e9
                 row[prec]["tflops"] = round(tf, 3)
-                row[prec]["frac_fp64_pipe"] = round(tf / fp64_peak, 4) if fp64_peak else None
+                row[prec]["frac_fp64_pipe"] = (round(2 * fp64_apply_ops(ctx.N, ctx.E) / ms / 1e9 / fp64_peak, 4)
+                                               if fp64_peak else None)
         rows.append(row)
         ctx.close()
         del ctx
@@ -940,8 +953,7 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                      "frac": (achieved / hbm_peak) if achieved else None,
                      "traffic": SOLVER_DRAM_BYTES_PER_LAUNCH if resident else None,
-                     "traffic_source": "ncu capture of one stage solve (constant in this file, "
-                                       "profiles/k_resident_64x64_p8.md)",
+                     "traffic_source": "ncu capture of one stage solve (constant in this file)",
                      "algorithmic_bytes_per_launch": alg_bytes / max(1, H["solver_launches"]),
                      "launches": H["solver_launches"],
                      "kernel": kern + " (persistent cooperative solver)",
@@ -966,7 +978,8 @@ def run_ours(args):
                    "fp64_gbs": app["fp64"]["gbs"], "fp64_tflops": app["fp64"]["tflops"],
                    "fp64_frac_fp64_pipe": app["fp64"]["frac_fp64_pipe"], "fp64_peak_tflops": fp64_peak,
                    "fp64_peak_source": "cuBLAS DGEMM 4096^3 measured in this run",
-                   "detail": app, "note": "n_loc*s*9 algorithmic words and n_loc*(16N+23) flops per apply; "
+                   "detail": app, "note": "n_loc*s*9 algorithmic words and n_loc*(16N+23) flops per apply "
+                                          "(dense contractions; frac_fp64_pipe counts the instructions executed); "
                                           "the FP64 apply is bound by GB300's FP64 pipe, the FP32 apply by HBM"}
                   if app else None),
         "sweep": sweep,

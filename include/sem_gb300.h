@@ -83,7 +83,8 @@ enum sem_option {
     SEM_OPT_REFINE_TOL_SCALE = 9, /* mixed mode stops at |r| < s (tol |r0| + tol), s in (0,1],
                                     default 1 (the reference's test on the true residual) */
     SEM_OPT_ADAPTIVE_INNER = 12, /* mixed mode: 1 (default) a sweep's inner tolerance is relaxed
-                                    to what the outer test still needs (x 0.3), 0 always
+                                    to what the outer test still needs (x 0.3, with
+                                    SEM_PRECOND_FDM x 0.1), 0 always
                                     SEM_OPT_INNER_TOL */
     SEM_OPT_LEARNED_STEP = 15,   /* SEM_GUESS_LEARNED: 0 (default) move from the base guess along
                                     the predicted correction by the step that minimises the

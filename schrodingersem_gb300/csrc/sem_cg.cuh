@@ -386,6 +386,8 @@ __device__ __forceinline__ void cg_fdm(const EoS<N, f2_t>& t, f2_t* s, const flo
 #pragma unroll
         for (int k = 0; k < N; ++k) {
             const float al = fmaf(ly, lam[k], lx);
+            // the symbol of a preconditioner (2 ulp; an exact division made no
+            // difference to the solutions' errors and cost 3 % at 96 x 96, p = 12)
             const float inv = __fdividef(1.f, fmaf(al, al, mm));
             const f2_t d = cg_cmul(m[k], g.x * inv, al * inv);
             float a, b, c, e;

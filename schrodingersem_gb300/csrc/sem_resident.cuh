@@ -45,7 +45,9 @@ namespace semgb {
 // one row of both components per thread: 243 rows at 27 elements of p = 8.  With
 // 512 threads half the warps had no row and 128 registers spilled the line
 // contractions: 18.0 us per iteration at 64 x 64 elements of p = 8 against 15.9,
-// 11.8 against 9.7 at 24 x 24, 12.0 against 10.9 at 48 x 48 of p = 4
+// 11.8 against 9.7 at 24 x 24, 12.0 against 10.9 at 48 x 48 of p = 4.  256 threads
+// have up to 255 registers, which N <= 7 and one row of N = 9 (208) keep to; 2 and
+// 4 rows of N = 9 spill 240 and 176 bytes, N = 11 between 764 and 1,300
 constexpr int RES_TPB = 256;
 constexpr int RES_MAXQ = 8;     // words polled per lane: grids up to 256 blocks
 constexpr int RES_PAIRS = 4;    // planes of FP32 pairs: p, q, z, preconditioner symbol
@@ -294,6 +296,9 @@ __device__ __forceinline__ bool res_exchange(const float (&v)[K], const DevMesh&
     __syncthreads();
     bool ok = true;
     if (wid == 0) {
+        // the block's sum in FP32, as the word that carries it; pairs (two_add) made
+        // no difference to the solutions' errors and cost 8 % at 48 x 48, p = 4
+        // (12.2 to 13.1 us per iteration)
         constexpr int nw = RES_TPB / 32;
 #pragma unroll
         for (int k = 0; k < K; ++k) a[k] = lane < nw ? red[k][lane] : 0.f;

@@ -914,7 +914,9 @@ __global__ void __launch_bounds__(SOLVER_TPB, 1)
 // Threads and blocks per SM: measured per iteration at 192x192, 100x100 and
 // 64x64, p = 8: 269, 83, 57 us; 128 x 5: 290, 102, 91; 256 x 3 (80 registers,
 // spills): 247, 94, 67; before the vectors were interleaved as pairs and the
-// factors packed in 16 bytes (then 209, 55, 38)
+// factors packed in 16 bytes (then 209, 55, 38).  At 128 registers the line passes
+// spill from N = 9 on (114 bytes of stores there, 302 at N = 10, 978 at N = 13,
+// 1,250 at N = 17)
 constexpr int CG_TPB = 256, CG_BLOCKS = 2;
 template <int N>
 __global__ void __launch_bounds__(CG_TPB, CG_BLOCKS)
