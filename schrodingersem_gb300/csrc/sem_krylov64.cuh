@@ -29,10 +29,13 @@
 
 namespace semgb {
 
-// threads (at most): with long lines half as many, whose 255 registers hold a
-// line's contraction without spills
+// threads, at most.  At 128 registers the line contractions spill from N = 10 on,
+// but half as many threads with 255 leave the loads of a pass and the vector updates
+// to 8 warps, which costs more: 60 iterations on 75 x 75 elements of p = 11 took 16.4 ms
+// (MINRES, stage operator; 13.2 now) and 8.46 (Helmholtz; 7.26), on 62 x 62 of p = 14
+// 19.6 (15.8), on 32 x 32 of p = 12 2.29 (2.22, Helmholtz); only shares of one element
+// at p = 12 to 15 were 3 to 5 % faster
 constexpr int K64_TPB = 512;
-__host__ __device__ constexpr int k64_tpb(int N) { return N <= 11 ? K64_TPB : K64_TPB / 2; }
 constexpr int K64_MAXQ = 5;  // lines polled per lane: grids up to 160 blocks
 constexpr int K64_WSTRIDE = RESIDENT_SLOT_STRIDE;
 constexpr int K64_PART = K64_TPB / 2 + 4;  // block sum: half-warp partials, then four
@@ -352,7 +355,7 @@ struct K64Givens {
 };
 
 template <int N, int OP>
-__global__ void __launch_bounds__(k64_tpb(N), 1)
+__global__ void __launch_bounds__(K64_TPB, 1)
     k_minres64(DevMesh m, SolveArgs a, KrylovWork<double> w, const __grid_constant__ EoD<N, double> et,
                unsigned long long* slots, unsigned epoch0)
 {
@@ -542,7 +545,7 @@ __device__ __forceinline__ double pcg64_threshold(double tol, double b2) { retur
 
 // PCG on the Poisson operator (pcg.hpp:59-97, identity preconditioner)
 template <int N>
-__global__ void __launch_bounds__(k64_tpb(N), 1)
+__global__ void __launch_bounds__(K64_TPB, 1)
     k_pcg64(DevMesh m, SolveArgs a, KrylovWork<double> w, const __grid_constant__ EoD<N, double> et,
             unsigned long long* slots, unsigned epoch0)
 {
@@ -704,7 +707,7 @@ __device__ __forceinline__ void k64_apply_r(K64Op<N, OP>& op, const EoD<N, doubl
 }
 
 template <int N, int OP>
-__global__ void __launch_bounds__(k64_tpb(N), 1)
+__global__ void __launch_bounds__(K64_TPB, 1)
     k_minres64r(DevMesh m, SolveArgs a, KrylovWork<double> w, const __grid_constant__ EoD<N, double> et,
                 unsigned long long* slots, unsigned epoch0)
 {
@@ -866,7 +869,7 @@ __global__ void __launch_bounds__(k64_tpb(N), 1)
 }
 
 template <int N>
-__global__ void __launch_bounds__(k64_tpb(N), 1)
+__global__ void __launch_bounds__(K64_TPB, 1)
     k_pcg64r(DevMesh m, SolveArgs a, KrylovWork<double> w, const __grid_constant__ EoD<N, double> et,
              unsigned long long* slots, unsigned epoch0)
 {

@@ -980,7 +980,7 @@ static const void* solver_fn(int op, int kind)
 // block, the cheaper its barriers), at most K64_TPB
 inline int k64_threads(int N, int nc, int share)
 {
-    const int v = nc * share * N * N, top = k64_tpb(N);
+    const int v = nc * share * N * N, top = K64_TPB;
     return v >= top ? top : v < 128 ? 128 : (v + 31) / 32 * 32;
 }
 
@@ -1059,7 +1059,7 @@ int solver_plan(int op, int kind, int E, int sms, size_t smem_budget, int* kmax_
         if (s64 > smem) smem = s64;
     }
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : f64 ? k64_tpb(N) : SOLVER_TPB,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fdm ? CG_TPB : f64 ? K64_TPB : SOLVER_TPB,
                                                       smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
