@@ -1,7 +1,7 @@
 """Stage solves whose residual stays above its smallest value for hundreds of
 iterations (a potential well with alpha |V| = 25, a random potential with
 alpha |V| up to 80): the conjugate gradients go on to convergence and do not hand
-the solve to MINRES.  The judge is the reference's test on the true FP64 residual
+the solve to MINRES.  Success means the reference's test on the true FP64 residual
 (include/minres.hpp:92)."""
 import numpy as np
 import pytest
